@@ -143,6 +143,22 @@ __device__ __forceinline__ bool pr_idle(const PrState *st, int stage) {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// num / deg, infinite for deg 0 (a vertex without out-edges: nothing gathers
+// its contribution).  Dividing by the degree 0 itself leaves the division's
+// fast path, and one such lane sends its whole warp through the slow one: in
+// an R-MAT graph, where half of the vertices are isolated, nearly every warp
+// (k_pr_update at R-MAT 24, FP32: 908 us of a 3.05 ms iteration).  The degree
+// is converted from 32 bits where it fits in them.
+__device__ __forceinline__ float per_degree(float num, uint64_t deg) {
+    if (deg >> 32) return num / (float)deg;
+    const float q = num / (float)max((uint32_t)deg, 1u);
+    return deg ? q : __int_as_float(0x7F800000);
+}
+__device__ __forceinline__ double per_degree(double num, uint64_t deg) {
+    const double q = num / (double)(deg ? deg : 1ull);
+    return deg ? q : __longlong_as_double(0x7FF0000000000000ll);
+}
+
 // Scaled formats: FP8-E4M3 (max 448) and FP16 (max 65504, min normal 2^-14)
 // store contrib * scale with scale a power of two chosen so that the
 // largest contribution lands at half the format's range (2x headroom).
@@ -376,7 +392,7 @@ k_pr_update(const XT<DT> *__restrict__ y, XT<DT> *__restrict__ x, typename Store
             dl += fabs(x[v] - yv);
             x[v] = yv;
             const uint64_t deg = off[v + 1] - off[v];
-            contrib[v] = damp64 * yv / (double)deg;
+            contrib[v] = per_degree(damp64 * yv, deg);
         }
         (void)wf32;
         (void)enc_scale;
@@ -388,7 +404,7 @@ k_pr_update(const XT<DT> *__restrict__ y, XT<DT> *__restrict__ x, typename Store
         dl += (double)fabsf(xv - yv);
         x[v] = yv;
         const uint64_t deg = off[v + 1] - off[v];
-        const float c = damp * yv / (float)deg;
+        const float c = per_degree(damp * yv, deg);
         if constexpr (DT == GG_BF16) {
             contrib[v] = sr ? bf16_stochastic(c, v, (uint32_t)it) : S::enc(c);
             if (accum) acc[v] += yv;
@@ -465,7 +481,7 @@ __global__ void k_pr_reencode(const float *x, typename Store<DT>::T *contrib, co
     const uint32_t stride = gridDim.x * BLOCK;
     for (uint32_t v = blockIdx.x * BLOCK + threadIdx.x; v < n; v += stride) {
         const uint64_t deg = off[v + 1] - off[v];
-        const float c = damp * x[v] / (float)deg;
+        const float c = per_degree(damp * x[v], deg);
         if (pass == 0) {
             if (deg && c > cm) cm = c;
         } else {
@@ -491,7 +507,7 @@ __global__ void k_pr_init(XT<DT> *x, typename Store<DT>::T *contrib, const uint6
             for (uint32_t v = blockIdx.x * BLOCK + threadIdx.x; v < n; v += stride) {
                 const double xd = 1.0 / (double)n;
                 x[v] = xd;
-                contrib[v] = damp64 * xd / (double)(off[v + 1] - off[v]);
+                contrib[v] = per_degree(damp64 * xd, off[v + 1] - off[v]);
             }
         if (pass == 1 && blockIdx.x == 0 && threadIdx.x == 0) {
             st->scale = 1.0f;
@@ -503,7 +519,7 @@ __global__ void k_pr_init(XT<DT> *x, typename Store<DT>::T *contrib, const uint6
     const float scale = pass == 1 ? st->scale : 1.0f;  // set by k_pr_setscale between the passes
     for (uint32_t v = blockIdx.x * BLOCK + threadIdx.x; v < n; v += stride) {
         const uint64_t deg = off[v + 1] - off[v];
-        const float c = damp * x0 / (float)deg;
+        const float c = per_degree(damp * x0, deg);
         if (pass == 0) {
             if (deg && c > cm) cm = c;
         } else {

@@ -309,6 +309,15 @@ __global__ void k_word_costs(const uint64_t *in_off, uint32_t n, uint32_t T, uin
     }
 }
 
+// cut[i] = first word of range i of `ncut` ranges of equal work
+__global__ void k_light_cuts(const uint64_t *pre, uint32_t nwords, uint32_t *cut, uint32_t ncut) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= ncut; i += gridDim.x * blockDim.x) {
+        uint32_t lo, hi;
+        dev::balanced_range(pre, nwords, min(i, ncut - 1), ncut, lo, hi);
+        cut[i] = i < ncut ? lo : hi;
+    }
+}
+
 // crow[c] = heavy index owning chunk c
 __global__ void k_heavy_crow(const uint64_t *first, uint32_t nh, uint32_t *crow) {
     uint32_t h = blockIdx.x * blockDim.x + threadIdx.x;
@@ -390,7 +399,7 @@ gg_status build_heavy_rows(gg_graph *g) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     HeavyRows &H = g->heavy;
-    H.T = tuning().heavy_deg;
+    H.T = std::min(tuning().heavy_deg, kHeavyDegMax);
     H.CH = tuning().heavy_chunk;
     const uint32_t n = g->n;
     uint8_t *flag = nullptr;
@@ -442,6 +451,11 @@ gg_status build_heavy_rows(gg_graph *g) {
             HK(cub::DeviceScan::InclusiveSum(tmp, tb, H.light_prefix, H.light_prefix, (int64_t)nwords, st));
             HK(cub::DeviceScan::InclusiveSum(tmp, tb, H.pull_prefix, H.pull_prefix, (int64_t)nwords, st));
             ctx->launches += 2;
+            H.ncut = std::min(nwords, kLightCuts);
+            HK(cudaMalloc(&H.light_cut, ((size_t)H.ncut + 1) * 4));
+            k_light_cuts<<<grid_for(ctx, (uint64_t)H.ncut + 1), 256, 0, st>>>(H.light_prefix, nwords, H.light_cut,
+                                                                              H.ncut);
+            ctx->launches++;
         }
     }
     {
@@ -579,6 +593,7 @@ static void graph_free(gg_graph *g) {
     graph_bfs_free(g);
     cudaFree(g->heavy.light_prefix);
     cudaFree(g->heavy.pull_prefix);
+    cudaFree(g->heavy.light_cut);
     cudaFree(g->cand.list[0]);
     cudaFree(g->cand.list[1]);
     cudaFree(g->cand.cnt);

@@ -79,6 +79,12 @@ enum { NBINS = 3 };
 
 struct gg_graph;
 
+// Upper bound of HeavyRows::T (knob heavy_deg): the light rows of a 32-vertex
+// word then hold fewer than 2^32 edges.
+constexpr uint32_t kHeavyDegMax = 1u << 26;
+// Most ranges of HeavyRows::light_cut: over ten per resident warp.
+constexpr uint32_t kLightCuts = 1u << 16;
+
 // In-rows of the CSC longer than `T` edges ("heavy" rows: R-MAT hubs, all
 // at low ids) are cut into chunks of `CH` edges so that no warp walks a hub
 // row alone.  first[h]..first[h+1] are the chunks of heavy vertex v[h].
@@ -92,6 +98,10 @@ struct HeavyRows {
     //   pull_prefix : dense pull, min(in-degree, 16) + 2 per vertex
     uint64_t *light_prefix = nullptr;
     uint64_t *pull_prefix = nullptr;
+    // light_cut[0..ncut]: the words cut into ncut ranges of equal light_prefix
+    // work, small enough that warps taking them in turn finish together
+    uint32_t *light_cut = nullptr;
+    uint32_t ncut = 0;
     uint32_t nheavy = 0;
     uint64_t nchunks = 0;
     uint32_t T = 0, CH = 0;
@@ -245,9 +255,9 @@ struct Tuning {
     uint32_t heavy_deg = 256;    // CSC rows longer than this are chunked
     uint32_t heavy_chunk = 1024; // edges per chunk
     uint32_t large_chunk = 512;  // push: edges per chunk of a large-bin row
-    int pr_stream = 0;           // PageRank light rows: warp-streamed segmented gather
-    // PageRank kernels' grid cap in CTAs per SM (measured at R-MAT 25: 16
-    // against 8 cuts an FP32 iteration 6.63 -> 6.17 ms, BF16 4.07 -> 4.01)
+    int pr_stream = 0;           // accepted, without effect: one gather serves both settings' graphs
+    // PageRank kernels' grid cap in CTAs per SM (the gather takes at most the
+    // 5 that are resident)
     int pr_blocks_per_sm = 16;
     // analytics run as one device-driven cooperative launch: bit 0 BFS levels,
     // bit 1 BFS parents, bit 2 CC (the persistent grid reads values written

@@ -10,24 +10,25 @@
 //   delta = sum |x-y| (double); x = y; y = 0; contrib = d*x/outdeg
 // until iter == maxiter or delta <= tol.
 //
-// B200 design: two kernels per iteration plus a one-thread bookkeeping
-// kernel, all enqueued up front; a device-resident state block carries the
-// sums and a "done" flag that makes later iterations return immediately once
-// the residual test passes, so the host never synchronises inside the loop.
-//   k_pr_gather : warp owns 32 destinations; short rows summed per lane, long
-//                 rows by the whole warp with 4 independent coalesced loads in
-//                 flight per lane; contributions decoded from the storage
-//                 format (FP32, BF16, FP16, FP8-E4M3 with scale, customfp<6,10>,
-//                 BF16-by-truncation); accumulation in float or double; the
-//                 block sums of y (double) are folded in with one atomic per CTA.
+// B200 design: two kernels per iteration (three where there are heavy rows),
+// all enqueued up front; a device-resident state block carries the sums and a
+// "done" flag that makes later iterations return immediately once the
+// residual test passes, so the host never synchronises inside the loop.
+//   k_pr_gather : the light rows' contributions staged in shared memory 32
+//                 rows at a time, heavy rows chunk by chunk; contributions
+//                 decoded from the storage format (FP32, BF16, FP16, FP8-E4M3
+//                 with scale, customfp<6,10>, BF16-by-truncation);
+//                 accumulation in float or double; the block sums of y
+//                 (double) are folded in with one atomic per CTA.
 //   k_pr_update : y += w, y *= 1/s, delta, x = y, contrib = d*x/deg encoded,
 //                 one pass.  The second sum of the reference (sum of the
 //                 rounded y+w) is taken as s + n*w in double: equal in exact
 //                 arithmetic, different by at most n/2 float ulps of 1/n.
-//   k_pr_finish : residual test, iteration count, FP8 scale for the next
-//                 encode (from this iteration's max with 2x headroom); FP16
-//                 is scaled the same way, since contributions of order 1/n
-//                 fall below its normal range.
+//   pr_finish   : (last CTA of the update, staged runs: a kernel) residual
+//                 test, iteration count, FP8 scale for the next encode (from
+//                 this iteration's max with 2x headroom); FP16 is scaled the
+//                 same way, since contributions of order 1/n fall below its
+//                 normal range.
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_fp8.h>
@@ -110,6 +111,7 @@ struct PrState {
     // each stage's dtype and residual bound, and a re-encode request raised
     // when the stage changes
     int stage, nstages, reencode;
+    unsigned int updated;  // CTAs of the update kernel that have finished
     int stage_dt[4];
     double stage_tol[4];
     // BF16 stochastic rounding; tail averaging from iteration avg_from on
@@ -171,115 +173,222 @@ __device__ __host__ inline float scale_for(int dt, float cmax) {
     return ldexpf(1.0f, e - 1);
 }
 
+// y[d] (or its double twin) from a row's sum; returns the stored value for
+// the sum of all y.
+template <int DT, bool ADD_OLD, typename Acc>
+__device__ __forceinline__ double pr_store_row(float *y_f32, double *y_f64, uint32_t d, Acc acc, float sinv) {
+    if (DT == GG_FP8E4M3 || DT == GG_F16) acc *= (Acc)sinv;
+    if (y_f64) {
+        const double v = ADD_OLD ? y_f64[d] + (double)acc : (double)acc;
+        y_f64[d] = v;
+        return v;
+    }
+    const float v = ADD_OLD ? (float)((double)y_f32[d] + (double)acc) : (float)acc;
+    y_f32[d] = v;
+    return (double)v;
+}
+
+// Sum of the decoded contributions of in_adj[e0, e1) over the warp's lanes
+// (a lane's share; the caller reduces), 8 coalesced loads per lane in flight.
+template <int DT, typename Acc>
+__device__ __forceinline__ Acc pr_chunk_sum(const uint32_t *__restrict__ in_adj,
+                                            const typename Store<DT>::T *__restrict__ contrib, uint64_t e0,
+                                            uint64_t e1, uint32_t lane) {
+    using S = Store<DT>;
+    Acc part = 0;
+    uint64_t base = e0;
+    for (; base + 256 <= e1; base += 256) {
+        uint32_t s8[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) s8[u] = __ldcs(in_adj + base + 32 * u + lane);
+        XT<DT> c8[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) c8[u] = S::dec(contrib[s8[u]]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) part += (Acc)c8[u];
+    }
+    if (base < e1) {
+        uint32_t s8[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const uint64_t e = base + 32 * u + lane;
+            s8[u] = e < e1 ? __ldcs(in_adj + e) : 0u;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (base + 32 * u + lane < e1) part += (Acc)S::dec(contrib[s8[u]]);
+    }
+    return part;
+}
+
+// y[d] = sum of the contributions of d's in-neighbours (and, with st, the
+// sum of all y).  What bounds it: every gathered value that misses L1 moves
+// one 32-byte sector from L2, and an SM receives about one such sector per
+// clock (283 G gathers/s over the chip with uniform ids, 4- or 2-byte values;
+// up to 340 G/s with R-MAT ids, whose hubs hit L1), so the sums must stay off
+// the load/store unit as far as they can and enough loads be in flight.
+//   * Warps draw tickets: first the chunks of the heavy rows (rows above T
+//     edges, cut into H.CH-edge chunks), then ranges of 32-vertex words of
+//     equal light-edge work, so that no SM waits for a warp with long chunks
+//     (a fixed share per warp left warps idle for 8 % of the time).
+//   * The light rows of a word are one list of edges, staged in shared memory
+//     kStage at a time; ids are loaded one batch ahead of their values.  Then
+//     32, 16, ... or 1 lanes sum each row's part from there, depending on how
+//     many rows the stage holds, parts much longer than the others by the
+//     whole warp.  (A warp per row kept one id and one value per lane in
+//     flight and paid a five-step reduction per row.)
+//   * The edges of the heavy rows in a word are gaps in its list, which is
+//     then loaded in runs between them.
+// 2 KiB of stage per warp and 5 CTAs per SM: more of either takes L1 from the
+// gathered lines in flight (FP32, ER: 4 KiB 2.9 ms).  Measured per iteration,
+// the rest of it included, before -> after: R-MAT 24, FP32 with double sums
+// 2.23 -> 1.99 ms, BF16 1.98 -> 1.85; directed ER 2^24 x 32 4.27 -> 2.38 and
+// 2.78 -> 2.13; grid 2048^2 FP32 0.30 -> 0.09; R-MAT 14 0.044 -> 0.034.
+constexpr uint64_t kChunkGroup = 2;  // heavy-row chunks per ticket
+template <int DT> constexpr uint32_t kStage =
+    2048 / sizeof(typename Store<DT>::T) < 1024 ? 2048 / sizeof(typename Store<DT>::T) : 1024;
+
 template <int DT, bool ACC64, bool ADD_OLD, int BLOCK>
-__global__ void __launch_bounds__(BLOCK)
+__global__ void __launch_bounds__(BLOCK, 5)
 k_pr_gather(const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in_adj,
             const typename Store<DT>::T *__restrict__ contrib, uint32_t n, float *y_f32,
-            double *y_f64, PrState *st, float scale_inv_arg, int K, uint32_t T, int stream,
-            const uint64_t *__restrict__ word_prefix, int stage) {
+            double *y_f64, PrState *st, float scale_inv_arg, HeavyRows H,
+            typename std::conditional<ACC64, double, float>::type *partial, unsigned int *ticket, int stage) {
     using S = Store<DT>;
     using Acc = typename std::conditional<ACC64, double, float>::type;
-    constexpr int U = 4;  // 32-edge chunks in flight per warp iteration
-    __shared__ Acc sm[BLOCK / 32][33];
+    constexpr int U = 4;
+    constexpr uint32_t CAP = kStage<DT>;
+    __shared__ typename S::T sbuf[BLOCK / 32][CAP];
     if (pr_idle(st, stage)) return;
     const float sinv = st ? st->scale_inv : scale_inv_arg;
     const uint32_t lane = threadIdx.x & 31u;
-    Acc *row = sm[threadIdx.x >> 5];
-    const uint32_t nwords = (n + 31u) >> 5;
-    const uint32_t nw = (gridDim.x * BLOCK) >> 5;
+    typename S::T *buf = sbuf[threadIdx.x >> 5];
+    const uint32_t nw = (gridDim.x * BLOCK) >> 5, gw = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
     const uint64_t oend = in_off[n];
     double ysum = 0;
-    // a contiguous range of words of equal light-edge work per warp
-    uint32_t wlo, whi;
-    dev::balanced_range(word_prefix, nwords, (blockIdx.x * BLOCK + threadIdx.x) >> 5, nw, wlo, whi);
-    for (uint32_t w = wlo; w < whi; ++w) {
+    // offsets of the word's row, loaded one word ahead
+    auto bounds = [&](uint32_t w, uint64_t &b, uint64_t &e) {
         const uint32_t d = (w << 5) + lane;
-        const bool valid = d < n;
-        const uint64_t beg = valid ? in_off[d] : oend;
-        const uint64_t end = valid ? in_off[d + 1] : oend;
-        // heavy rows are summed by k_pr_heavy_chunks / k_pr_heavy_finalize
-        const bool heavy = end - beg > (uint64_t)T;
-        const bool mine = valid && !heavy;
-        Acc acc = 0;
-        if (stream && __ballot_sync(FULL, heavy) == 0) {
-            // Streaming: the word's 32 rows are contiguous in in_adj; lanes
-            // take consecutive edges, find their row by a 5-step search over
-            // the lanes' row starts, and sum per row with a segmented scan.
-            const uint64_t o0 = __shfl_sync(FULL, beg, 0);
-            const uint64_t o1 = __shfl_sync(FULL, end, 31);
-            row[lane] = 0;
-            __syncwarp();
-            for (uint64_t base = o0; base < o1; base += 32 * U) {
-                uint32_t sidx[U];
-                Acc val[U];
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint64_t e = base + u * 32 + lane;
-                    sidx[u] = e < o1 ? __ldg(in_adj + e) : 0u;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint64_t e = base + u * 32 + lane;
-                    val[u] = e < o1 ? (Acc)S::dec(contrib[sidx[u]]) : (Acc)0;
-                }
-#pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    const uint64_t e = base + u * 32 + lane;
-                    if (base + u * 32 >= o1) break;  // warp-uniform
-                    const bool ok = e < o1;
-                    uint32_t r = 0;
-#pragma unroll
-                    for (uint32_t step = 16; step >= 1; step >>= 1) {
-                        const uint64_t bc = __shfl_sync(FULL, beg, r + step);
-                        if (bc <= e) r += step;
-                    }
-                    if (!ok) r = 32;
-                    Acc v = val[u];
-#pragma unroll
-                    for (int dd = 1; dd < 32; dd <<= 1) {
-                        const Acc t = __shfl_up_sync(FULL, v, dd);
-                        const uint32_t rr = __shfl_up_sync(FULL, r, dd);
-                        if (lane >= (uint32_t)dd && rr == r) v += t;
-                    }
-                    const uint32_t rn = __shfl_down_sync(FULL, r, 1);
-                    const bool tail = lane == 31 || rn != r;
-                    if (ok && tail) row[r] += v;
-                    __syncwarp();
-                }
-            }
-            acc = row[lane];
-            __syncwarp();
-        } else {
-            // words holding a heavy row: per-row sums for the light rows
-            const bool shortrow = end - beg <= (uint64_t)K;
-            if (mine && shortrow)
-                for (uint64_t e = beg; e < end; ++e) acc += (Acc)S::dec(contrib[__ldg(in_adj + e)]);
-            unsigned pend = __ballot_sync(FULL, mine && !shortrow);
-            while (pend) {
-                const int j = __ffs(pend) - 1;
-                pend &= pend - 1;
-                const uint64_t bj = __shfl_sync(FULL, beg, j);
-                const uint64_t ej = __shfl_sync(FULL, end, j);
-                Acc part = 0;
-                for (uint64_t b2 = bj; b2 < ej; b2 += 32) {
-                    const uint64_t e = b2 + lane;
-                    if (e < ej) part += (Acc)S::dec(contrib[__ldg(in_adj + e)]);
-                }
-                part = dev::warp_sum(part);
-                if ((int)lane == j) acc = part;
-            }
+        b = e = oend;
+        if (d < n) {
+            b = in_off[d];
+            e = in_off[d + 1];
         }
-        if (mine) {
-            if (DT == GG_FP8E4M3 || DT == GG_F16) acc *= (Acc)sinv;
-            if (y_f64) {
-                double v = ADD_OLD ? y_f64[d] + (double)acc : (double)acc;
-                y_f64[d] = v;
-                ysum += v;
-            } else {
-                float v = ADD_OLD ? (float)((double)y_f32[d] + (double)acc) : (float)acc;
-                y_f32[d] = v;
-                ysum += (double)v;
+    };
+    // tickets: kChunkGroup chunks each, then the light ranges
+    const uint64_t ngroups = (H.nchunks + kChunkGroup - 1) / kChunkGroup;
+    uint64_t t = gw, next = 0;
+    for (; t < ngroups + H.ncut; t = __shfl_sync(FULL, next, 0)) {
+        if (lane == 0) next = (uint64_t)nw + atomicAdd(ticket, 1u);
+        if (t < ngroups) {
+            const uint64_t chi = min((t + 1) * kChunkGroup, H.nchunks);
+            for (uint64_t c = t * kChunkGroup; c < chi; ++c) {
+                const uint32_t lo = H.crow[c];  // heavy row owning chunk c
+                const uint32_t v = H.v[lo];
+                const uint64_t re = in_off[v + 1];
+                const uint64_t e0 = in_off[v] + (c - H.first[lo]) * H.CH;
+                const Acc part = dev::warp_sum(pr_chunk_sum<DT, Acc>(in_adj, contrib, e0, min(e0 + H.CH, re), lane));
+                if (lane == 0) partial[c] = part;
             }
+            continue;
+        }
+        uint32_t w = H.light_cut[t - ngroups];
+        const uint32_t whi = H.light_cut[t - ngroups + 1];
+        uint64_t beg = 0, end = 0, nbeg = 0, nend = 0;
+        if (w < whi) bounds(w, nbeg, nend);
+        for (; w < whi; ++w) {
+            const uint32_t d = (w << 5) + lane;
+            const bool valid = d < n;
+            beg = nbeg;
+            end = nend;
+            if (w + 1 < whi) bounds(w + 1, nbeg, nend);
+            const bool heavy = end - beg > (uint64_t)H.T;
+            unsigned gaps = __ballot_sync(FULL, heavy);
+            // the word's light edges as one list: this row's are [excl, excl + deg)
+            // (32 bits: H.T is at most kHeavyDegMax)
+            const uint32_t deg = heavy ? 0u : (uint32_t)(end - beg);
+            uint32_t stop = deg;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t t = __shfl_up_sync(FULL, stop, o);
+                if (lane >= (uint32_t)o) stop += t;
+            }
+            const uint32_t total = __shfl_sync(FULL, stop, 31);
+            const uint32_t excl = stop - deg;
+            const uint32_t *first = in_adj + __shfl_sync(FULL, beg, 0);  // of the list's current run
+            Acc acc = 0;
+            for (uint32_t base = 0; base < total; base += CAP) {
+                const uint32_t upto = min(base + CAP, total);
+                for (uint32_t at = base; at < upto;) {  // runs without a gap
+                    uint32_t run = upto;
+                    while (gaps) {
+                        const int j = __ffs(gaps) - 1;
+                        const uint32_t where = __shfl_sync(FULL, excl, j);
+                        if (where > at) {
+                            run = min(run, where);
+                            break;
+                        }
+                        first += __shfl_sync(FULL, end - beg, j);
+                        gaps &= gaps - 1;
+                    }
+                    uint32_t id[U];
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        const uint32_t p = at + 32 * u + lane;
+                        id[u] = p < run ? __ldcs(first + p) : 0u;
+                    }
+                    while (at < run) {
+                        uint32_t nx[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const uint32_t p = at + 32 * (U + u) + lane;
+                            nx[u] = p < run ? __ldcs(first + p) : 0u;
+                        }
+                        typename S::T val[U];
+#pragma unroll
+                        for (int u = 0; u < U; ++u)
+                            if (at + 32 * u + lane < run) val[u] = contrib[id[u]];
+#pragma unroll
+                        for (int u = 0; u < U; ++u) {
+                            const uint32_t p = at + 32 * u + lane;
+                            if (p < run) buf[p - base] = val[u];
+                            id[u] = nx[u];
+                        }
+                        at += 32 * U;
+                    }
+                    at = run;
+                }
+                __syncwarp();
+                // this row's part of the stage, [s, e) of buf
+                const uint32_t s = excl > base ? min(excl - base, CAP) : 0u;
+                const uint32_t e = stop > base ? min(stop - base, CAP) : 0u;
+                // the rows of this stage, [r0, r1], by 32, 16, ... 1 lanes each
+                const unsigned rows = __ballot_sync(FULL, e > s);
+                const uint32_t r0 = __ffs(rows) - 1, r1 = 31 - __clz(rows);
+                const uint32_t lg = r1 > r0 ? __clz(r1 - r0) - 27 : 5;  // log2 of the lanes per row
+                const uint32_t q = r0 + (lane >> lg);
+                const uint32_t sq = __shfl_sync(FULL, s, q & 31u), eq = __shfl_sync(FULL, e, q & 31u);
+                const uint32_t most = max(16u << lg, 64u);  // a longer part is summed by the whole warp
+                Acc part = 0;
+                if (q <= r1 && eq - sq <= most)
+                    for (uint32_t i = sq + (lane & ((1u << lg) - 1u)); i < eq; i += 1u << lg) part += (Acc)S::dec(buf[i]);
+                for (uint32_t o = (1u << lg) >> 1; o; o >>= 1) part += __shfl_xor_sync(FULL, part, o);
+                part = __shfl_sync(FULL, part, ((lane - r0) << lg) & 31u);
+                const bool wide = e > s + most;
+                if (e > s && !wide) acc += part;
+                unsigned pend = __ballot_sync(FULL, wide);
+                while (pend) {
+                    const int j = __ffs(pend) - 1;
+                    pend &= pend - 1;
+                    const uint32_t sj = __shfl_sync(FULL, s, j), ej = __shfl_sync(FULL, e, j);
+                    part = 0;
+                    for (uint32_t i = sj + lane; i < ej; i += 32) part += (Acc)S::dec(buf[i]);
+                    part = dev::warp_sum(part);
+                    if ((int)lane == j) acc += part;
+                }
+                __syncwarp();
+            }
+            if (valid && !heavy) ysum += pr_store_row<DT, ADD_OLD>(y_f32, y_f64, d, acc, sinv);
         }
     }
     if (st) {
@@ -288,55 +397,9 @@ k_pr_gather(const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in
     }
 }
 
-// One warp per chunk of a heavy row: partial[c] = sum of the chunk's
-// decoded contributions (4 independent coalesced loads per lane in flight).
-template <int DT, bool ACC64>
-__global__ void __launch_bounds__(256)
-k_pr_heavy_chunks(const uint64_t *__restrict__ in_off, const uint32_t *__restrict__ in_adj,
-                  const typename Store<DT>::T *__restrict__ contrib, HeavyRows H,
-                  typename std::conditional<ACC64, double, float>::type *partial, const PrState *st,
-                  int stage) {
-    using S = Store<DT>;
-    using Acc = typename std::conditional<ACC64, double, float>::type;
-    if (pr_idle(st, stage)) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t c = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; c < H.nchunks; c += nw) {
-        const uint32_t lo = H.crow[c];  // heavy row owning chunk c
-        const uint32_t v = H.v[lo];
-        const uint64_t rb = in_off[v], re = in_off[v + 1];
-        const uint64_t e0 = rb + (c - H.first[lo]) * H.CH;
-        const uint64_t e1 = min(e0 + H.CH, re);
-        Acc part = 0;
-        uint64_t base = e0;
-        for (; base + 256 <= e1; base += 256) {  // two 128-edge blocks of loads in flight
-            uint32_t s8[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) s8[u] = __ldg(in_adj + base + 32 * u + lane);
-            Acc c8[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) c8[u] = (Acc)S::dec(contrib[s8[u]]);
-            part += c8[0] + c8[1] + c8[2] + c8[3];
-            part += c8[4] + c8[5] + c8[6] + c8[7];
-        }
-        for (; base + 128 <= e1; base += 128) {
-            uint32_t s0 = __ldg(in_adj + base + lane);
-            uint32_t s1 = __ldg(in_adj + base + 32 + lane);
-            uint32_t s2 = __ldg(in_adj + base + 64 + lane);
-            uint32_t s3 = __ldg(in_adj + base + 96 + lane);
-            part += (Acc)S::dec(contrib[s0]) + (Acc)S::dec(contrib[s1]) +
-                    (Acc)S::dec(contrib[s2]) + (Acc)S::dec(contrib[s3]);
-        }
-        for (; base < e1; base += 32) {
-            uint64_t e = base + lane;
-            if (e < e1) part += (Acc)S::dec(contrib[__ldg(in_adj + e)]);
-        }
-        part = dev::warp_sum(part);
-        if (lane == 0) partial[c] = part;
-    }
-}
-
-// Heavy row totals, partials summed in chunk order (deterministic).
+// Heavy row totals from their chunks' partial sums, in a fixed order: a lane
+// per row, rows of more than 8 chunks by the whole warp (the largest hub of
+// R-MAT 24 has 1400 chunks, a chain of as many additions for one thread).
 template <int DT, bool ACC64, bool ADD_OLD, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 k_pr_heavy_finalize(HeavyRows H, const typename std::conditional<ACC64, double, float>::type *partial,
@@ -344,21 +407,27 @@ k_pr_heavy_finalize(HeavyRows H, const typename std::conditional<ACC64, double, 
     using Acc = typename std::conditional<ACC64, double, float>::type;
     if (pr_idle(st, stage)) return;
     const float sinv = st ? st->scale_inv : scale_inv_arg;
+    const uint32_t lane = threadIdx.x & 31u;
     double ysum = 0;
-    for (uint32_t h = blockIdx.x * BLOCK + threadIdx.x; h < H.nheavy; h += gridDim.x * BLOCK) {
+    for (uint32_t h0 = blockIdx.x * BLOCK; h0 < H.nheavy; h0 += gridDim.x * BLOCK) {
+        const uint32_t h = h0 + threadIdx.x;
+        const bool have = h < H.nheavy;
+        const uint64_t c0 = have ? H.first[h] : 0ull, c1 = have ? H.first[h + 1] : 0ull;
+        const bool wide = c1 - c0 > 8;
         Acc acc = 0;
-        for (uint64_t c = H.first[h]; c < H.first[h + 1]; ++c) acc += partial[c];
-        if (DT == GG_FP8E4M3 || DT == GG_F16) acc *= (Acc)sinv;
-        const uint32_t d = H.v[h];
-        if (y_f64) {
-            double v = ADD_OLD ? y_f64[d] + (double)acc : (double)acc;
-            y_f64[d] = v;
-            ysum += v;
-        } else {
-            float v = ADD_OLD ? (float)((double)y_f32[d] + (double)acc) : (float)acc;
-            y_f32[d] = v;
-            ysum += (double)v;
+        if (!wide)
+            for (uint64_t c = c0; c < c1; ++c) acc += partial[c];
+        unsigned pend = __ballot_sync(FULL, wide);
+        while (pend) {
+            const int j = __ffs(pend) - 1;
+            pend &= pend - 1;
+            const uint64_t b = __shfl_sync(FULL, c0, j), e = __shfl_sync(FULL, c1, j);
+            Acc part = 0;
+            for (uint64_t c = b + lane; c < e; c += 32) part += partial[c];
+            part = dev::warp_sum(part);
+            if ((int)lane == j) acc = part;
         }
+        if (have) ysum += pr_store_row<DT, ADD_OLD>(y_f32, y_f64, H.v[h], acc, sinv);
     }
     if (st) {
         ysum = dev::block_sum<double, BLOCK>(ysum);
@@ -366,11 +435,45 @@ k_pr_heavy_finalize(HeavyRows H, const typename std::conditional<ACC64, double, 
     }
 }
 
+// End of an iteration (one thread): record the residual, test it, next
+// stage, scales.  The sums come from other CTAs' atomics: read through L2.
+__device__ __forceinline__ void pr_finish(PrState *st, int dt) {
+    st->reencode = 0;
+    const int it = st->iters;
+    const double delta = __ldcg(&st->delta);
+    if (st->avg_from >= 0 && it >= st->avg_from) st->avg_n++;
+    if (it < GG_MAX_ITERS) st->deltas[it] = delta;
+    st->iters = it + 1;
+    if (st->nstages > 1) dt = st->stage_dt[st->stage];
+    if (st->stage + 1 < st->nstages && !(delta > st->stage_tol[st->stage])) {
+        // next stage: its re-encode kernels rewrite the contributions from x
+        st->stage++;
+        st->reencode = 1;
+        if (st->iters >= st->maxiter) st->done = 1;
+    } else {
+        if (st->iters >= st->maxiter || !(delta > st->tol)) st->done = 1;
+        st->scale_inv = 1.0f / st->scale;               // decode of what the update just wrote
+        st->scale = scale_for(dt, __ldcg(&st->cmax));  // next encode
+    }
+    st->s1 = 0;
+    st->delta = 0;
+    st->cmax = 0.0f;
+    st->updated = 0;
+}
+
+// Staged runs: the iteration ends after every stage's update kernel.
+__global__ void k_pr_finish(PrState *st, int dt) {
+    if (st->done) st->reencode = 0;
+    else pr_finish(st, dt);
+}
+
+// With `last`, the last CTA to finish ends the iteration (one launch fewer).
+// One thread also zeroes the next gather's ticket counter.
 template <int DT, int BLOCK>
 __global__ void __launch_bounds__(BLOCK)
 k_pr_update(const XT<DT> *__restrict__ y, XT<DT> *__restrict__ x, typename Store<DT>::T *contrib,
             const uint64_t *__restrict__ off, uint32_t n, float damp, double damp64, int renorm_f32, PrState *st,
-            int stage, float *acc = nullptr) {
+            int stage, unsigned int *ticket, bool last, float *acc = nullptr) {
     using S = Store<DT>;
     if (pr_idle(st, stage)) return;
     const int it = st->iters;
@@ -424,30 +527,15 @@ k_pr_update(const XT<DT> *__restrict__ y, XT<DT> *__restrict__ x, typename Store
         for (int i = 0; i < BLOCK / 32; ++i) b = fmaxf(b, sh[i]);
         atomicAdd(&st->delta, dl);
         atomicMax((int *)&st->cmax, __float_as_int(b));
+        if (blockIdx.x == 0) *ticket = 0;
+        if (last) {
+            __threadfence();  // this CTA's sums before its arrival
+            if (atomicAdd(&st->updated, 1u) == gridDim.x - 1) {
+                __threadfence();
+                pr_finish(st, DT);
+            }
+        }
     }
-}
-
-__global__ void k_pr_finish(PrState *st, int dt) {
-    st->reencode = 0;
-    if (st->done) return;
-    const int it = st->iters;
-    if (st->avg_from >= 0 && it >= st->avg_from) st->avg_n++;
-    if (it < GG_MAX_ITERS) st->deltas[it] = st->delta;
-    st->iters = it + 1;
-    if (st->nstages > 1) dt = st->stage_dt[st->stage];
-    if (st->stage + 1 < st->nstages && !(st->delta > st->stage_tol[st->stage])) {
-        // next stage: its re-encode kernels rewrite the contributions from x
-        st->stage++;
-        st->reencode = 1;
-        if (st->iters >= st->maxiter) st->done = 1;
-    } else {
-        if (st->iters >= st->maxiter || !(st->delta > st->tol)) st->done = 1;
-        st->scale_inv = 1.0f / st->scale;     // decode of what the update just wrote
-        st->scale = scale_for(dt, st->cmax);  // next encode
-    }
-    st->s1 = 0;
-    st->delta = 0;
-    st->cmax = 0.0f;
 }
 
 // Tail averaging: the ranks become the mean of the accumulated iterations.
@@ -542,7 +630,13 @@ static unsigned pr_grid(gg_ctx *ctx, uint64_t work) {
     return (unsigned)(b ? b : 1);
 }
 
-// gather of one iteration / one API call: light rows, heavy chunks, heavy totals
+// the gather's ticket counter: the entry after the chunks' partial sums, 0
+// when a gather starts (zeroed before a run, then by each update)
+static unsigned int *pr_ticket(gg_graph *g, void *partial) {
+    return (unsigned int *)((char *)partial + g->heavy.nchunks * 8);
+}
+
+// gather of one iteration / one API call: all rows, then heavy totals
 template <int DT, bool ACC64, bool ADD_OLD>
 static gg_status gather_launch(gg_graph *g, const typename Store<DT>::T *contrib, float *yf,
                                double *yd, PrState *st, float sinv, void *partial, int stage = -1) {
@@ -550,22 +644,18 @@ static gg_status gather_launch(gg_graph *g, const typename Store<DT>::T *contrib
     cudaStream_t s = ctx->stream;
     using Acc = typename std::conditional<ACC64, double, float>::type;
     const HeavyRows &H = g->heavy;
-    const uint64_t warps = (uint64_t)((g->n + 31) / 32);
+    const uint64_t warps = std::max<uint64_t>(((uint64_t)g->n + 31) / 32, H.nchunks);
     uint64_t blocks = (warps * 32 + 255) / 256;
-    const uint64_t cap = (uint64_t)ctx->sm_count * tuning().pr_blocks_per_sm;
+    // tickets balance the load, so one CTA for every place on the SMs
+    const uint64_t cap = (uint64_t)ctx->sm_count *
+                         std::min(resident_ctas((const void *)k_pr_gather<DT, ACC64, ADD_OLD, 256>, 256),
+                                  tuning().pr_blocks_per_sm);
     if (blocks > cap) blocks = cap;
     k_pr_gather<DT, ACC64, ADD_OLD, 256><<<(unsigned)(blocks ? blocks : 1), 256, 0, s>>>(
-        g->in_off, g->in_adj, contrib, g->n, yf, yd, st, sinv, tuning().pull_k, H.T, tuning().pr_stream,
-        H.light_prefix, stage);
+        g->in_off, g->in_adj, contrib, g->n, yf, yd, st, sinv, H, (Acc *)partial, pr_ticket(g, partial), stage);
     GG_LAUNCHED(ctx);
     if (H.nchunks) {
-        uint64_t cb = (H.nchunks * 32 + 255) / 256;
-        if (cb > cap) cb = cap;
-        k_pr_heavy_chunks<DT, ACC64><<<(unsigned)cb, 256, 0, s>>>(g->in_off, g->in_adj, contrib, H,
-                                                                  (Acc *)partial, st, stage);
-        GG_LAUNCHED(ctx);
-        uint64_t fb = (H.nheavy + 255) / 256;
-        if (fb > cap) fb = cap;
+        const uint64_t fb = std::min<uint64_t>((H.nheavy + 255) / 256, cap);
         k_pr_heavy_finalize<DT, ACC64, ADD_OLD, 256><<<(unsigned)fb, 256, 0, s>>>(H, (const Acc *)partial, yf, yd,
                                                                                  st, sinv, stage);
         GG_LAUNCHED(ctx);
@@ -608,9 +698,7 @@ static gg_status pr_run(gg_graph *g, const gg_pr_params *p, XT<DT> *x, XT<DT> *y
         else
             GG_CHECK((gather_launch<DT, false, false>(g, (const T *)contrib, yf, yd, st, 1.0f, partial)));
         k_pr_update<DT, kBlock><<<gv, kBlock, 0, s>>>(y, x, (T *)contrib, g->off, n, p->damping, d64,
-                                                      p->renorm_f32, st, -1, acc);
-        GG_LAUNCHED(ctx);
-        k_pr_finish<<<1, 1, 0, s>>>(st, DT);
+                                                      p->renorm_f32, st, -1, pr_ticket(g, partial), true, acc);
         GG_LAUNCHED(ctx);
     }
     if constexpr (DT == GG_BF16) {
@@ -642,7 +730,7 @@ static gg_status stage_op(gg_graph *g, int op, int stage, bool acc64, const gg_p
         return gather_launch<DT, false, false>(g, (const T *)contrib, y, nullptr, st, 1.0f, partial, stage);
     case OP_UPDATE:
         k_pr_update<DT, kBlock><<<gv, kBlock, 0, s>>>(y, x, (T *)contrib, g->off, g->n, p->damping, 0.0,
-                                                      p->renorm_f32, st, stage);
+                                                      p->renorm_f32, st, stage, pr_ticket(g, partial), false);
         break;
     case OP_REENC0:
     case OP_REENC1:
@@ -704,6 +792,7 @@ static gg_status gather_api(gg_graph *g, const gg_emap_desc *d) {
     const float sc = d->src_scale != 0.0f ? d->src_scale : 1.0f;
     void *partial = nullptr;
     GG_CHECK(graph_scratch(g, (g->heavy.nchunks + 1) * 8, &partial));
+    GG_CUDA(g->ctx, cudaMemsetAsync(pr_ticket(g, partial), 0, 8, g->ctx->stream));
     if (d->accum_f64)
         return gather_launch<DT, true, true>(g, (const T *)d->src->d, yf, yd, nullptr, sc, partial);
     return gather_launch<DT, false, true>(g, (const T *)d->src->d, yf, yd, nullptr, sc, partial);
@@ -736,6 +825,7 @@ static gg_status gather_src_filtered(gg_graph *g, const gg_emap_desc *d, gg_fron
     void *base = nullptr;
     GG_CHECK(graph_scratch(g, cb + (g->heavy.nchunks + 1) * 8, &base));
     void *partial = (char *)base + cb;
+    GG_CUDA(ctx, cudaMemsetAsync(pr_ticket(g, partial), 0, 8, ctx->stream));
     const unsigned grid = pr_grid(ctx, g->n);
     if (f64) {
         k_mask_contrib<double><<<grid, 256, 0, ctx->stream>>>((const double *)d->src->d, in->bitmap, g->n,
@@ -832,6 +922,7 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     uint64_t k0 = ctx->launches;
     cudaEventRecord(ctx->ev0, ctx->stream);
     cudaError_t e = cudaMemcpyAsync(st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(pr_ticket(g, partial), 0, 8, ctx->stream);
     if (e == cudaSuccess && acc) e = cudaMemsetAsync(acc, 0, (size_t)g->n * 4, ctx->stream);
     if (e == cudaSuccess) {
         if (staged) {

@@ -3162,6 +3162,26 @@ gg_status gg_kcore(gg_graph *g, const gg_run_opts *o, gg_prop *coreness, uint32_
     uint64_t k0 = ctx->launches;
     RunTimer tm(ctx);
     uint32_t *count = (uint32_t *)coreness->d;
+    // every step a sparse push and no per-step records wanted: the whole peel
+    // as one resident launch (R-MAT 20: 25.1 ms below, 7.5 ms there)
+    if (g->n && opt.threshold == GG_THRESH_ALWAYS_SPARSE && opt.variant == GG_VAR_AUTO && !opt.collect_stats) {
+        bool ran = false;
+        uint32_t big = 0;
+        int nsteps = 0, nfloors = 0;
+        GG_CHECK(kcore_resident(g, count, &ran, &big, &nsteps, &nfloors));
+        if (ran) {
+            const double ms = tm.stop();
+            if (st) {
+                st->iterations = nsteps;
+                st->total_ms = ms;
+                st->kernels = ctx->launches - k0;
+                st->vertices_reached = (uint64_t)nfloors;
+            }
+            if (largest_core) *largest_core = big;
+            if (host_coreness) GG_CHECK(gg_prop_download(coreness, host_coreness));
+            return gg_ctx_sync(ctx);
+        }
+    }
     GG_CUDA(ctx, cudaMemsetAsync(g->kc_cnt + 3, 0, 8, sm));
     if (g->n) {
         k_kc_init<<<persistent_grid(ctx, ((uint64_t)g->n + 31) / 32), 256, 0, sm>>>(g->off, g->n, count,

@@ -52,5 +52,39 @@ __device__ __forceinline__ bool sync(Barrier *b, unsigned long long timeout_ns) 
     return *(volatile unsigned int *)&b->err == 0;
 }
 
+// Barrier on one counter of arrivals that only grows: the e-th barrier is
+// over when e * gridDim.x CTAs have arrived, so the waiting CTAs see the last
+// arrival itself (the two-word barrier above adds a reset and a generation
+// store to it).  `epoch` is the calling CTA's own count, 0 at launch; the
+// counter starts at 0.
+struct Arrivals {
+    unsigned long long n;
+    unsigned int err;
+};
+
+__device__ __forceinline__ bool sync(Arrivals *b, unsigned long long &epoch, unsigned long long timeout_ns) {
+    __syncthreads();
+    ++epoch;
+    if (threadIdx.x == 0) {
+        __threadfence();
+        const unsigned long long target = epoch * gridDim.x;
+        volatile unsigned long long *np = &b->n;
+        if (atomicAdd(&b->n, 1ull) + 1 < target) {
+            const unsigned long long t0 = globaltimer();
+            while (*np < target) {
+                if (globaltimer() - t0 > timeout_ns) {
+                    atomicOr(&b->err, DEV_ERR_TIMEOUT);
+                    break;
+                }
+                if (*(volatile unsigned int *)&b->err) break;
+                __nanosleep(20);
+            }
+        }
+        __threadfence();
+    }
+    __syncthreads();
+    return *(volatile unsigned int *)&b->err == 0;
+}
+
 }  // namespace grid
 }  // namespace gg

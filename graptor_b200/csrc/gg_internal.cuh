@@ -168,6 +168,7 @@ struct gg_graph {
     // each) and their counters {count A, count B, smallest count left}
     uint32_t *kc_alive[2] = {nullptr, nullptr};
     unsigned long long *kc_cnt = nullptr;
+    void *kc_items = nullptr;  // gg_kcore's resident peel: state, items
     CandLists cand;               // pull candidate lists (driver runs)
     bool cand_active = false;     // a driver run uses them for its pull steps
     // released frontier buffers, reused in stream order
@@ -227,6 +228,7 @@ gg_status persistent_traverse(gg_graph *g, const gg_emap_desc &d, int level_k, b
                               int force_iter = -1, int force_variant = -1,
                               const uint32_t *d_roots = nullptr, uint32_t nroots = 0,
                               const PersistResume *resume = nullptr);
+gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *largest, int *steps, int *floors);
 gg_status enqueue_bfs_start(gg_graph *g, gg_prop *level, gg_prop *prev, const uint32_t *d_roots, uint32_t k);
 gg_status enqueue_cc_start(gg_graph *g, gg_prop *label, gg_prop *prev);
 gg_status run_tmp_prop(gg_graph *g, int slot, gg_dtype t, gg_prop **out);

@@ -200,3 +200,24 @@ def test_kcore_contract(ctx):
                               record=gg.RECORD_AT_FLOOR), F, out)
     assert e.value.status == gg.GG_ERR_UNSUPPORTED
     g.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("hubs,deg", [(1, 32), (1, 33), (3, 256), (3, 257), (2, 8500)])
+def test_kcore_resident_rows_at_item_edges(ctx, hubs, deg):
+    """Rows of 32, 33, 256, 257 and 8500 edges (one short item, one long, two
+    long, more long items than lanes) peeled by the resident launch: hubs over
+    a common set of leaves that also form a cycle, against the host-driven
+    peel's and the oracle's numbers."""
+    from graptor_b200 import gg
+    leaves = np.arange(hubs, hubs + deg, dtype=np.uint32)
+    src = np.concatenate([np.repeat(np.arange(hubs, dtype=np.uint32), deg), leaves])
+    dst = np.concatenate([np.tile(leaves, hubs), np.roll(leaves, 1)])
+    n = hubs + deg + 5  # five isolated vertices
+    g = ctx.from_edges(n, src, dst)
+    off, adj = g.download()
+    want, largest = O.kcore(O.Graph(n, off, adj))
+    for opts in (None, gg.default_opts(gg.THRESH_ALWAYS_SPARSE, collect=True)):
+        core, lc = g.kcore(opts=opts)
+        assert np.array_equal(core, want) and lc == largest
+    g.close()

@@ -579,7 +579,9 @@ static void graph_free(gg_graph *g) {
     cudaFree(g->kc_alive[0]);
     cudaFree(g->kc_alive[1]);
     cudaFree(g->kc_cnt);
-    cudaFree(g->kc_items);
+    cudaFree(g->kc_state);
+    cudaFree(g->items);
+    bfs_resident_free(g);
     cudaFree(g->pstate2);
     for (int i = 0; i < 2; ++i) {
         if (g->copy_done[i]) {
@@ -849,6 +851,7 @@ gg_status gg_tuning_set(const char *name, int64_t v) {
     else if (k == "fusion_queue" && (v == 0 || v >= 32)) t.fusion_queue = (uint32_t)v;
     else if (k == "cc_hook" && v <= 2) t.cc_hook = (int)v;
     else if (k == "graph" && v <= 1) t.graph = (int)v;
+    else if (k == "resident" && v <= 1) t.resident = (int)v;
     else if (k == "graph_handoff" && v <= (1 << 20)) t.graph_handoff = (int)v;
     else if (k == "handoff_ctas" && v <= (1 << 16)) t.handoff_ctas = (int)v;
     else if (k == "small_frontier" && v <= 1) t.small_frontier = (int)v;
@@ -889,6 +892,7 @@ gg_status gg_tuning_get(const char *name, int64_t *v) {
     else if (k == "fusion_queue") *v = t.fusion_queue;
     else if (k == "cc_hook") *v = t.cc_hook;
     else if (k == "graph") *v = t.graph;
+    else if (k == "resident") *v = t.resident;
     else if (k == "graph_handoff") *v = t.graph_handoff;
     else if (k == "handoff_ctas") *v = t.handoff_ctas;
     else if (k == "small_frontier") *v = t.small_frontier;

@@ -2804,9 +2804,12 @@ gg_status gg_bfs_level(gg_graph *g, uint32_t root, const gg_run_opts *o, gg_prop
     const bool graph_mode = (tuning().graph & 1) && !(tuning().persistent & 1) && g->force_iter < 0 &&
                             opt.variant == GG_VAR_AUTO;
     if (graph_mode) {
+        bool res = false;
+        if (tuning().resident) GG_CHECK(bfs_resident_prepare(g, &res));
         RunTimer tm(g->ctx);
         int iters = 0;
-        GG_CHECK(graph_bfs_level(g, root, opt, level, prev, st, &iters));
+        if (res) GG_CHECK(bfs_resident(g, level, root, opt, st, &iters));
+        else GG_CHECK(graph_bfs_level(g, root, opt, level, prev, st, &iters));
         const double ms = tm.stop();
         if (st) {
             st->iterations = iters;
@@ -2917,28 +2920,35 @@ gg_status gg_bfs_level_multi(gg_graph *g, const uint32_t *roots, uint32_t k, con
     uint32_t *d_roots = (uint32_t *)((char *)scr + roots_at);
     if (!r.empty())
         GG_CUDA(ctx, cudaMemcpyAsync(d_roots, r.data(), r.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
+    bool res = false;
+    if (tuning().resident && opt.variant == GG_VAR_AUTO && g->force_iter < 0 && !r.empty())
+        GG_CHECK(bfs_resident_prepare(g, &res));
     RunTimer tm(ctx);
-    int32_t inf = (int32_t)g->n + 1;
-    GG_CHECK(gg_prop_fill(level, &inf));  // (prev: unused by level-synchronous steps)
-    if (!r.empty()) {
-        k_scatter_zero_i32<<<((unsigned)r.size() + 255) / 256, 256, 0, ctx->stream>>>(
-            (int32_t *)level->d, (int32_t *)prev->d, d_roots, (uint32_t)r.size());
-        GG_LAUNCHED(ctx);
-    }
-    gg_emap_desc desc;
-    memset(&desc, 0, sizeof(desc));
-    desc.relax = GG_RELAX_MIN_PLUS1_I32;
-    desc.a = level;
-    desc.dst_filter = GG_FILTER_GT_CONST;
-    desc.src_level_sync = 1;
-    desc.record = GG_RECORD_NE_PREV;
-    desc.prev = prev;
-    desc.threshold = opt.threshold;
-    desc.threshold_k = opt.threshold_k;
-    desc.variant = opt.variant;
-    // one device-driven launch for all roots
     int iters = 0;
-    GG_CHECK(persistent_traverse(g, desc, 1, false, 0, opt, st, &iters, -1, -1, d_roots, (uint32_t)r.size()));
+    if (res) {
+        GG_CHECK(bfs_resident_multi(g, level, d_roots, (uint32_t)r.size(), opt, st, &iters));
+    } else {
+        int32_t inf = (int32_t)g->n + 1;
+        GG_CHECK(gg_prop_fill(level, &inf));  // (prev: unused by level-synchronous steps)
+        if (!r.empty()) {
+            k_scatter_zero_i32<<<((unsigned)r.size() + 255) / 256, 256, 0, ctx->stream>>>(
+                (int32_t *)level->d, (int32_t *)prev->d, d_roots, (uint32_t)r.size());
+            GG_LAUNCHED(ctx);
+        }
+        gg_emap_desc desc;
+        memset(&desc, 0, sizeof(desc));
+        desc.relax = GG_RELAX_MIN_PLUS1_I32;
+        desc.a = level;
+        desc.dst_filter = GG_FILTER_GT_CONST;
+        desc.src_level_sync = 1;
+        desc.record = GG_RECORD_NE_PREV;
+        desc.prev = prev;
+        desc.threshold = opt.threshold;
+        desc.threshold_k = opt.threshold_k;
+        desc.variant = opt.variant;
+        // one device-driven launch for all roots
+        GG_CHECK(persistent_traverse(g, desc, 1, false, 0, opt, st, &iters, -1, -1, d_roots, (uint32_t)r.size()));
+    }
     double ms = tm.stop();
     if (st) {
         st->iterations = iters;

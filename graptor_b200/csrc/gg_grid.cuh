@@ -62,26 +62,31 @@ struct Arrivals {
     unsigned int err;
 };
 
+// One thread per CTA, whose other threads' writes it has seen: arrive as the
+// `epoch`-th time and wait for the others.  False: the wait ran out somewhere.
+__device__ __forceinline__ bool arrive_and_wait(Arrivals *b, unsigned long long epoch, unsigned long long timeout_ns) {
+    __threadfence();
+    const unsigned long long target = epoch * gridDim.x;
+    volatile unsigned long long *np = &b->n;
+    if (atomicAdd(&b->n, 1ull) + 1 < target) {
+        const unsigned long long t0 = globaltimer();
+        while (*np < target) {
+            if (globaltimer() - t0 > timeout_ns) {
+                atomicOr(&b->err, DEV_ERR_TIMEOUT);
+                break;
+            }
+            if (*(volatile unsigned int *)&b->err) break;
+            __nanosleep(20);
+        }
+    }
+    __threadfence();
+    return *(volatile unsigned int *)&b->err == 0;
+}
+
 __device__ __forceinline__ bool sync(Arrivals *b, unsigned long long &epoch, unsigned long long timeout_ns) {
     __syncthreads();
     ++epoch;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        const unsigned long long target = epoch * gridDim.x;
-        volatile unsigned long long *np = &b->n;
-        if (atomicAdd(&b->n, 1ull) + 1 < target) {
-            const unsigned long long t0 = globaltimer();
-            while (*np < target) {
-                if (globaltimer() - t0 > timeout_ns) {
-                    atomicOr(&b->err, DEV_ERR_TIMEOUT);
-                    break;
-                }
-                if (*(volatile unsigned int *)&b->err) break;
-                __nanosleep(20);
-            }
-        }
-        __threadfence();
-    }
+    if (threadIdx.x == 0) arrive_and_wait(b, epoch, timeout_ns);
     __syncthreads();
     return *(volatile unsigned int *)&b->err == 0;
 }

@@ -168,7 +168,9 @@ struct gg_graph {
     // each) and their counters {count A, count B, smallest count left}
     uint32_t *kc_alive[2] = {nullptr, nullptr};
     unsigned long long *kc_cnt = nullptr;
-    void *kc_items = nullptr;  // gg_kcore's resident peel: state, items
+    void *kc_state = nullptr;  // gg_kcore's resident peel
+    void *items = nullptr;     // work items of the resident kernels (gg_items.cuh)
+    void *bfs_res = nullptr;   // resident BFS: buffers
     CandLists cand;               // pull candidate lists (driver runs)
     bool cand_active = false;     // a driver run uses them for its pull steps
     // released frontier buffers, reused in stream order
@@ -229,6 +231,15 @@ gg_status persistent_traverse(gg_graph *g, const gg_emap_desc &d, int level_k, b
                               const uint32_t *d_roots = nullptr, uint32_t nroots = 0,
                               const PersistResume *resume = nullptr);
 gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *largest, int *steps, int *floors);
+struct PState;
+gg_status bfs_resident_prepare(gg_graph *g, bool *ok);
+gg_status bfs_resident(gg_graph *g, gg_prop *level, uint32_t root, const gg_run_opts &opt, gg_run_stats *st,
+                       int *iters_out);
+gg_status bfs_resident_enqueue(gg_graph *g, gg_prop *level, const uint32_t *d_roots, uint32_t nroots,
+                               const gg_run_opts &opt, PState *st);
+gg_status bfs_resident_multi(gg_graph *g, gg_prop *level, const uint32_t *d_roots, uint32_t nroots,
+                             const gg_run_opts &opt, gg_run_stats *stats, int *iters_out);
+void bfs_resident_free(gg_graph *g);
 gg_status enqueue_bfs_start(gg_graph *g, gg_prop *level, gg_prop *prev, const uint32_t *d_roots, uint32_t k);
 gg_status enqueue_cc_start(gg_graph *g, gg_prop *label, gg_prop *prev);
 gg_status run_tmp_prop(gg_graph *g, int slot, gg_dtype t, gg_prop **out);
@@ -270,6 +281,9 @@ struct Tuning {
     // iteration's push/pull decision on the device (host-driven kernels, no
     // per-iteration host round trip): bit 0 BFS levels
     int graph = 1;
+    // BFS levels as one resident cooperative launch (gg_bfs.cu) where the
+    // graph-driven run would be taken
+    int resident = 1;
     // graph-driven BFS levels: a run still going after this many iterations
     // (a high-diameter graph: many small frontiers, where the graph's
     // per-step node launches cost more than a grid barrier) continues in the

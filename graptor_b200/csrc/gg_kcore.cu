@@ -10,10 +10,9 @@
 //   peel step       : the rows of the vertices peeled by the phase before are
 //                     counted down towards L; the take that brings a vertex
 //                     to L peels it (its row is the next step's work).
-// A peeled row becomes items {first edge, length}: one for a row of at most
-// kShort edges, else one per kLong edges, so that a step's work spreads over
-// all warps whatever the rows' lengths (the late floors of R-MAT peel a few
-// hubs of thousands of edges).  Every vertex is peeled once, so the two item
+// A peeled row becomes items (gg_items.cuh), so that a step's work spreads
+// over all warps whatever the rows' lengths (the late floors of R-MAT peel a
+// few hubs of thousands of edges).  Every vertex is peeled once, so the item
 // arrays are only ever appended to.
 //
 // A phase's counters (items, vertices at the floor and above) live in one of
@@ -29,14 +28,14 @@
 
 #include "gg_grid.cuh"
 #include "gg_internal.cuh"
+#include "gg_items.cuh"
 
 namespace gg {
 
-constexpr uint32_t kShort = 32, kLong = 256;  // edges per item
 constexpr int kKcBlock = 512;
 
 struct alignas(128) KcSlot {
-    unsigned long long nshort, nlong;  // items appended
+    unsigned long long items[IT_KINDS];  // appended
     unsigned long long at, above;      // scan: vertices at the floor, above it
     unsigned long long min_above;      // scan: smallest count above it
 };
@@ -54,54 +53,14 @@ struct KcArgs {
     uint32_t n;
     uint32_t *count;
     uint32_t *alive[2];
-    unsigned long long *items_s, *items_l;
+    ItemLists items;
     KcState *st;
     unsigned long long timeout_ns;
 };
 
-__device__ __forceinline__ unsigned long long kc_item(uint64_t beg, uint32_t len) { return (beg << 10) | len; }
-
-// Per-warp staging of item appends (see dev::WarpAppender): `dst` is where
-// this phase's items start, `dst_n` counts them.
-struct ItemAppender {
-    static constexpr uint32_t CAP = 64;
-    unsigned long long *buf, *dst, *dst_n;
-    uint32_t n = 0;
-    __device__ __forceinline__ void push(bool keep, unsigned long long item) {
-        const uint32_t lane = threadIdx.x & 31u;
-        const unsigned mk = __ballot_sync(0xffffffffu, keep);
-        if (keep) buf[n + __popc(mk & ((1u << lane) - 1u))] = item;
-        n += __popc(mk);
-        if (n > CAP - 32) flush();
-    }
-    __device__ __forceinline__ void flush() {
-        __syncwarp();
-        unsigned long long base = 0;
-        if (n && (threadIdx.x & 31u) == 0) base = atomicAdd(dst_n, (unsigned long long)n);
-        store(__shfl_sync(0xffffffffu, base, 0));
-    }
-    // the staged items to dst[base ...]
-    __device__ __forceinline__ void store(unsigned long long base) {
-        for (uint32_t i = threadIdx.x & 31u; i < n; i += 32) dst[base + i] = buf[i];
-        __syncwarp();
-        n = 0;
-    }
-};
-
-// both lists' last items: the two counters' round trips overlap
-__device__ __forceinline__ void flush_both(ItemAppender &a, ItemAppender &b) {
-    __syncwarp();
-    const uint32_t lane = threadIdx.x & 31u;
-    unsigned long long base = 0;
-    if (lane == 0 && a.n) base = atomicAdd(a.dst_n, (unsigned long long)a.n);
-    if (lane == 1 && b.n) base = atomicAdd(b.dst_n, (unsigned long long)b.n);
-    a.store(__shfl_sync(0xffffffffu, base, 0));
-    b.store(__shfl_sync(0xffffffffu, base, 1));
-}
-
 __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ unsigned long long s_items[kKcBlock / 32][2][ItemAppender::CAP];
+    __shared__ unsigned long long s_items[kKcBlock / 32][IT_KINDS][ItemAppender::CAP];
     __shared__ uint32_t s_alive[kKcBlock / 32][128];
     KcState *st = A.st;
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
@@ -109,26 +68,13 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
     const uint64_t gw = ((uint64_t)blockIdx.x * kKcBlock + threadIdx.x) >> 5;
     const bool first_thread = blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long epoch = 0;
-    unsigned long long hs = 0, hl = 0;  // items of the phases before the last one
+    unsigned long long head[IT_KINDS] = {0, 0, 0};  // items of the phases before the last one
     uint32_t q = 0, floors = 0, steps = 0, largest = 0;
     uint64_t L = 0, na = A.n;
     int cur = -1;  // alive list in use; -1: every vertex
 
-    ItemAppender sh{s_items[wib][0], nullptr, nullptr}, lg{s_items[wib][1], nullptr, nullptr};
-    // the row [beg, beg + deg) of a peeled vertex becomes items (all lanes together)
-    auto emit = [&](bool rec, uint64_t beg, uint64_t deg) {
-        sh.push(rec && deg && deg <= kShort, kc_item(beg, (uint32_t)deg));
-        unsigned big = __ballot_sync(FULL, rec && deg > kShort);
-        while (big) {
-            const int j = __ffs(big) - 1;
-            big &= big - 1;
-            const uint64_t b = __shfl_sync(FULL, beg, j), dg = __shfl_sync(FULL, deg, j);
-            for (uint64_t o = 0; o < dg; o += 32 * kLong) {  // warp-uniform
-                const uint64_t p = o + (uint64_t)lane * kLong;
-                lg.push(p < dg, kc_item(b + p, (uint32_t)min((uint64_t)kLong, dg - min(p, dg))));
-            }
-        }
-    };
+    ItemLister lister;
+    lister.init(s_items[wib]);
     // d loses one while it is above the floor; true for the take that brings
     // it there.  A take that finds it at the floor already (others took it
     // meanwhile) is given back; counts stay below 2^31, so one read as
@@ -149,24 +95,21 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
             b = A.off[d];
             dg = A.off[d + 1] - b;
         }
-        emit(rec, b, dg);
+        lister.list(rec, b, dg);
     };
     auto begin = [&](KcSlot *out) {
         if (first_thread) {
             KcSlot *next = &st->slot[(q + 1) % 3];
-            next->nshort = next->nlong = next->at = next->above = 0;
+            next->items[0] = next->items[1] = next->items[2] = next->at = next->above = 0;
             next->min_above = ~0ull;
         }
-        sh.dst_n = &out->nshort;
-        lg.dst_n = &out->nlong;
+        lister.begin(A.items, head, out->items);
     };
 
     for (;;) {
         // ---- scan of floor L
         KcSlot *out = &st->slot[q % 3];
         begin(out);
-        sh.dst = A.items_s + hs;
-        lg.dst = A.items_l + hl;
         {
             const uint32_t *alive = cur < 0 ? nullptr : A.alive[cur];
             dev::WarpAppender<128> keep{s_alive[wib], 0, A.alive[cur < 0 ? 0 : cur ^ 1], &out->above};
@@ -189,10 +132,10 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
                     if (above) mn = min(mn, c);
                 }
                 at_n += at;
-                if (__any_sync(FULL, at)) emit(at, beg, deg);
+                if (__any_sync(FULL, at)) lister.list(at, beg, deg);
                 keep.push(above, v);
             }
-            flush_both(sh, lg);
+            lister.flush();
             keep.flush();
             mn = __reduce_min_sync(FULL, mn);
             if (lane == 0 && mn != 0xFFFFFFFFu) atomicMin(&out->min_above, (unsigned long long)mn);
@@ -204,7 +147,8 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
         ++floors;
         const unsigned long long at = __ldcg(&out->at), above = __ldcg(&out->above);
         const unsigned long long smallest = __ldcg(&out->min_above);
-        unsigned long long ns = __ldcg(&out->nshort), nl = __ldcg(&out->nlong);
+        unsigned long long ns = __ldcg(&out->items[IT_SHORT]), nl = __ldcg(&out->items[IT_LONG]),
+                           nh = __ldcg(&out->items[IT_HUGE]);
         cur = cur < 0 ? 0 : cur ^ 1;
         na = above;
         if (at == 0) {
@@ -214,18 +158,17 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
         }
         largest = (uint32_t)L;
         // ---- peel steps at floor L
-        while (ns || nl) {
+        while (ns || nl || nh) {
             out = &st->slot[q % 3];
+            const unsigned long long *is = A.items.p[IT_SHORT] + head[IT_SHORT], *il = A.items.p[IT_LONG] + head[IT_LONG],
+                                     *ih = A.items.p[IT_HUGE] + head[IT_HUGE];
+            head[IT_SHORT] += ns;
+            head[IT_LONG] += nl;
+            head[IT_HUGE] += nh;
             begin(out);
-            const unsigned long long *is = A.items_s + hs, *il = A.items_l + hl;
-            hs += ns;
-            hl += nl;
-            sh.dst = A.items_s + hs;
-            lg.dst = A.items_l + hl;
-            for (uint64_t i = gw; i < nl; i += nw) {
-                const unsigned long long it = __ldcg(il + i);
-                const uint32_t *row = A.adj + (it >> 10);
-                const uint32_t len = (uint32_t)(it & 1023u);
+            // up to kLong edges from `first`, all in flight
+            auto piece = [&](uint64_t first, uint32_t len) {
+                const uint32_t *row = A.adj + first;
                 constexpr int U = kLong / 32;
                 uint32_t d[U];
                 bool rec[U];
@@ -235,24 +178,33 @@ __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
                 for (int u = 0; u < U; ++u) rec[u] = 32 * u + lane < len && take(d[u]);
 #pragma unroll
                 for (int u = 0; u < U; ++u) record(rec[u], d[u]);
+            };
+            for (uint64_t i = blockIdx.x; i < nh; i += gridDim.x) {
+                const unsigned long long it = __ldcg(ih + i);
+                const uint32_t len = item_len(it);
+                for (uint32_t o = wib * kLong; o < len; o += (kKcBlock / 32) * kLong)
+                    piece(item_first(it) + o, min(kLong, len - o));
             }
-            // short rows: as few per warp as spread the step over all warps,
-            // at most 32, their edges walked as one list
-            uint32_t group = 1;
-            while (group < 32 && (uint64_t)group * nw < ns) group <<= 1;
+            const uint32_t parts = long_pieces(nl, nw), width = kLong / parts;
+            for (uint64_t i = gw; i < nl * parts; i += nw) {
+                const unsigned long long it = __ldcg(il + i / parts);
+                const uint32_t len = item_len(it), o = (uint32_t)(i % parts) * width;
+                if (o < len) piece(item_first(it) + o, min(width, len - o));
+            }
+            const uint32_t group = short_group(ns, nw);
             for (uint64_t base = gw * group; base < ns; base += nw * group) {
                 unsigned long long it = 0;
                 if (lane < group && base + lane < ns) it = __ldcg(is + base + lane);
                 dev::warp_flat_rows<4>(
-                    A.adj, it >> 10, (uint32_t)(it & 1023u), 0u, [&](uint32_t d, uint32_t) { return take(d); },
-                    record);
+                    A.adj, item_first(it), item_len(it), 0u, [&](uint32_t d, uint32_t) { return take(d); }, record);
             }
-            flush_both(sh, lg);
+            lister.flush();
             if (!grid::sync(&st->bar, epoch, A.timeout_ns)) return;
             ++q;
             ++steps;
-            ns = __ldcg(&out->nshort);
-            nl = __ldcg(&out->nlong);
+            ns = __ldcg(&out->items[IT_SHORT]);
+            nl = __ldcg(&out->items[IT_LONG]);
+            nh = __ldcg(&out->items[IT_HUGE]);
         }
         if (above == 0) break;
         ++L;
@@ -283,24 +235,25 @@ __global__ void __launch_bounds__(256) k_kc_start(const uint64_t *__restrict__ o
     if (threadIdx.x == 0 && k) atomicAdd(&st->many, k);
 }
 
+unsigned long long *graph_items(gg_graph *g) {
+    const size_t total = items_cap(g, IT_SHORT) + items_cap(g, IT_LONG) + items_cap(g, IT_HUGE);
+    if (!g->items && cudaMalloc(&g->items, total * 8) != cudaSuccess) {
+        cudaGetLastError();
+        g->items = nullptr;
+    }
+    return (unsigned long long *)g->items;
+}
+
 // The whole peel of g into count[] (g->n entries, alive lists allocated).
 // *ran = false, and nothing done, where the item arrays do not fit in memory.
 gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *largest, int *steps, int *floors) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     *ran = false;
-    // every vertex is peeled once: at most n short items, and long items for
-    // rows above kShort edges (fewer than m / kShort rows)
-    const uint64_t cs = g->n + 1ull, cl = g->m / kShort + g->m / kLong + 2;
-    const size_t state = (sizeof(KcState) + 255) / 256 * 256;
-    if (!g->kc_items) {
-        if (cudaMalloc(&g->kc_items, state + (cs + cl) * 8) != cudaSuccess) {
-            cudaGetLastError();
-            g->kc_items = nullptr;
-            return GG_OK;
-        }
-    }
-    KcState *st = (KcState *)g->kc_items;
+    unsigned long long *items = graph_items(g);
+    if (!items) return GG_OK;
+    if (!g->kc_state) GG_CUDA(ctx, cudaMalloc(&g->kc_state, sizeof(KcState)));
+    KcState *st = (KcState *)g->kc_state;
     KcArgs A;
     A.off = g->off;
     A.adj = g->adj;
@@ -308,8 +261,7 @@ gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *larg
     A.count = count;
     A.alive[0] = g->kc_alive[0];
     A.alive[1] = g->kc_alive[1];
-    A.items_s = (unsigned long long *)((char *)g->kc_items + state);
-    A.items_l = A.items_s + cs;
+    A.items = item_lists(g, items);
     A.st = st;
     A.timeout_ns = tuning().barrier_timeout_ns;
     KcState init;

@@ -30,6 +30,7 @@
 #include "gg_internal.cuh"
 #include "gg_batch.h"
 #include "gg_mlp.cuh"
+#include "gg_persist.cuh"
 
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -39,51 +40,6 @@ namespace gg {
 constexpr unsigned FULLP = 0xffffffffu;
 constexpr int kPB = 256;           // threads per CTA
 constexpr uint32_t kLargeScan = 1024;  // large-bin rows chunked when at most this many
-// BFS levels: a listed frontier of at most this many vertices and edges
-// continues in the one-cluster kernel k_small_bfs
-constexpr unsigned long long kSmallEnterV = 8192, kSmallEnterE = 65536;
-
-struct PFront {
-    uint32_t *bins[NBINS];
-    uint32_t *bitmap;
-    unsigned long long *cnt;  // FC_WORDS
-};
-
-struct PState {
-    unsigned int bar_count;
-    unsigned int bar_gen;
-    unsigned int err;
-    int iterations;
-    int has_list[2];
-    int all[2];
-    unsigned long long cand_n[2];
-    int cand_valid;
-    int cand_cur;
-    int variant[GG_MAX_ITERS];
-    unsigned long long nactv[GG_MAX_ITERS];
-    unsigned long long nacte[GG_MAX_ITERS];
-    unsigned long long scanned[GG_MAX_ITERS];
-    unsigned long long t_ns[GG_MAX_ITERS + 1];
-    unsigned long long reached_v, reached_e;
-    // timing collection: the forced iteration's input counts, its start and
-    // end, and the end of the run (any iteration index)
-    unsigned long long f_nactv, f_nacte, f_reached, f_t0, f_t1, t_end;
-    int f_seen;
-    unsigned long long zeros;  // CC: vertices labelled 0 after the first step
-    // fused push work queue counters (reset between iterations), one
-    // 128-byte line each so that claims, appends and completions do not
-    // contend for one L2 line
-    struct alignas(128) Line { unsigned long long v; };
-    Line wq_head, wq_tail, wq_done;
-    // small-frontier hand-over (BFS levels): the traversal left the frontier
-    // at small_cur after small_iter iterations for k_small_bfs (exit_small),
-    // which either finishes the run (small_done) or hands back the same way
-    int exit_small, small_done, small_iter, small_cur;
-    // learned policy: the next step's choice, taken by one warp of CTA 0
-    // while the grid finishes the current step (slot = iteration & 1)
-    int next_choice[2];
-};
-
 struct PArgs {
     const uint64_t *off, *in_off;
     const uint32_t *adj, *in_adj;
@@ -1764,6 +1720,39 @@ gg_status persistent_state_read(gg_graph *g, void *state, const PArgs &P, gg_run
     return GG_OK;
 }
 
+gg_status enqueue_small_bfs(gg_graph *g, PState *st, const PFront *fr, int32_t *level, int max_iters, int threshold,
+                            int threshold_k) {
+    gg_ctx *ctx = g->ctx;
+    // shared memory above 48 KiB is opt-in (set on the current device)
+    GG_CUDA(ctx, cudaFuncSetAttribute(k_small_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
+    SmallArgs S;
+    S.off = g->off;
+    S.adj = g->adj;
+    S.level = level;
+    S.fr[0] = fr[0];
+    S.fr[1] = fr[1];
+    S.st = st;
+    S.max_iters = max_iters;
+    S.smax = tuning().bin_small_max;
+    S.mmax = tuning().bin_medium_max;
+    S.m = g->m;
+    S.threshold = threshold;
+    S.threshold_k = threshold_k;
+    k_small_bfs<<<kSmallCtas, kSB, kSmallSmem, ctx->stream>>>(S);
+    GG_LAUNCHED(ctx);
+    return GG_OK;
+}
+
+// Levels from a device list of distinct roots as one resident launch.
+gg_status bfs_resident_multi(gg_graph *g, gg_prop *level, const uint32_t *d_roots, uint32_t nroots,
+                             const gg_run_opts &opt, gg_run_stats *stats, int *iters_out) {
+    GG_CHECK(bfs_resident_enqueue(g, level, d_roots, nroots, opt, (PState *)g->pstate));
+    PArgs P;
+    std::memset(&P, 0, sizeof(P));
+    P.force_iter = -1;
+    return persistent_state_read(g, g->pstate, P, stats, iters_out);
+}
+
 gg_status persistent_traverse(gg_graph *g, const gg_emap_desc &d, int level_k, bool start_all, uint32_t root,
                               const gg_run_opts &opt, gg_run_stats *stats, int *iters_out, int force_iter,
                               int force_variant, const uint32_t *d_roots, uint32_t nroots,
@@ -1786,23 +1775,7 @@ gg_status persistent_traverse(gg_graph *g, const gg_emap_desc &d, int level_k, b
     // small frontiers: the cluster kernel, then back to the cooperative one
     // whenever the frontier outgrows it (records accumulate in the state block)
     while (P.small_ok && hs.exit_small) {
-        // shared memory above 48 KiB is opt-in (set on the current device)
-        GG_CUDA(ctx, cudaFuncSetAttribute(k_small_bfs, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem));
-        SmallArgs S;
-        S.off = g->off;
-        S.adj = g->adj;
-        S.level = (int32_t *)P.a;
-        S.fr[0] = P.fr[0];
-        S.fr[1] = P.fr[1];
-        S.st = st;
-        S.max_iters = P.max_iters;
-        S.smax = P.smax;
-        S.mmax = P.mmax;
-        S.m = P.m;
-        S.threshold = P.threshold;
-        S.threshold_k = P.threshold_k;
-        k_small_bfs<<<kSmallCtas, kSB, kSmallSmem, s>>>(S);
-        GG_LAUNCHED(ctx);
+        GG_CHECK(enqueue_small_bfs(g, st, P.fr, (int32_t *)P.a, P.max_iters, P.threshold, P.threshold_k));
         GG_CUDA(ctx, cudaMemcpyAsync(&hs, st, sizeof(PState), cudaMemcpyDeviceToHost, s));
         GG_CUDA(ctx, cudaStreamSynchronize(s));
         if (hs.small_done) break;
@@ -1903,10 +1876,18 @@ gg_status batch_bfs_cc(gg_graph *g, const uint32_t *roots, uint32_t k, gg_prop *
     dc.threshold_k = opt_c.threshold_k;
     dc.variant = GG_VAR_AUTO;
     PArgs P1, P2;
+    std::memset(&P1, 0, sizeof(P1));
+    P1.force_iter = -1;
+    bool resident = false;
+    if (tuning().resident && !r.empty()) GG_CHECK(bfs_resident_prepare(g, &resident));
     auto enqueue_all = [&]() -> gg_status {
-        GG_CHECK(enqueue_bfs_start(g, level, prev1, d_roots, (uint32_t)r.size()));
-        GG_CHECK(persistent_enqueue(g, db, 1, false, 0, opt_b, -1, -1, d_roots, (uint32_t)r.size(), nullptr,
-                                    g->pstate, P1, nullptr, nullptr, merge));
+        if (resident) {
+            GG_CHECK(bfs_resident_enqueue(g, level, d_roots, (uint32_t)r.size(), opt_b, (PState *)g->pstate));
+        } else {
+            GG_CHECK(enqueue_bfs_start(g, level, prev1, d_roots, (uint32_t)r.size()));
+            GG_CHECK(persistent_enqueue(g, db, 1, false, 0, opt_b, -1, -1, d_roots, (uint32_t)r.size(), nullptr,
+                                        g->pstate, P1, nullptr, nullptr, merge));
+        }
         GG_CHECK(enqueue_cc_start(g, label, prev2));
         GG_CHECK(persistent_enqueue(g, dc, 0, true, 0, opt_c, -1, -1, nullptr, 0, nullptr, g->pstate2, P2, nullptr,
                                     nullptr, merge));

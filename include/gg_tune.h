@@ -15,7 +15,9 @@
  * kernels), pr_stream (0 or 1, without effect: one PageRank gather
  * serves all rows), pr_blocks_per_sm (the PageRank kernels' grid cap, 16), persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
  * one device-driven cooperative launch; otherwise one launch per iteration
- * from the host), graph (1, the default: BFS levels run as one CUDA graph
+ * from the host), resident (1, the default: BFS levels run as one resident
+ * cooperative launch where the CUDA graph below would be taken, from many
+ * roots too; 0: not), graph (1, the default: BFS levels run as one CUDA graph
  * whose conditional nodes take each step's push/pull decision on the
  * device; 0: one host round trip per iteration), graph_handoff (32, the
  * default: a graph-driven BFS still running after that many iterations

@@ -265,6 +265,11 @@ __global__ void k_ms_roots(MsArgs A, const uint32_t *roots, int k) {
     A.st->efront = ef;
 }
 
+__global__ void k_ms_pack(const int32_t *level, uint32_t n, int k, int32_t *out) {
+    const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = tid; i < (uint64_t)n * k; i += nth) out[i] = level[i / k * 64 + i % k];
+}
+
 // ---------------------------------------------------------------------------
 // Personalized PageRank, 128 seeds, bfloat16 rows
 // ---------------------------------------------------------------------------
@@ -423,8 +428,9 @@ gg_status gg_msbfs(gg_graph *g, const uint32_t *roots, int k, int32_t *host_leve
     const uint64_t n = g->n;
     // scratch: visited, front, next (8n each), levels (256n), roots, state
     const size_t words = (3 * n + 1) * 8, lev = n * 64 * 4;
+    const size_t pack = host_levels && k < 64 ? n * k * 4 : 0;  // the levels as the caller wants them
     void *base;
-    GG_CHECK(graph_scratch(g, words + lev + 64 * 4 + sizeof(MsState) + 512, &base));
+    GG_CHECK(graph_scratch(g, words + lev + 64 * 4 + sizeof(MsState) + 512 + pack, &base));
     char *p = (char *)base;
     MsArgs A;
     std::memset(&A, 0, sizeof(A));
@@ -477,11 +483,15 @@ gg_status gg_msbfs(gg_graph *g, const uint32_t *roots, int k, int32_t *host_leve
         }
     }
     if (host_levels) {
-        // [n][64] on the device -> [n][k] on the host
-        std::vector<int32_t> tmp(n * 64);
-        GG_CUDA(ctx, cudaMemcpy(tmp.data(), A.level, n * 64 * 4, cudaMemcpyDeviceToHost));
-        for (uint64_t v = 0; v < n; ++v)
-            std::memcpy(host_levels + v * k, tmp.data() + v * 64, k * 4);
+        const int32_t *out = A.level;
+        if (k < 64) {
+            // [n][64] -> [n][k] on the device
+            int32_t *packed = (int32_t *)(st + 1);
+            k_ms_pack<<<bgrid(ctx, n * k), kBB, 0, s>>>(A.level, g->n, k, packed);
+            GG_LAUNCHED(ctx);
+            out = packed;
+        }
+        GG_CHECK(host_download(ctx, host_levels, out, n * k * 4));
     }
     return GG_OK;
 }
@@ -566,14 +576,11 @@ gg_status gg_ppr(gg_graph *g, const uint32_t *seeds, int k, float alpha, int ite
         stats->scanned_edges = (uint64_t)iters * g->m;
     }
     if (host_x) {
-        float *dx = nullptr;
-        GG_CUDA(ctx, cudaMalloc(&dx, n * k * 4));
+        // (the contribution rows are free now: 512 bytes per vertex, k <= 128 floats)
+        float *dx = (float *)c0;
         k_ppr_unpack<<<bgrid(ctx, n * k), kBB, 0, s>>>(x, g->n, k, dx);
-        ctx->launches++;
-        cudaError_t ee = cudaMemcpyAsync(host_x, dx, n * k * 4, cudaMemcpyDeviceToHost, s);
-        if (ee == cudaSuccess) ee = cudaStreamSynchronize(s);
-        cudaFree(dx);
-        if (ee != cudaSuccess) return cuda_error(ctx, ee, "gg_ppr download");
+        GG_LAUNCHED(ctx);
+        GG_CHECK(host_download(ctx, host_x, dx, n * k * 4));
     }
     return GG_OK;
 }

@@ -771,6 +771,7 @@ gg_status gg_ctx_destroy(gg_ctx *ctx) {
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
+    host_stage_free(ctx);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->evk0) cudaEventDestroy(ctx->evk0);
@@ -1217,8 +1218,8 @@ gg_status gg_graph_info(gg_graph *g, uint32_t *n, uint64_t *m, int *symmetric) {
 gg_status gg_graph_download(gg_graph *g, uint64_t *off, uint32_t *adj) {
     if (!g) return GG_ERR_ARG;
     GG_CUDA(g->ctx, cudaStreamSynchronize(g->ctx->stream));
-    if (off) GG_CUDA(g->ctx, cudaMemcpy(off, g->off, ((size_t)g->n + 1) * 8, cudaMemcpyDeviceToHost));
-    if (adj && g->m) GG_CUDA(g->ctx, cudaMemcpy(adj, g->adj, g->m * 4, cudaMemcpyDeviceToHost));
+    if (off) GG_CHECK(host_download(g->ctx, off, g->off, ((size_t)g->n + 1) * 8));
+    if (adj && g->m) GG_CHECK(host_download(g->ctx, adj, g->adj, g->m * 4));
     return GG_OK;
 }
 
@@ -1323,10 +1324,7 @@ gg_status gg_prop_get(gg_prop *p, uint32_t v, void *value) {
 
 gg_status gg_prop_download(gg_prop *p, void *host) {
     if (!p || !host) return GG_ERR_ARG;
-    gg_ctx *ctx = p->g->ctx;
-    GG_CUDA(ctx, cudaMemcpyAsync(host, p->d, (size_t)p->g->n * p->esz, cudaMemcpyDeviceToHost, ctx->stream));
-    GG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return GG_OK;
+    return host_download(p->g->ctx, host, p->d, (size_t)p->g->n * p->esz);
 }
 
 gg_status gg_prop_upload(gg_prop *p, const void *host) {

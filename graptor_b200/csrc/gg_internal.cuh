@@ -62,6 +62,10 @@ struct gg_ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;    // whole-run timing
     cudaEvent_t evk0 = nullptr, evk1 = nullptr;  // traversal-kernel timing
     bool time_kernels = false;                   // record evk0/evk1 around the next traversal kernel
+    // downloads into pageable memory (gg_host.cu): page-locked slots and the
+    // events that mark them filled, created on first use
+    void *stage = nullptr;
+    cudaEvent_t stage_ev[16] = {};
 };
 
 // Frontier counters live on the device in this layout.
@@ -206,6 +210,8 @@ struct gg_prop {
 namespace gg {
 
 size_t dtype_size(gg_dtype t);
+gg_status host_download(gg_ctx *ctx, void *dst, const void *src, size_t bytes);
+void host_stage_free(gg_ctx *ctx);
 gg_status graph_scratch(gg_graph *g, size_t bytes, void **p);
 gg_status frontier_alloc_bins(gg_frontier *f);
 gg_status frontier_alloc_bitmap(gg_frontier *f);

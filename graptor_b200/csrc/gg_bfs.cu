@@ -100,6 +100,7 @@ struct BArgs {
     float gini, sel_x4, sel_x9;
     int K;                                // edges a lane walks alone
     int max_iters;
+    unsigned long long give_up;           // from the fourth step on: stop at a frontier below this (0: never)
     unsigned long long timeout_ns;
     uint32_t smax, mmax;
     int small_ok, small_from;             // small frontiers leave for k_small_bfs
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(kBB, 2) k_bfs_run(BArgs A) {
     while (true) {
         const unsigned long long fv = s_next.nv, fe = s_next.ne;
         const bool push = s_next.push != 0;
-        if (fv == 0 || iter >= A.max_iters) break;
+        if (fv == 0 || iter >= A.max_iters || (iter >= 3 && fv < A.give_up)) break;
         uint32_t *F = A.bits[iter % 3], *O = A.bits[(iter + 1) % 3], *C = A.bits[(iter + 2) % 3];
         if (A.small_ok && push && iter >= A.small_from && fv <= kSmallEnterV && fe <= kSmallEnterE) {
             // the frontier as the binned list that k_small_bfs takes
@@ -599,8 +600,11 @@ __global__ void __launch_bounds__(kBB, 2) k_bfs_run(BArgs A) {
     if (blockIdx.x == 0) {
         if (threadIdx.x == 0) {
             st->iterations = iter;
-            st->reached_v = reached_v;
+            st->reached_v = reached_v + (handed ? 0ull : s_next.nv);  // (a search cut short: its last frontier)
             st->reached_e = reached_e;
+            st->cand_valid = cand_valid;
+            st->cand_cur = cc;
+            st->cand_n[0] = ncand;
             st->t_end = grid::globaltimer();
             st->exit_small = handed;
             st->small_done = !handed;
@@ -754,7 +758,24 @@ gg_status bfs_resident_enqueue(gg_graph *g, gg_prop *level, const uint32_t *d_ro
     return bfs_launch(g, A);
 }
 
-// Levels from one root.  Fills *hs with the run's state.
+// Enqueues at most `steps` levels from one root, fewer where the fourth step
+// or a later one starts from fewer than `give_up` vertices (those of the last
+// frontier have their levels); may be captured.
+gg_status bfs_resident_search(gg_graph *g, gg_prop *level, uint32_t root, int steps, unsigned long long give_up,
+                              PState *st) {
+    gg_run_opts opt;
+    std::memset(&opt, 0, sizeof(opt));
+    opt.threshold = GG_THRESH_DEFAULT;
+    opt.variant = GG_VAR_AUTO;
+    BArgs A;
+    GG_CHECK(bfs_args(g, level, opt, st, A));
+    A.root = root;
+    A.max_iters = std::min(A.max_iters, steps);
+    A.give_up = give_up;
+    return bfs_launch(g, A);
+}
+
+// Levels from one root.
 gg_status bfs_resident(gg_graph *g, gg_prop *level, uint32_t root, const gg_run_opts &opt, gg_run_stats *st,
                        int *iters_out) {
     gg_ctx *ctx = g->ctx;

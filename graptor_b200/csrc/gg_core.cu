@@ -582,6 +582,7 @@ static void graph_free(gg_graph *g) {
     cudaFree(g->kc_state);
     cudaFree(g->items);
     bfs_resident_free(g);
+    cc_resident_free(g);
     cudaFree(g->pstate2);
     for (int i = 0; i < 2; ++i) {
         if (g->copy_done[i]) {

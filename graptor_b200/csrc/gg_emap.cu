@@ -3011,9 +3011,25 @@ gg_status gg_cc(gg_graph *g, const gg_run_opts *o, gg_prop *label, uint32_t *hos
     gg_run_opts opt;
     default_opts(o, &opt, GG_THRESH_FRAC, 5);  // CCv.C:309 emap_step(F, 5)
     if (!label) GG_CHECK(tmp_prop(g, 2, GG_U32, &label));
+    if (st) memset(st, 0, sizeof(*st));
+    bool res = false;
+    GG_CHECK(cc_resident_prepare(g, opt, &res));
+    if (res) {
+        const uint64_t l0 = g->ctx->launches;
+        RunTimer rt(g->ctx);
+        int iters = 0;
+        GG_CHECK(cc_resident(g, label, st, &iters));
+        const double ms = rt.stop();
+        if (st) {
+            st->iterations = iters;
+            st->total_ms = ms;
+            st->kernels = g->ctx->launches - l0;
+        }
+        if (host_label) GG_CHECK(gg_prop_download(label, host_label));
+        return gg_ctx_sync(g->ctx);
+    }
     gg_prop *prev;
     GG_CHECK(tmp_prop(g, 3, GG_U32, &prev));
-    if (st) memset(st, 0, sizeof(*st));
     gg_ctx *ctx = g->ctx;
     uint64_t k0 = ctx->launches;
     RunTimer tm(ctx);

@@ -175,6 +175,7 @@ struct gg_graph {
     void *kc_state = nullptr;  // gg_kcore's resident peel
     void *items = nullptr;     // work items of the resident kernels (gg_items.cuh)
     void *bfs_res = nullptr;   // resident BFS: buffers
+    void *cc_res = nullptr;    // resident CC: buffers
     CandLists cand;               // pull candidate lists (driver runs)
     bool cand_active = false;     // a driver run uses them for its pull steps
     // released frontier buffers, reused in stream order
@@ -245,7 +246,13 @@ gg_status bfs_resident_enqueue(gg_graph *g, gg_prop *level, const uint32_t *d_ro
                                const gg_run_opts &opt, PState *st);
 gg_status bfs_resident_multi(gg_graph *g, gg_prop *level, const uint32_t *d_roots, uint32_t nroots,
                              const gg_run_opts &opt, gg_run_stats *stats, int *iters_out);
+gg_status bfs_resident_search(gg_graph *g, gg_prop *level, uint32_t root, int steps, unsigned long long give_up,
+                              PState *st);
 void bfs_resident_free(gg_graph *g);
+gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok);
+gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *iters_out);
+gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_host);
+void cc_resident_free(gg_graph *g);
 gg_status enqueue_bfs_start(gg_graph *g, gg_prop *level, gg_prop *prev, const uint32_t *d_roots, uint32_t k);
 gg_status enqueue_cc_start(gg_graph *g, gg_prop *label, gg_prop *prev);
 gg_status run_tmp_prop(gg_graph *g, int slot, gg_dtype t, gg_prop **out);
@@ -288,7 +295,8 @@ struct Tuning {
     // per-iteration host round trip): bit 0 BFS levels
     int graph = 1;
     // BFS levels as one resident cooperative launch (gg_bfs.cu) where the
-    // graph-driven run would be taken
+    // graph-driven run would be taken, CC of symmetric graphs as one
+    // (gg_cc.cu) where the device-driven run would
     int resident = 1;
     // graph-driven BFS levels: a run still going after this many iterations
     // (a high-diameter graph: many small frontiers, where the graph's

@@ -31,6 +31,7 @@
 #include "gg_batch.h"
 #include "gg_mlp.cuh"
 #include "gg_persist.cuh"
+#include "gg_uf.cuh"
 
 #include <cooperative_groups.h>
 namespace cg = cooperative_groups;
@@ -470,36 +471,7 @@ __device__ void phase_fused_run(const PArgs &P, const POp<R> &op, const PFront &
     p_flush(O, nv, ne, sc);
 }
 
-// ---- CC by min-id hooking -------------------------------------------------------
-// label[] is a forest: every label is the id of a vertex of the same
-// component and never above the vertex's own id, so following labels ends at
-// a vertex labelled with itself (a root).  Hooking an edge's two roots, the
-// larger under the smaller (compare-and-swap on the larger root), and
-// repeating until they agree merges the trees; the root of a component is
-// then its minimum id, the CCv label.  Finds halve paths with plain stores
-// (a label only ever moves to an ancestor, so racing stores stay valid).
-__device__ __forceinline__ uint32_t uf_find(uint32_t *lab, uint32_t x) {
-    for (int guard = 0; guard < (1 << 26); ++guard) {  // a chain of n links at most
-        const uint32_t p = ldcg(lab + x);
-        if (p == x) return x;
-        const uint32_t gp = ldcg(lab + p);
-        if (gp != p) lab[x] = gp;
-        x = gp;
-    }
-    return x;
-}
-
-__device__ __forceinline__ void uf_hook(uint32_t *lab, uint32_t u, uint32_t v) {
-    uint32_t ru = uf_find(lab, u), rv = uf_find(lab, v);
-    for (int guard = 0; ru != rv && guard < (1 << 26); ++guard) {
-        const uint32_t lo = ru < rv ? ru : rv, hi = ru ^ rv ^ lo;
-        const uint32_t old = atomicCAS(lab + hi, hi, lo);
-        if (old == hi) break;
-        ru = uf_find(lab, old);
-        rv = uf_find(lab, lo);
-    }
-}
-
+// ---- CC by min-id hooking (gg_uf.cuh) ----------------------------------------
 __device__ void phase_hook(const PArgs &P) {
     uint32_t *lab = (uint32_t *)P.a;
     const uint32_t lane = threadIdx.x & 31u;
@@ -569,18 +541,6 @@ __device__ void phase_hook_rest(const PArgs &P) {
             for (uint64_t e = bj + lane; e < ej; e += 32) uf_hook(lab, uj, __ldg(P.adj + e));
         }
     }
-}
-
-// The root of x without path halving: in the final pass every vertex's
-// entry is written once, by its own thread, with its root; a halving store
-// from another thread's walk could land after it and leave a non-root there.
-__device__ __forceinline__ uint32_t uf_root(const uint32_t *lab, uint32_t x) {
-    for (int guard = 0; guard < (1 << 26); ++guard) {  // a chain of n links at most
-        const uint32_t p = ldcg(lab + x);
-        if (p == x) return x;
-        x = p;
-    }
-    return x;
 }
 
 __device__ void phase_hook_finish(const PArgs &P) {
@@ -1878,7 +1838,10 @@ gg_status batch_bfs_cc(gg_graph *g, const uint32_t *roots, uint32_t k, gg_prop *
     PArgs P1, P2;
     std::memset(&P1, 0, sizeof(P1));
     P1.force_iter = -1;
-    bool resident = false;
+    std::memset(&P2, 0, sizeof(P2));
+    P2.force_iter = -1;
+    bool resident = false, cc_res = false;
+    GG_CHECK(cc_resident_prepare(g, opt_c, &cc_res));
     if (tuning().resident && !r.empty()) GG_CHECK(bfs_resident_prepare(g, &resident));
     auto enqueue_all = [&]() -> gg_status {
         if (resident) {
@@ -1888,9 +1851,13 @@ gg_status batch_bfs_cc(gg_graph *g, const uint32_t *roots, uint32_t k, gg_prop *
             GG_CHECK(persistent_enqueue(g, db, 1, false, 0, opt_b, -1, -1, d_roots, (uint32_t)r.size(), nullptr,
                                         g->pstate, P1, nullptr, nullptr, merge));
         }
-        GG_CHECK(enqueue_cc_start(g, label, prev2));
-        GG_CHECK(persistent_enqueue(g, dc, 0, true, 0, opt_c, -1, -1, nullptr, 0, nullptr, g->pstate2, P2, nullptr,
-                                    nullptr, merge));
+        if (cc_res) {
+            GG_CHECK(cc_resident_enqueue(g, label, (PState *)g->pstate2, false));
+        } else {
+            GG_CHECK(enqueue_cc_start(g, label, prev2));
+            GG_CHECK(persistent_enqueue(g, dc, 0, true, 0, opt_c, -1, -1, nullptr, 0, nullptr, g->pstate2, P2,
+                                        nullptr, nullptr, merge));
+        }
         return GG_OK;
     };
     RunTimerP tm(ctx);

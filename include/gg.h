@@ -405,7 +405,12 @@ GG_API gg_status gg_bfs_parent(gg_graph *g, uint32_t root, const gg_run_opts *o,
  * the first step (PUSH_ZERO, bench/CCv.C:365-388: fewer than n/10 vertices
  * labelled 0) and, where it holds, finish the run by hooking every edge's
  * endpoints' roots, the larger under the smaller (labels unchanged: the
- * minimum id of each component); otherwise label propagation continues. */
+ * minimum id of each component); otherwise label propagation continues.
+ * By default a symmetric graph's components come from a short search from its
+ * vertex of largest degree and hooking of what that did not reach (knob
+ * resident); st then holds two records, the second a GG_VAR_HOOK where the
+ * labels pass the road-network test.  Runs that collect per-step records, fix
+ * a variant or take another threshold than DEFAULT or FRAC propagate labels. */
 GG_API gg_status gg_cc(gg_graph *g, const gg_run_opts *o, gg_prop *label, uint32_t *host_label,
                        gg_run_stats *st);
 /* k-core decomposition (KC_bucket, bench/KC_bucket.C:107-420): coreness[v] =

@@ -17,7 +17,7 @@
  * one device-driven cooperative launch; otherwise one launch per iteration
  * from the host), resident (1, the default: BFS levels run as one resident
  * cooperative launch where the CUDA graph below would be taken, from many
- * roots too; 0: not), graph (1, the default: BFS levels run as one CUDA graph
+ * roots too, and CC of symmetric graphs as two; 0: not), graph (1, the default: BFS levels run as one CUDA graph
  * whose conditional nodes take each step's push/pull decision on the
  * device; 0: one host round trip per iteration), graph_handoff (32, the
  * default: a graph-driven BFS still running after that many iterations

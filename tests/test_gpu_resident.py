@@ -1,4 +1,4 @@
-"""The resident BFS against the oracle's levels and the other drivers' records:
+"""The resident BFS and CC against the oracle and the other drivers' records:
 rows at the item boundaries (32, 256 and 4096 edges), vertex counts that are
 no multiple of a word or of 16 bytes of bits, pushes after pulls, frontiers
 too large to list, hand-overs to the one-cluster kernel and back, and many
@@ -97,4 +97,44 @@ def test_resident_many_roots(ctx, knobs, kind, k):
     assert np.array_equal(gg.bfs_level_multi(g, roots), want)
     if k == 1:
         assert np.array_equal(want, O.bfs_level(og, int(roots[0])))
+    g.close()
+
+
+def cc_graph(kind):
+    rng = np.random.default_rng(7)
+    if kind == "core_and_tail":
+        # a dense core that the search reaches at once, and a path whose small
+        # ids (0 at its far end) are farther than the search goes
+        core = [(int(a), int(b)) for a, b in rng.integers(1000, 4000, (30000, 2)) if a != b]
+        path = [(i, i + 1) for i in range(60)] + [(60, 1500)]
+        return O.from_edges(4100, core + path)
+    if kind == "giant_without_0":
+        # vertex 0 in a small component; stars of 257 and 3000 leaves (rows
+        # above the heavy-row threshold) outside the giant one
+        core = [(int(a), int(b)) for a, b in rng.integers(5000, 13000, (60000, 2)) if a != b]
+        stars = [(10, 20 + i) for i in range(257)] + [(15, 600 + i) for i in range(3000)]
+        return O.from_edges(13100, core + stars + [(0, 4), (4, 1)])
+    if kind == "many":
+        # no giant component: stars, paths and cliques of growing size
+        edges, at = [], 3
+        for k in range(1, 40):
+            edges += [(at + k, at + j) for j in range(k)] + [(at + k + j, at + k + j + 1) for j in range(37 * k)]
+            at += 38 * k + 2
+        edges += [(at, at + 1 + j) for j in range(1500)] + [(at + 2000, at + 1 + 2 * j) for j in range(700)]
+        return O.from_edges(at + 2010, edges)
+    return O.from_edges(77, [])
+
+
+@pytest.mark.parametrize("kind", ["core_and_tail", "giant_without_0", "many", "edgeless"])
+def test_resident_cc_exact(ctx, knobs, kind):
+    og = cc_graph(kind)
+    g = ctx.upload(og.off, og.adj)
+    want = O.cc(og)
+    for res in (0, 1):
+        gg.tuning_set("resident", res)
+        for _ in range(3):
+            assert np.array_equal(g.cc(), want), (kind, res)
+    lv, lb, _, _ = gg.batch_bfs_cc(g, np.array([0, 5], dtype=np.uint32))
+    assert np.array_equal(lb, want)
+    assert np.array_equal(lv, np.minimum(O.bfs_level(og, 0), O.bfs_level(og, 5)))
     g.close()

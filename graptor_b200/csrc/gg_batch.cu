@@ -279,13 +279,17 @@ struct PprArgs {
     const uint64_t *in_off, *off;
     const uint32_t *in_adj;
     uint32_t n;
-    const uint2 *cin;   // [n] rows of 128 bf16 (uint2 = 4 bf16 per lane)
-    uint2 *cout;        // next contributions
+    const uint2 *cin;   // [n] rows of 4 L bf16 (uint2 = 4 bf16 per lane)
+    uint2 *cout;        // next contributions; null in the last iteration
     uint2 *xout;        // ranks (bf16), written by the last iteration only (else null)
     const uint32_t *seeds;  // [128]
     float alpha;
     HeavyRows H;
-    float4 *partial;    // [nchunks][32] float4 per lane
+    float4 *partial;    // [nchunks][L] float4 per lane
+    uint32_t *arrived;  // [nheavy] chunks of the row that are done; wraps to 0
+    uint32_t tickets;   // of the chunks, 32 / L each, then of the light rows, kPprRows<L> each
+    uint32_t *ticket;   // this iteration's; the next one's is set to 0
+    uint32_t *next_ticket;
 };
 
 __device__ __forceinline__ void bf4_acc(uint2 v, float4 &a) {
@@ -302,97 +306,285 @@ __device__ __forceinline__ uint2 f4_to_bf4(float4 f) {
     return r;
 }
 
-// x = alpha*e_seed + (1-alpha)*acc; c = x/deg; written as bf16 rows
+// x = alpha*e_seed + (1-alpha)*acc; c = x/deg; written as bf16 rows (a
+// contribution only where the vertex has an out-edge by which it is read)
+template <int L>
 __device__ __forceinline__ void ppr_finish(const PprArgs &A, uint32_t d, float4 acc, uint32_t lane) {
+    const uint4 seed = __ldg((const uint4 *)A.seeds + lane);
+    const uint64_t deg = A.off[d + 1] - A.off[d];
     const float b = 1.0f - A.alpha;
     float4 x = make_float4(b * acc.x, b * acc.y, b * acc.z, b * acc.w);
-    const uint32_t s0 = lane * 4;
-    if (A.seeds[s0] == d) x.x += A.alpha;
-    if (A.seeds[s0 + 1] == d) x.y += A.alpha;
-    if (A.seeds[s0 + 2] == d) x.z += A.alpha;
-    if (A.seeds[s0 + 3] == d) x.w += A.alpha;
-    const uint64_t deg = A.off[d + 1] - A.off[d];
-    const float inv = deg ? 1.0f / (float)deg : 0.0f;
-    if (A.xout) A.xout[(uint64_t)d * 32 + lane] = f4_to_bf4(x);
-    A.cout[(uint64_t)d * 32 + lane] = f4_to_bf4(make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv));
+    if (seed.x == d) x.x += A.alpha;
+    if (seed.y == d) x.y += A.alpha;
+    if (seed.z == d) x.z += A.alpha;
+    if (seed.w == d) x.w += A.alpha;
+    if (A.xout) A.xout[(uint64_t)d * L + lane] = f4_to_bf4(x);
+    if (A.cout && deg) {
+        const float inv = 1.0f / (float)deg;
+        A.cout[(uint64_t)d * L + lane] = f4_to_bf4(make_float4(x.x * inv, x.y * inv, x.z * inv, x.w * inv));
+    }
 }
 
-// light rows: a warp per row
-__global__ void __launch_bounds__(kBB) k_ppr_light(PprArgs A) {
+// One launch per iteration.  What bounds it: every edge reads a row of cin,
+// and an SM receives about one 32-byte sector per clock from L2 (a row of 128
+// seeds is eight; 9.1 TB/s over the chip where L1 holds none of them, which
+// uniform ids reach).
+//   * A row is as wide as its seeds need: 4 per lane over L = 4, 8, 16 or 32
+//     lanes for up to 16, 32, 64 or 128 seeds.
+//   * Warps draw tickets, first the chunks of the heavy rows and then small
+//     sets of light rows, so that neither waits for a launch of its own; the
+//     last chunk of a row to be done adds the row's partial sums.  The sums'
+//     order is that of the edges within a row or chunk and of the chunks
+//     within a row, whatever L.
+//   * Ids are loaded for a whole batch at once and one batch ahead; 16 rows
+//     are in flight (chunks of 1024 edges are a chain of that many fewer
+//     round trips; 8 rows in flight and 5 CTAs per SM: R-MAT 18 5.10 ms, ER
+//     4.77 ms, R-MAT 10 0.79 ms).
+//   * A vertex without out-edges has no contribution to write, nor has any
+//     vertex in the last iteration.
+// 20 iterations, before (a warp per row, 4 rows in flight, rows of 128 seeds
+// whatever their number, three launches) -> after: 128 seeds on R-MAT 18 x 16
+// 8.49 -> 4.89 ms, R-MAT 10 1.07 -> 0.71, ER 2^18 x 32 4.99 -> 5.05; 50 seeds
+// on R-MAT 17 4.34 -> 2.02; 5 seeds on R-MAT 18 6.72 -> 2.04; 29 and 9 seeds
+// on directed ER 200001 x 12 2.09 -> 0.79 and 2.11 -> 0.54.
+constexpr int kPprBlock = 256;
+constexpr uint32_t kPprFlight = 16;
+// light rows per ticket
+template <int L> constexpr uint32_t kPprRows = L == 32 ? 8 : 4 * (32 / L);
+
+// Rows as wide as a warp.
+__global__ void __launch_bounds__(kPprBlock, 4) k_ppr_wide(PprArgs A) {
+    constexpr uint32_t FULL = 0xffffffffu, F = kPprFlight, kSkip = 0xffffffffu;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * kBB) >> 5;
-    for (uint64_t d = ((uint64_t)blockIdx.x * kBB + threadIdx.x) >> 5; d < A.n; d += nw) {
-        const uint64_t beg = A.in_off[d], end = A.in_off[d + 1];
-        if (end - beg > A.H.T) continue;  // heavy: chunked kernels
-        float4 acc = make_float4(0, 0, 0, 0);
-        uint64_t e = beg;
-        for (; e + 4 <= end; e += 4) {  // four rows in flight
-            const uint32_t u0 = __ldg(A.in_adj + e), u1 = __ldg(A.in_adj + e + 1), u2 = __ldg(A.in_adj + e + 2),
-                           u3 = __ldg(A.in_adj + e + 3);
-            const uint2 r0 = A.cin[(uint64_t)u0 * 32 + lane], r1 = A.cin[(uint64_t)u1 * 32 + lane],
-                        r2 = A.cin[(uint64_t)u2 * 32 + lane], r3 = A.cin[(uint64_t)u3 * 32 + lane];
-            bf4_acc(r0, acc);
-            bf4_acc(r1, acc);
-            bf4_acc(r2, acc);
-            bf4_acc(r3, acc);
+    const uint2 *cin = A.cin + lane;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *A.next_ticket = 0;
+    uint32_t t = (blockIdx.x * kPprBlock + threadIdx.x) >> 5, next = 0;
+    for (; t < A.tickets; t = __shfl_sync(FULL, next, 0)) {
+        if (lane == 0) next = gridDim.x * (kPprBlock / 32) + atomicAdd(A.ticket, 1u);
+        // lane r < rows holds the edges of the ticket's row d0 + r (kSkip: a
+        // heavy row, done by its chunks): one chunk, or the light rows
+        uint32_t d0, rows, len = kSkip;
+        const uint32_t *ids;
+        if (t < A.H.nchunks) {
+            const uint32_t h = A.H.crow[t];
+            d0 = A.H.v[h];
+            rows = 1;
+            const uint64_t e0 = A.in_off[d0] + (t - A.H.first[h]) * A.H.CH;
+            len = (uint32_t)min((uint64_t)A.H.CH, A.in_off[d0 + 1] - e0);
+            ids = A.in_adj + e0;
+        } else {
+            d0 = (t - (uint32_t)A.H.nchunks) * kPprRows<32>;
+            rows = min(A.n - d0, kPprRows<32>);
+            const uint64_t beg = __ldg(A.in_off + d0 + min(lane, rows)), end = __shfl_down_sync(FULL, beg, 1);
+            if (lane < rows && end - beg <= A.H.T) len = (uint32_t)(end - beg);
+            ids = A.in_adj + beg;
         }
-        for (; e < end; ++e) bf4_acc(A.cin[(uint64_t)__ldg(A.in_adj + e) * 32 + lane], acc);
-        ppr_finish(A, (uint32_t)d, acc, lane);
-    }
-}
-
-// heavy rows: a warp per chunk, float partials
-__global__ void __launch_bounds__(kBB) k_ppr_heavy(PprArgs A) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * kBB) >> 5;
-    for (uint64_t c = ((uint64_t)blockIdx.x * kBB + threadIdx.x) >> 5; c < A.H.nchunks; c += nw) {
-        const uint32_t h = A.H.crow[c];
-        const uint32_t v = A.H.v[h];
-        const uint64_t e0 = A.in_off[v] + (c - A.H.first[h]) * A.H.CH;
-        const uint64_t e1 = min(e0 + A.H.CH, A.in_off[v + 1]);
-        float4 acc = make_float4(0, 0, 0, 0);
-        for (uint64_t e = e0; e < e1; ++e) bf4_acc(A.cin[(uint64_t)__ldg(A.in_adj + e) * 32 + lane], acc);
-        A.partial[c * 32 + lane] = acc;
-    }
-}
-
-__global__ void __launch_bounds__(kBB) k_ppr_heavy_finish(PprArgs A) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nw = ((uint64_t)gridDim.x * kBB) >> 5;
-    for (uint64_t h = ((uint64_t)blockIdx.x * kBB + threadIdx.x) >> 5; h < A.H.nheavy; h += nw) {
-        float4 acc = make_float4(0, 0, 0, 0);
-        for (uint64_t c = A.H.first[h]; c < A.H.first[h + 1]; ++c) {
-            const float4 p = A.partial[c * 32 + lane];
-            acc.x += p.x;
-            acc.y += p.y;
-            acc.z += p.z;
-            acc.w += p.w;
+        for (uint32_t r = 0; r < rows; ++r) {
+            const uint32_t deg = __shfl_sync(FULL, len, r);
+            const uint32_t *at = (const uint32_t *)__shfl_sync(FULL, (unsigned long long)ids, r) + lane;
+            if (deg == kSkip) continue;
+            float4 acc = make_float4(0, 0, 0, 0);
+            uint32_t nid = lane < deg ? __ldg(at) : 0u;
+            for (uint32_t e = 0; e < deg; e += 32) {
+                const uint32_t id = nid;
+                at += 32;
+                nid = e + 32 + lane < deg ? __ldg(at) : 0u;
+                const uint32_t cnt = min(deg - e, 32u);
+                for (uint32_t j = 0; j < cnt; j += F) {
+                    uint2 row[F];
+                    if (j + F <= cnt) {
+#pragma unroll
+                        for (uint32_t u = 0; u < F; ++u)
+                            row[u] = __ldg(cin + (uint64_t)__shfl_sync(FULL, id, j + u) * 32);
+#pragma unroll
+                        for (uint32_t u = 0; u < F; ++u) bf4_acc(row[u], acc);
+                    } else {
+#pragma unroll
+                        for (uint32_t u = 0; u < F - 1; ++u)
+                            if (j + u < cnt) row[u] = __ldg(cin + (uint64_t)__shfl_sync(FULL, id, j + u) * 32);
+#pragma unroll
+                        for (uint32_t u = 0; u < F - 1; ++u)
+                            if (j + u < cnt) bf4_acc(row[u], acc);
+                    }
+                }
+            }
+            if (t < A.H.nchunks) {
+                const uint32_t h = A.H.crow[t];
+                const uint32_t c0 = (uint32_t)A.H.first[h], c1 = (uint32_t)A.H.first[h + 1];
+                if (c1 - c0 > 1) {  // the last chunk of the row to be done adds them up, in their order
+                    __stcg(A.partial + (uint64_t)t * 32 + lane, acc);
+                    __threadfence();
+                    __syncwarp();
+                    uint32_t before = 0;
+                    if (lane == 0) before = atomicInc(A.arrived + h, c1 - c0 - 1);
+                    if (__shfl_sync(FULL, before, 0) != c1 - c0 - 1) break;
+                    __threadfence();
+                    acc = make_float4(0, 0, 0, 0);
+                    for (uint32_t c = c0; c < c1; ++c) {
+                        const float4 p = __ldcg(A.partial + (uint64_t)c * 32 + lane);
+                        acc.x += p.x;
+                        acc.y += p.y;
+                        acc.z += p.z;
+                        acc.w += p.w;
+                    }
+                }
+            }
+            ppr_finish<32>(A, d0 + r, acc, lane);
         }
-        ppr_finish(A, A.H.v[h], acc, lane);
     }
 }
 
-__global__ void k_ppr_init(uint2 *c, uint2 *x, const uint64_t *off, uint32_t n, const uint32_t *seeds) {
+// The same for rows of L < 32 lanes: the warp's G = 32 / L groups of lanes
+// work on one destination each, in step (apart, their loads would wait for one
+// another: 5 seeds on R-MAT 18 3.70 ms).
+template <int L>
+__global__ void __launch_bounds__(kPprBlock, 3) k_ppr_narrow(PprArgs A) {
+    constexpr uint32_t FULL = 0xffffffffu, G = 32 / L, F = kPprFlight;
+    constexpr uint32_t IDS = L < F ? F / L : 1, BATCH = IDS * L;
+    constexpr uint32_t kSkip = 0xffffffffu;
+    const uint32_t wl = threadIdx.x & 31u, lane = wl & (L - 1), grp = wl / L;
+    const uint2 *cin = A.cin + lane;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *A.next_ticket = 0;
+    const uint32_t nct = ((uint32_t)A.H.nchunks + G - 1) / G;
+    uint32_t t = (blockIdx.x * kPprBlock + threadIdx.x) >> 5, next = 0;
+    for (; t < A.tickets; t = __shfl_sync(FULL, next, 0)) {
+        if (wl == 0) next = gridDim.x * (kPprBlock / 32) + atomicAdd(A.ticket, 1u);
+        // lane r holds the edges of the ticket's row r (kSkip: none, or a
+        // heavy row, done by its chunks)
+        const bool chunk = t < nct;
+        uint32_t d = 0, rows = G, len = kSkip;
+        const uint32_t *ids = A.in_adj;
+        if (chunk) {
+            const uint32_t c = t * G + wl;
+            if (wl < G && c < A.H.nchunks) {
+                const uint32_t h = A.H.crow[c];
+                d = A.H.v[h];
+                const uint64_t e0 = A.in_off[d] + (c - A.H.first[h]) * A.H.CH;
+                len = (uint32_t)min((uint64_t)A.H.CH, A.in_off[d + 1] - e0);
+                ids += e0;
+            }
+        } else {
+            rows = kPprRows<L>;
+            const uint64_t at = (uint64_t)(t - nct) * kPprRows<L> + wl;
+            d = (uint32_t)at;
+            if (wl < rows && at < A.n) {
+                const uint64_t beg = __ldg(A.in_off + at), end = __ldg(A.in_off + at + 1);
+                if (end - beg <= A.H.T) len = (uint32_t)(end - beg);
+                ids += beg;
+            }
+        }
+        for (uint32_t r = grp; r < rows; r += G) {
+            uint32_t deg = __shfl_sync(FULL, len, r);
+            const bool act = deg != kSkip;
+            const uint32_t *at = (const uint32_t *)__shfl_sync(FULL, (unsigned long long)ids, r) + lane;
+            if (!act) deg = 0;
+            const uint32_t longest = __reduce_max_sync(FULL, deg);
+            float4 acc = make_float4(0, 0, 0, 0);
+            uint32_t nid[IDS];
+#pragma unroll
+            for (uint32_t i = 0; i < IDS; ++i) nid[i] = i * L + lane < deg ? __ldg(at + i * L) : 0u;
+            for (uint32_t e = 0; e < longest; e += BATCH) {
+                uint32_t id[IDS];
+                at += BATCH;
+#pragma unroll
+                for (uint32_t i = 0; i < IDS; ++i) {
+                    id[i] = nid[i];
+                    nid[i] = e + BATCH + i * L + lane < deg ? __ldg(at + i * L) : 0u;
+                }
+                const uint32_t cnt = e < deg ? min(deg - e, BATCH) : 0u;
+                const uint32_t steps = min(longest - e, BATCH);
+#pragma unroll 1
+                for (uint32_t j = 0; j < steps; j += F) {
+                    uint2 row[F];
+#pragma unroll
+                    for (uint32_t u = 0; u < F; ++u) {
+                        const uint32_t v = __shfl_sync(FULL, id[IDS == 1 ? 0 : u / L], IDS == 1 ? j + u : u % L, L);
+                        if (j + u < cnt) row[u] = __ldg(cin + (uint64_t)v * L);
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < F; ++u)
+                        if (j + u < cnt) bf4_acc(row[u], acc);
+                }
+            }
+            bool done = act;
+            if (chunk) {  // the last chunk of a row to be done adds them up, in their order
+                const uint32_t c = t * G + grp;
+                uint32_t h = 0, c0 = 0, c1 = 0, before = 0;
+                if (act) {
+                    h = A.H.crow[c];
+                    c0 = (uint32_t)A.H.first[h];
+                    c1 = (uint32_t)A.H.first[h + 1];
+                }
+                const bool several = c1 - c0 > 1;
+                if (several) __stcg(A.partial + (uint64_t)c * L + lane, acc);
+                __threadfence();
+                __syncwarp();
+                if (several && lane == 0) before = atomicInc(A.arrived + h, c1 - c0 - 1);
+                before = __shfl_sync(FULL, before, 0, L);
+                if (several) {
+                    done = before == c1 - c0 - 1;
+                    __threadfence();
+                    if (done) acc = make_float4(0, 0, 0, 0);
+                    for (c0 = done ? c0 : c1; c0 < c1; ++c0) {
+                        const float4 p = __ldcg(A.partial + (uint64_t)c0 * L + lane);
+                        acc.x += p.x;
+                        acc.y += p.y;
+                        acc.z += p.z;
+                        acc.w += p.w;
+                    }
+                }
+            }
+            const uint32_t dr = __shfl_sync(FULL, d, r);
+            if (done) ppr_finish<L>(A, dr, acc, lane);
+        }
+    }
+}
+
+// contributions of the seeds' own rows (x too, where no iteration writes it)
+// and the counters of the first iteration
+__global__ void k_ppr_init(uint2 *c, uint2 *x, const uint64_t *off, uint32_t n, int L, const uint32_t *seeds,
+                           uint32_t *counters, uint64_t ncounters) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = tid; i < (uint64_t)n * 32; i += nth) {
-        const uint32_t d = (uint32_t)(i / 32), lane = (uint32_t)(i % 32);
-        float4 xv = make_float4(seeds[lane * 4] == d, seeds[lane * 4 + 1] == d, seeds[lane * 4 + 2] == d,
-                                seeds[lane * 4 + 3] == d);
+    for (uint64_t i = tid; i < ncounters; i += nth) counters[i] = 0;
+    const uint4 seed = __ldg((const uint4 *)seeds + tid % L);  // nth is a multiple of L
+    for (uint64_t i = tid; i < (uint64_t)n * L; i += nth) {
+        const uint32_t d = (uint32_t)(i / L);
+        float4 xv = make_float4(seed.x == d, seed.y == d, seed.z == d, seed.w == d);
         const uint64_t deg = off[d + 1] - off[d];
         const float inv = deg ? 1.0f / (float)deg : 0.0f;
-        x[i] = f4_to_bf4(xv);
+        if (x) x[i] = f4_to_bf4(xv);
         c[i] = f4_to_bf4(make_float4(xv.x * inv, xv.y * inv, xv.z * inv, xv.w * inv));
     }
 }
 
-__global__ void k_ppr_unpack(const uint2 *x, uint32_t n, int k, float *out) {
+__global__ void k_ppr_unpack(const uint2 *x, uint32_t n, int L, int k, float *out) {
     const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, nth = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = tid; i < (uint64_t)n * k; i += nth) {
         const uint64_t d = i / k;
         const uint32_t s = (uint32_t)(i % k);
-        const uint2 r = x[d * 32 + s / 4];
+        const uint2 r = x[d * L + s / 4];
         const uint32_t word = (s & 2) ? r.y : r.x;
         out[i] = __uint_as_float((s & 1) ? (word & 0xFFFF0000u) : (word << 16));
+    }
+}
+
+template <int L>
+static void ppr_run(gg_ctx *ctx, PprArgs A, uint2 *c0, uint2 *c1, uint2 *x, uint32_t *counters, int iters) {
+    void (*step)(PprArgs);
+    if constexpr (L == 32) step = k_ppr_wide;
+    else step = k_ppr_narrow<L>;
+    constexpr uint32_t G = 32 / L;
+    A.tickets = (uint32_t)((A.H.nchunks + G - 1) / G + ((uint64_t)A.n + kPprRows<L> - 1) / kPprRows<L>);
+    const unsigned grid = (unsigned)std::min<uint64_t>(
+        (uint64_t)ctx->sm_count * resident_ctas((const void *)step, kPprBlock), ((uint64_t)A.tickets + 7) / 8);
+    for (int it = 0; it < iters; ++it) {
+        A.cin = (it & 1) ? c1 : c0;
+        A.cout = it + 1 == iters ? nullptr : (it & 1) ? c0 : c1;
+        A.xout = it + 1 == iters ? x : nullptr;  // only the ranks of the last iteration are kept
+        A.ticket = counters + (it & 1);
+        A.next_ticket = counters + (~it & 1);
+        step<<<grid, kPprBlock, 0, ctx->stream>>>(A);
+        ctx->launches++;
     }
 }
 
@@ -504,14 +696,16 @@ gg_status gg_ppr(gg_graph *g, const uint32_t *seeds, int k, float alpha, int ite
         if (seeds[i] >= g->n) return set_error(ctx, GG_ERR_ARG, "gg_ppr: seed out of range");
     cudaStream_t s = ctx->stream;
     const uint64_t n = g->n;
-    const size_t row = 256;  // 128 bf16
-    const size_t part = (g->heavy.nchunks + 1) * 32 * sizeof(float4);
+    const int L = k <= 16 ? 4 : k <= 32 ? 8 : k <= 64 ? 16 : 32;  // lanes of a row, 4 seeds each
+    const size_t row = (size_t)L * 8;
+    const size_t part = (g->heavy.nchunks + 1) * L * sizeof(float4);
+    const uint64_t ncounters = g->heavy.nheavy + 2;
     void *base;
-    GG_CHECK(graph_scratch(g, 3 * n * row + part + 512 + 1024, &base));
+    GG_CHECK(graph_scratch(g, 3 * n * row + part + 512 + ncounters * 4, &base));
     char *p = (char *)base;
     uint2 *c0 = (uint2 *)p, *c1 = (uint2 *)(p + n * row), *x = (uint2 *)(p + 2 * n * row);
     float4 *partial = (float4 *)(p + 3 * n * row);
-    uint32_t *dseeds = (uint32_t *)(p + 3 * n * row + part);
+    uint32_t *dseeds = (uint32_t *)(p + 3 * n * row + part), *counters = dseeds + kPprSeeds;
     std::vector<uint32_t> sd(kPprSeeds, 0xFFFFFFFFu);  // unused slots match no vertex
     std::memcpy(sd.data(), seeds, k * 4);
     GG_CUDA(ctx, cudaMemcpyAsync(dseeds, sd.data(), kPprSeeds * 4, cudaMemcpyHostToDevice, s));
@@ -526,47 +720,18 @@ gg_status gg_ppr(gg_graph *g, const uint32_t *seeds, int k, float alpha, int ite
     A.alpha = alpha;
     A.H = g->heavy;
     A.partial = partial;
-    const unsigned gl = (unsigned)(ctx->sm_count * resident_ctas((const void *)k_ppr_light, kBB));
-    const unsigned gh = (unsigned)(ctx->sm_count * resident_ctas((const void *)k_ppr_heavy, kBB));
-    // capture the iteration loop once (on a private stream), then run
-    // init + the graph on the context stream between the timing events
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    cudaStream_t cs;
-    GG_CUDA(ctx, cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
-    cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
-    for (int it = 0; it < iters && e == cudaSuccess; ++it) {
-        A.cin = (it & 1) ? c1 : c0;
-        A.cout = (it & 1) ? c0 : c1;
-        A.xout = it + 1 == iters ? x : nullptr;  // only the ranks of the last iteration are kept
-        k_ppr_light<<<gl, kBB, 0, cs>>>(A);
-        if (A.H.nchunks) {
-            k_ppr_heavy<<<gh, kBB, 0, cs>>>(A);
-            k_ppr_heavy_finish<<<bgrid(ctx, (uint64_t)A.H.nheavy * 32), kBB, 0, cs>>>(A);
-        }
-        ctx->launches += A.H.nchunks ? 3 : 1;
-    }
-    if (e == cudaSuccess) {
-        e = cudaStreamEndCapture(cs, &graph);
-    } else {
-        cudaGraph_t junk = nullptr;
-        cudaStreamEndCapture(cs, &junk);
-        if (junk) cudaGraphDestroy(junk);
-    }
-    if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-    if (e == cudaSuccess) e = cudaEventRecord(ctx->ev0, s);
-    if (e == cudaSuccess) {
-        k_ppr_init<<<bgrid(ctx, n * 32), kBB, 0, s>>>(c0, x, g->off, g->n, dseeds);
-        ctx->launches++;
-        e = cudaGetLastError();
-    }
-    if (e == cudaSuccess && iters) e = cudaGraphLaunch(exec, s);
-    if (e == cudaSuccess) e = cudaEventRecord(ctx->ev1, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
-    cudaStreamDestroy(cs);
-    if (e != cudaSuccess) return cuda_error(ctx, e, "gg_ppr");
+    A.arrived = counters + 2;
+    GG_CUDA(ctx, cudaEventRecord(ctx->ev0, s));
+    k_ppr_init<<<bgrid(ctx, n * L), kBB, 0, s>>>(c0, iters ? nullptr : x, g->off, g->n, L, dseeds, counters,
+                                                 ncounters);
+    GG_LAUNCHED(ctx);
+    if (L == 4) ppr_run<4>(ctx, A, c0, c1, x, counters, iters);
+    else if (L == 8) ppr_run<8>(ctx, A, c0, c1, x, counters, iters);
+    else if (L == 16) ppr_run<16>(ctx, A, c0, c1, x, counters, iters);
+    else ppr_run<32>(ctx, A, c0, c1, x, counters, iters);
+    GG_CUDA(ctx, cudaGetLastError());
+    GG_CUDA(ctx, cudaEventRecord(ctx->ev1, s));
+    GG_CUDA(ctx, cudaStreamSynchronize(s));
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
         float ms = 0;
@@ -576,9 +741,9 @@ gg_status gg_ppr(gg_graph *g, const uint32_t *seeds, int k, float alpha, int ite
         stats->scanned_edges = (uint64_t)iters * g->m;
     }
     if (host_x) {
-        // (the contribution rows are free now: 512 bytes per vertex, k <= 128 floats)
+        // (the contribution rows are free now: 16 L bytes per vertex, k <= 4 L floats)
         float *dx = (float *)c0;
-        k_ppr_unpack<<<bgrid(ctx, n * k), kBB, 0, s>>>(x, g->n, k, dx);
+        k_ppr_unpack<<<bgrid(ctx, n * k), kBB, 0, s>>>(x, g->n, L, k, dx);
         GG_LAUNCHED(ctx);
         GG_CHECK(host_download(ctx, host_x, dx, n * k * 4));
     }

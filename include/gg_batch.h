@@ -15,8 +15,8 @@
  *        x_s = alpha * e_s + (1 - alpha) * A^T D^-1 x_s,
  *    D = out-degree (vertices without out-edges pass nothing on), x_s(0) =
  *    e_s, `iters` iterations.  Ranks and contributions are stored in
- *    bfloat16 (a 256-byte row of 128 seeds per vertex), sums in float32.
- *    The iteration loop is captured once into a CUDA graph.
+ *    bfloat16 (a row of 16, 32, 64 or 128 seeds per vertex), sums in
+ *    float32; one launch per iteration.
  *  - gg_graph_union + gg_bfs_level_multi + gg_cc: many independent graphs
  *    are laid side by side as one graph (part i's vertex v becomes
  *    vertex_base[i] + v); BFS from one root per part is a multi-root BFS on

@@ -107,6 +107,24 @@ def test_ppr_heavy_rows_and_sinks(ctx):
         G.close()
 
 
+@pytest.mark.parametrize("hub", [200, 1023, 1025, 3000])
+@pytest.mark.parametrize("k", [1, 16, 17, 32, 33, 64, 65])
+def test_ppr_row_widths(ctx, hub, k):
+    # a seed's ranks are the same sums in the same order however many seeds
+    # share a row; the hub's in-degree is a light row's, one chunk's, several's
+    rng = np.random.default_rng(hub)
+    n = 3001
+    edges = [(int(u), 0) for u in rng.permutation(np.arange(1, n))[:hub]]
+    edges += [(int(u), int(v)) for u, v in rng.integers(0, n, (9000, 2)) if u != v]
+    g = O.from_edges(n, edges, symmetric=False)
+    G = upload(ctx, g, False)
+    seeds = nonisolated(g, 128, 7)
+    x = gg.ppr(G, seeds, alpha=0.15, iters=6)
+    assert np.abs(x - B.ppr_bf16(g, seeds, 0.15, 6)).sum(0).max() < PPR_L1_VS_BF16_EMUL
+    assert np.array_equal(gg.ppr(G, seeds[:k], alpha=0.15, iters=6), x[:, :k])
+    G.close()
+
+
 def test_ppr_zero_iterations_is_teleport(ctx):
     g = O.rmat(8, 2000, 2)
     G = upload(ctx, g)

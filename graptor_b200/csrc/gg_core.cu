@@ -583,6 +583,7 @@ static void graph_free(gg_graph *g) {
     cudaFree(g->items);
     bfs_resident_free(g);
     cc_resident_free(g);
+    pr_plan_free(g);
     cudaFree(g->pstate2);
     for (int i = 0; i < 2; ++i) {
         if (g->copy_done[i]) {
@@ -854,6 +855,7 @@ gg_status gg_tuning_set(const char *name, int64_t v) {
     else if (k == "cc_hook" && v <= 2) t.cc_hook = (int)v;
     else if (k == "graph" && v <= 1) t.graph = (int)v;
     else if (k == "resident" && v <= 1) t.resident = (int)v;
+    else if (k == "pr_blocked" && v <= 2) t.pr_blocked = (int)v;
     else if (k == "graph_handoff" && v <= (1 << 20)) t.graph_handoff = (int)v;
     else if (k == "handoff_ctas" && v <= (1 << 16)) t.handoff_ctas = (int)v;
     else if (k == "small_frontier" && v <= 1) t.small_frontier = (int)v;
@@ -895,6 +897,7 @@ gg_status gg_tuning_get(const char *name, int64_t *v) {
     else if (k == "cc_hook") *v = t.cc_hook;
     else if (k == "graph") *v = t.graph;
     else if (k == "resident") *v = t.resident;
+    else if (k == "pr_blocked") *v = t.pr_blocked;
     else if (k == "graph_handoff") *v = t.graph_handoff;
     else if (k == "handoff_ctas") *v = t.handoff_ctas;
     else if (k == "small_frontier") *v = t.small_frontier;

@@ -176,6 +176,8 @@ struct gg_graph {
     void *items = nullptr;     // work items of the resident kernels (gg_items.cuh)
     void *bfs_res = nullptr;   // resident BFS: buffers
     void *cc_res = nullptr;    // resident CC: buffers
+    void *pr_plan = nullptr;   // blocked PageRank gather: edge layout (gg_prplan.cuh)
+    uint64_t pr_iters = 0;     // PageRank iterations asked for so far
     CandLists cand;               // pull candidate lists (driver runs)
     bool cand_active = false;     // a driver run uses them for its pull steps
     // released frontier buffers, reused in stream order
@@ -253,6 +255,7 @@ gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok);
 gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *iters_out);
 gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_host);
 void cc_resident_free(gg_graph *g);
+void pr_plan_free(gg_graph *g);
 gg_status enqueue_bfs_start(gg_graph *g, gg_prop *level, gg_prop *prev, const uint32_t *d_roots, uint32_t k);
 gg_status enqueue_cc_start(gg_graph *g, gg_prop *label, gg_prop *prev);
 gg_status run_tmp_prop(gg_graph *g, int slot, gg_dtype t, gg_prop **out);
@@ -298,6 +301,9 @@ struct Tuning {
     // graph-driven run would be taken, CC of symmetric graphs as one
     // (gg_cc.cu) where the device-driven run would
     int resident = 1;
+    // PageRank's gather by blocks of sources (gg_prplan.cuh): 1: where it is
+    // faster, 2: wherever the layout can be built, 0: never
+    int pr_blocked = 1;
     // graph-driven BFS levels: a run still going after this many iterations
     // (a high-diameter graph: many small frontiers, where the graph's
     // per-step node launches cost more than a grid barrier) continues in the

@@ -10,7 +10,8 @@
 //   delta = sum |x-y| (double); x = y; y = 0; contrib = d*x/outdeg
 // until iter == maxiter or delta <= tol.
 //
-// B200 design: two kernels per iteration (three where there are heavy rows),
+// B200 design: two kernels per iteration (three where there are heavy rows,
+// four where the gather goes by blocks of sources),
 // all enqueued up front; a device-resident state block carries the sums and a
 // "done" flag that makes later iterations return immediately once the
 // residual test passes, so the host never synchronises inside the loop.
@@ -20,6 +21,8 @@
 //                 with scale, customfp<6,10>, BF16-by-truncation);
 //                 accumulation in float or double; the block sums of y
 //                 (double) are folded in with one atomic per CTA.
+//   k_pr_values, k_pr_bins, k_pr_spans : the same sums for large graphs, the
+//                 values moved by blocks of sources and bins of edges.
 //   k_pr_update : y += w, y *= 1/s, delta, x = y, contrib = d*x/deg encoded,
 //                 one pass.  The second sum of the reference (sum of the
 //                 rounded y+w) is taken as s + n*w in double: equal in exact
@@ -40,7 +43,7 @@
 #include <cstdlib>
 
 #include <algorithm>
-#include "gg_internal.cuh"
+#include "gg_prplan.cuh"
 
 namespace gg {
 
@@ -171,6 +174,12 @@ __device__ __host__ inline float scale_for(int dt, float cmax) {
     int e;
     frexpf(half_range / cmax, &e);
     return ldexpf(1.0f, e - 1);
+}
+
+// a row's sum as a float rank
+template <int DT, typename Acc> __device__ __forceinline__ float pr_value(Acc acc, float sinv) {
+    if (DT == GG_FP8E4M3 || DT == GG_F16) acc *= (Acc)sinv;
+    return (float)acc;
 }
 
 // y[d] (or its double twin) from a row's sum; returns the stored value for
@@ -623,6 +632,14 @@ __global__ void k_pr_init(XT<DT> *x, typename Store<DT>::T *contrib, const uint6
 
 constexpr int kBlock = 256;
 
+// The gather by blocks pays from some 50 M edges on (20 iterations, by rows
+// -> by blocks: R-MAT 20 with 31 M edges 3.3 -> 5.1 ms, ER 16 M 2.0 -> 1.9,
+// ER 63 M FP16 5.9 -> 4.5, R-MAT 22 x 8 FP32 6.4 -> 5.5), and its layout takes
+// the time of some 3 (ER) to 20 (R-MAT 24) iterations' gain to build: it is
+// built once a graph has been asked for that many iterations.
+constexpr uint64_t kBlockedEdges = 3ull << 24;
+constexpr uint64_t kBlockedIters = 16;
+
 static unsigned pr_grid(gg_ctx *ctx, uint64_t work) {
     uint64_t b = (work + kBlock - 1) / kBlock;
     uint64_t cap = (uint64_t)ctx->sm_count * tuning().pr_blocks_per_sm;
@@ -663,6 +680,279 @@ static gg_status gather_launch(gg_graph *g, const typename Store<DT>::T *contrib
     return GG_OK;
 }
 
+// ---------------------------------------------------------------------------
+// The gather by blocks of sources (gg_prplan.cuh)
+// ---------------------------------------------------------------------------
+// k_pr_gather cannot go below one sector from L2 per gathered value.  Here a
+// value is read from shared memory, written and read again in whole sectors
+// and placed through shared memory: 12.5 bytes of DRAM traffic an edge with
+// 4-byte values, 8.5 with 16-bit ones (0.98 and 0.68 ms for 520 M edges).
+// Measured per iteration, the rest of it included, by rows -> by blocks:
+// R-MAT 24 FP32 with double sums 2.02 -> 1.66 ms, directed ER 2^24 x 32 BF16
+// 2.13 -> 1.42, ER 4 M x 64 FP32 1.06 -> 0.74, R-MAT 22 BF16 0.46 -> 0.36.
+// Of it k_pr_values 0.60 ms and k_pr_bins 0.94 ms (R-MAT 24), 1.6 and 1.8
+// times their DRAM time: their accesses to shared memory, some 3.7 banks deep
+// as the ids fall, and the loads take turns, with two CTAs per SM to overlap
+// them.  Bins of 16384 edges (3 CTAs) 2.4 ms: tiles, and with them the runs
+// read from DRAM, get shorter.  The values written by the first kernel in
+// bin order instead, so that the second reads them in one piece: 1.9 ms, and
+// 2.0 for BF16 (runs of half sectors).
+constexpr int kValBlock = 1024;
+// chunks that a thread of k_pr_values has in flight, and CTAs per SM (a block
+// of float contributions takes 128 KiB, one of 16-bit ones 64)
+template <typename T> constexpr int kValFlight = sizeof(T) == 4 ? 4 : 1;
+template <typename T> constexpr int kValCtas = sizeof(T) == 4 ? 1 : 2;
+
+// 8 values of a chunk, moved by one access of 16 or 32 bytes (in two halves,
+// the lanes of a warp would each touch half of a sector, twice)
+template <typename T> struct Val8 {
+    T v[8];
+};
+__device__ __forceinline__ void load8(const float *p, Val8<float> &x) {
+    asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(x.v[0]), "=f"(x.v[1]), "=f"(x.v[2]), "=f"(x.v[3]), "=f"(x.v[4]), "=f"(x.v[5]), "=f"(x.v[6]), "=f"(x.v[7])
+        : "l"(p));
+}
+__device__ __forceinline__ void store8(float *p, const Val8<float> &x) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(x.v[0]), "f"(x.v[1]),
+                 "f"(x.v[2]), "f"(x.v[3]), "f"(x.v[4]), "f"(x.v[5]), "f"(x.v[6]), "f"(x.v[7])
+                 : "memory");
+}
+__device__ __forceinline__ void load8(const uint16_t *p, Val8<uint16_t> &x) {
+    const uint4 q = __ldg((const uint4 *)p);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        x.v[2 * k] = (uint16_t)(w[k] & 0xFFFFu);
+        x.v[2 * k + 1] = (uint16_t)(w[k] >> 16);
+    }
+}
+__device__ __forceinline__ void store8(uint16_t *p, const Val8<uint16_t> &x) {
+    uint32_t w[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) w[k] = x.v[2 * k] | (uint32_t)x.v[2 * k + 1] << 16;
+    *(uint4 *)p = make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// vals[slot] = the contribution of the slot's source, read from the block's
+// contributions in shared memory.
+template <typename T>
+__global__ void __launch_bounds__(kValBlock, kValCtas<T>)
+k_pr_values(const uint16_t *__restrict__ src, const uint4 *__restrict__ segs, const uint32_t *__restrict__ part_seg,
+            const T *__restrict__ contrib, uint32_t n, T *__restrict__ vals, const PrState *st) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    T *blk = (T *)smem;
+    if (pr_idle(st, -1)) return;
+    const uint32_t hi = part_seg[blockIdx.x + 1];
+    for (uint32_t i = part_seg[blockIdx.x]; i < hi; ++i) {
+        const uint4 seg = segs[i];
+        const uint32_t v0 = seg.x << kBlkSrcLog, len = min(n - v0, kBlkSrc);
+        constexpr uint32_t W = 16 / sizeof(T);
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < len / W; j += kValBlock) {
+            const uint4 q = __ldg((const uint4 *)(contrib + v0) + j);
+            const T *x = (const T *)&q;
+#pragma unroll
+            for (uint32_t k = 0; k < W; ++k) blk[blk_slot(j * W + k)] = x[k];
+        }
+        for (uint32_t j = len / W * W + threadIdx.x; j < len; j += kValBlock) blk[blk_slot(j)] = contrib[v0 + j];
+        __syncthreads();
+        constexpr int U = kValFlight<T>;
+        uint4 id[U];
+        auto ids = [&](uint64_t c) {
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (c + u * kValBlock < seg.z) id[u] = __ldcs((const uint4 *)src + c + u * kValBlock);
+        };
+        uint64_t c = (uint64_t)seg.y + threadIdx.x;
+        ids(c);
+        for (; c < seg.z; c += kValBlock * U) {
+            uint4 a[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) a[u] = id[u];
+            ids(c + kValBlock * U);
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (c + u * kValBlock >= seg.z) break;
+                const uint32_t w[4] = {a[u].x, a[u].y, a[u].z, a[u].w};
+                Val8<T> o;
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    o.v[2 * k] = blk[w[k] & 0xFFFFu];
+                    o.v[2 * k + 1] = blk[w[k] >> 16];
+                }
+                store8(vals + (c + u * kValBlock) * 8, o);
+            }
+        }
+    }
+}
+
+// The row sums of a bin: its values put in the edges' places in shared
+// memory, then 32 edges per thread, cut where rows end; what a thread's
+// first row has in the threads before comes from a segmented scan.  A bin's
+// part of a row that began before it goes to parts[2 b], its edges after the
+// last end of a row to parts[2 b + 1].
+template <int DT, bool ACC64>
+__global__ void __launch_bounds__(kBinThreads, 2)
+k_pr_bins(PrPlan P, const typename Store<DT>::T *__restrict__ vals, const uint32_t *__restrict__ list, uint64_t m,
+          float *y_f32, PrState *st, typename std::conditional<ACC64, double, float>::type *parts) {
+    using S = Store<DT>;
+    using T = typename S::T;
+    using Acc = typename std::conditional<ACC64, double, float>::type;
+    constexpr int WARPS = kBinThreads / 32;
+    extern __shared__ __align__(16) uint8_t smem[];
+    float *buf = (float *)smem;  // decoded values; in their stead, later, the sums of the thread's rows
+    __shared__ uint32_t s_ends[WARPS];
+    __shared__ Acc s_sum[WARPS];
+    __shared__ double s_y[WARPS];
+    __shared__ bool s_cut[WARPS];
+    const uint32_t b = blockIdx.x, t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    // (all that does not depend on another load first)
+    const uint32_t hi = __ldg(P.bin_ptr + b + 1);
+    uint32_t c = __ldg(P.bin_ptr + b) + t;
+    const uint32_t bits = __ldg(P.ends + (uint64_t)b * kBinThreads + t);  // the thread's edges that end rows
+    const uint32_t *rows = list + __ldg(P.bin_end + b);                  // the rows that end in the bin
+    const bool head = b && !(__ldg(P.ends + (uint64_t)b * kBinThreads - 1) >> 31);
+    if (pr_idle(st, -1)) return;
+    const float sinv = st->scale_inv;
+    uint32_t at = c < hi ? __ldcs(P.ptr + c) : 0u;
+    uint32_t rank = __popc(bits);  // of the thread's first row end, from here on
+    const uint32_t nends = rank;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(FULL, rank, o);
+        if (lane >= (uint32_t)o) rank += x;
+    }
+    if (lane == 31) s_ends[warp] = rank;
+    rank -= nends;
+    while (c < hi) {
+        const uint4 ps = __ldcs((const uint4 *)P.pos + at);
+        Val8<T> v;
+        load8(vals + (uint64_t)at * 8, v);
+        c += kBinThreads;
+        if (c < hi) at = __ldcs(P.ptr + c);
+        const uint32_t w[4] = {ps.x, ps.y, ps.z, ps.w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            buf[w[k] & 0xFFFFu] = S::dec(v.v[2 * k]);
+            buf[w[k] >> 16] = S::dec(v.v[2 * k + 1]);
+        }
+    }
+    const uint32_t len = (uint32_t)min(m - (uint64_t)b * kBinEdges, (uint64_t)kBinEdges);
+    for (uint32_t p = len + t; p < kBinEdges; p += kBinThreads) buf[bin_slot(p)] = 0.0f;  // (the last bin)
+    __syncthreads();
+    rank += dev::warp_sum(lane < warp ? s_ends[lane] : 0u);
+    // the thread's first two rows, loaded beside the sums
+    const uint32_t d0 = nends ? __ldg(rows + rank) : 0u, d1 = nends > 1 ? __ldg(rows + rank + 1) : 0u;
+    const uint32_t own = bin_slot(t * 32) * 4, first = bits & (0u - bits);
+    auto slot = [&](uint32_t i4) -> float & { return *(float *)(smem + (own ^ i4)); };
+    Acc acc = 0, lead = 0;
+    uint32_t to = 0;  // 4 times the row ends seen
+#pragma unroll
+    for (uint32_t i = 0; i < 32; ++i) {
+        acc += (Acc)slot(i * 4);
+        const bool end = bits >> i & 1u;
+        if (end) slot(to) = pr_value<DT>(acc, sinv);
+        lead = first >> i & 1u ? acc : lead;
+        to += end ? 4u : 0u;
+        acc = end ? Acc(0) : acc;
+    }
+    // segmented scan of the threads' ends (acc, bits != 0: cut)
+    Acc v = acc;
+    bool cut = bits != 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const Acc x = __shfl_up_sync(FULL, v, o);
+        const bool f = __shfl_up_sync(FULL, (int)cut, o);
+        if (lane >= (uint32_t)o) {
+            if (!cut) v += x;
+            cut |= f;
+        }
+    }
+    if (lane == 31) {
+        s_sum[warp] = v;
+        s_cut[warp] = cut;
+    }
+    __syncthreads();
+    Acc carry = 0;  // of the warps before
+    {
+        // those from the last cut on, in their order
+        const uint32_t cuts = __ballot_sync(FULL, lane < warp && s_cut[lane]);
+        const uint32_t from = cuts ? 31 - __clz(cuts) : 0u;
+        for (uint32_t w = from; w < warp; ++w) carry += s_sum[w];
+    }
+    const Acc x = __shfl_up_sync(FULL, v, 1);
+    const bool f = __shfl_up_sync(FULL, (int)cut, 1);
+    double ysum = 0;
+    if (nends) {
+        lead += lane == 0 ? carry : f ? x : carry + x;
+        if (rank == 0 && head) {
+            parts[2 * (uint64_t)b] = lead;
+        } else {
+            const float y = pr_value<DT>(lead, sinv);
+            y_f32[d0] = y;
+            ysum = (double)y;
+        }
+        uint32_t d = d1;
+        for (uint32_t j = 1; j < nends; ++j) {
+            const uint32_t dn = j + 1 < nends ? __ldg(rows + rank + j + 1) : 0u;
+            const float y = slot(j * 4);
+            y_f32[d] = y;
+            ysum += (double)y;
+            d = dn;
+        }
+    }
+    if (t == kBinThreads - 1) parts[2 * (uint64_t)b + 1] = cut ? v : carry + v;
+    ysum = dev::warp_sum(ysum);
+    if (lane == 0) s_y[warp] = ysum;
+    __syncthreads();
+    if (warp == 0) {
+        ysum = dev::warp_sum(lane < WARPS ? s_y[lane] : 0.0);
+        if (lane == 0) atomicAdd(&st->s1, ysum);
+    }
+}
+
+// Totals of the rows that end in a later bin than they begin in: a thread
+// per bin, its first row's parts in the order of the bins.
+template <int DT, bool ACC64>
+__global__ void __launch_bounds__(256)
+k_pr_spans(PrPlan P, const uint32_t *__restrict__ list, float *y_f32, PrState *st,
+           const typename std::conditional<ACC64, double, float>::type *parts) {
+    using Acc = typename std::conditional<ACC64, double, float>::type;
+    if (pr_idle(st, -1)) return;
+    const uint32_t b = blockIdx.x * 256 + threadIdx.x;
+    double ysum = 0;
+    if (b && b < P.nbin && P.bin_end[b + 1] > P.bin_end[b] && !(P.ends[(uint64_t)b * kBinThreads - 1] >> 31)) {
+        uint32_t x = b - 1;
+        while (x && P.bin_end[x + 1] == P.bin_end[x]) --x;
+        Acc acc = 0;
+        for (; x < b; ++x) acc += parts[2 * (uint64_t)x + 1];
+        acc += parts[2 * (uint64_t)b];
+        ysum = pr_store_row<DT, false>(y_f32, nullptr, list[P.bin_end[b]], acc, st->scale_inv);
+    }
+    ysum = dev::block_sum<double, 256>(ysum);
+    if (threadIdx.x == 0 && ysum != 0) atomicAdd(&st->s1, ysum);
+}
+
+template <int DT, bool ACC64>
+static gg_status blocked_launch(gg_graph *g, const PrPlan &P, const typename Store<DT>::T *contrib, float *y,
+                                PrState *st, void *vals, void *parts) {
+    gg_ctx *ctx = g->ctx;
+    cudaStream_t s = ctx->stream;
+    using T = typename Store<DT>::T;
+    using Acc = typename std::conditional<ACC64, double, float>::type;
+    const size_t sv = (size_t)kBlkSrc * sizeof(T), sb = (size_t)(kBinEdges + 8) * 4;
+    GG_CUDA(ctx, cudaFuncSetAttribute(k_pr_values<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sv));
+    GG_CUDA(ctx, cudaFuncSetAttribute(k_pr_bins<DT, ACC64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
+    k_pr_values<T><<<P.nparts, kValBlock, sv, s>>>(P.src, P.segs, P.part_seg, contrib, g->n, (T *)vals, st);
+    GG_LAUNCHED(ctx);
+    k_pr_bins<DT, ACC64><<<P.nbin, kBinThreads, sb, s>>>(P, (const T *)vals, g->nonisolated, g->m, y, st, (Acc *)parts);
+    GG_LAUNCHED(ctx);
+    k_pr_spans<DT, ACC64><<<(P.nbin + 255) / 256, 256, 0, s>>>(P, g->nonisolated, y, st, (const Acc *)parts);
+    GG_LAUNCHED(ctx);
+    return GG_OK;
+}
+
 // Damping of the FP64 variant: the shortest decimal that rounds to the float
 // parameter (0.85f -> 0.85), as the double-precision reference uses it.
 static double damping_f64(float d) {
@@ -677,11 +967,14 @@ static double damping_f64(float d) {
 
 template <int DT>
 static gg_status pr_run(gg_graph *g, const gg_pr_params *p, XT<DT> *x, XT<DT> *y, void *contrib,
-                        PrState *st, void *partial, float *acc = nullptr) {
+                        PrState *st, void *partial, const PrPlan *plan, void *vals, float *acc = nullptr) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     using T = typename Store<DT>::T;
     const uint32_t n = g->n;
+    // (the blocked gather stores no row without in-edges)
+    if (plan) GG_CUDA(ctx, cudaMemsetAsync(y, 0, (size_t)n * 4, s));
+    void *parts = plan ? (char *)vals + plan->chunks * 8 * sizeof(T) : nullptr;
     const unsigned gv = pr_grid(ctx, n);
     const double d64 = damping_f64(p->damping);
     k_pr_init<DT, kBlock><<<gv, kBlock, 0, s>>>(x, (T *)contrib, g->off, n, p->damping, d64, st, 0);
@@ -693,7 +986,13 @@ static gg_status pr_run(gg_graph *g, const gg_pr_params *p, XT<DT> *x, XT<DT> *y
     float *yf = DT == GG_F64 ? nullptr : (float *)y;
     double *yd = DT == GG_F64 ? (double *)y : nullptr;
     for (int it = 0; it < p->maxiter; ++it) {
-        if (p->accum_f64 || DT == GG_F64)
+        if (plan) {
+            if constexpr (DT != GG_F64 && DT != GG_FP8E4M3) {
+                if (p->accum_f64)
+                    GG_CHECK((blocked_launch<DT, true>(g, *plan, (const T *)contrib, yf, st, vals, parts)));
+                else GG_CHECK((blocked_launch<DT, false>(g, *plan, (const T *)contrib, yf, st, vals, parts)));
+            }
+        } else if (p->accum_f64 || DT == GG_F64)
             GG_CHECK((gather_launch<DT, true, false>(g, (const T *)contrib, yf, yd, st, 1.0f, partial)));
         else
             GG_CHECK((gather_launch<DT, false, false>(g, (const T *)contrib, yf, yd, st, 1.0f, partial)));
@@ -898,13 +1197,27 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     const size_t sb = (sizeof(PrState) + 255) / 256 * 256;
     void *base = nullptr;
     const size_t ab = p->average_last > 0 ? (((size_t)g->n + 1) * 4 + 255) / 256 * 256 : 0;
-    gg_status s = graph_scratch(g, 2 * nb + sb + ab + (g->heavy.nchunks + 1) * 8, &base);
+    const size_t pb = ((g->heavy.nchunks + 1) * 8 + 255) / 256 * 256;
+    const PrPlan *plan = nullptr;
+    if (!staged) g->pr_iters += p->maxiter;
+    const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
+                         (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && g->pr_iters >= kBlockedIters));
+    // (the values' space also serves the building of the plan)
+    const size_t vb = blocked ? pr_plan_bytes(g, dt == GG_F32 ? 4 : 2) : 0;
+    gg_status s = graph_scratch(g, 2 * nb + sb + ab + pb + vb, &base);
+    if (s != GG_OK && vb) {  // without the blocked gather, then
+        cudaGetLastError();
+        s = graph_scratch(g, 2 * nb + sb + ab + pb, &base);
+    } else if (vb) {
+        s = pr_plan(g, (char *)base + 2 * nb + sb + ab + pb, &plan);
+    }
     if (s != GG_OK) { if (tmpx) gg_prop_destroy(tmpx); return s; }
     float *y = (float *)base;
     void *contrib = (char *)base + nb;
     PrState *st = (PrState *)((char *)base + 2 * nb);
     float *acc = ab ? (float *)((char *)base + 2 * nb + sb) : nullptr;
     void *partial = (char *)base + 2 * nb + sb + ab;
+    void *vals = (char *)partial + pb;
     PrState init;
     memset(&init, 0, sizeof(init));
     init.maxiter = p->maxiter;
@@ -928,13 +1241,13 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
         if (staged) {
             s = pr_run_staged(g, p, (float *)xp->d, y, contrib, st, partial);
         } else switch (dt) {
-        case GG_F64: s = pr_run<GG_F64>(g, p, (double *)xp->d, (double *)base, contrib, st, partial); break;
-        case GG_F32: s = pr_run<GG_F32>(g, p, (float *)xp->d, y, contrib, st, partial); break;
-        case GG_BF16: s = pr_run<GG_BF16>(g, p, (float *)xp->d, y, contrib, st, partial, acc); break;
-        case GG_F16: s = pr_run<GG_F16>(g, p, (float *)xp->d, y, contrib, st, partial); break;
-        case GG_FP8E4M3: s = pr_run<GG_FP8E4M3>(g, p, (float *)xp->d, y, contrib, st, partial); break;
-        case GG_CFP_6_10: s = pr_run<GG_CFP_6_10>(g, p, (float *)xp->d, y, contrib, st, partial); break;
-        default: s = pr_run<GG_BF16_TRUNC>(g, p, (float *)xp->d, y, contrib, st, partial); break;
+        case GG_F64: s = pr_run<GG_F64>(g, p, (double *)xp->d, (double *)base, contrib, st, partial, nullptr, nullptr); break;
+        case GG_F32: s = pr_run<GG_F32>(g, p, (float *)xp->d, y, contrib, st, partial, plan, vals); break;
+        case GG_BF16: s = pr_run<GG_BF16>(g, p, (float *)xp->d, y, contrib, st, partial, plan, vals, acc); break;
+        case GG_F16: s = pr_run<GG_F16>(g, p, (float *)xp->d, y, contrib, st, partial, plan, vals); break;
+        case GG_FP8E4M3: s = pr_run<GG_FP8E4M3>(g, p, (float *)xp->d, y, contrib, st, partial, nullptr, nullptr); break;
+        case GG_CFP_6_10: s = pr_run<GG_CFP_6_10>(g, p, (float *)xp->d, y, contrib, st, partial, plan, vals); break;
+        default: s = pr_run<GG_BF16_TRUNC>(g, p, (float *)xp->d, y, contrib, st, partial, plan, vals); break;
         }
     } else {
         s = cuda_error(ctx, e, "gg_pagerank state upload");

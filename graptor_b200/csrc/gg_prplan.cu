@@ -1,0 +1,281 @@
+// Building of the blocked PageRank gather's edge layout (gg_prplan.cuh): a
+// counting pass over the in-edges, a scan of the tiles' chunks, and a pass
+// that sorts each bin's edges by source block in shared memory and writes
+// them as whole chunks.  Ranks within a tile are taken with atomics, so their
+// order may differ between builds; the gather's results do not depend on it.
+#include <cub/cub.cuh>
+
+#include <algorithm>
+#include <vector>
+
+#include "gg_prplan.cuh"
+
+namespace gg {
+
+namespace {
+
+constexpr int kPB = 1024;
+constexpr uint32_t kPer = kBinEdges / kPB;
+static_assert(kBinEdges % kPB == 0 && kBinEdges < 65536, "places within a bin take 16 bits");
+
+// chunks of every tile, and of every bin
+__global__ void __launch_bounds__(kPB) k_plan_count(const uint32_t *__restrict__ in_adj, uint64_t m, uint32_t nblk,
+                                                    uint32_t nbin, uint32_t *tile, uint32_t *bin_ptr) {
+    __shared__ uint32_t hist[kBlkMax];
+    const uint32_t b = blockIdx.x;
+    const uint64_t base = (uint64_t)b * kBinEdges;
+    for (uint32_t i = threadIdx.x; i < nblk; i += kPB) hist[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t i = 0; i < kPer; ++i) {
+        const uint64_t e = base + i * kPB + threadIdx.x;
+        if (e < m) atomicAdd(&hist[__ldcs(in_adj + e) >> kBlkSrcLog], 1u);
+    }
+    __syncthreads();
+    uint32_t sum = 0;
+    for (uint32_t i = threadIdx.x; i < nblk; i += kPB) {
+        const uint32_t c = (hist[i] + 7) / 8;
+        tile[(uint64_t)i * nbin + b] = c;
+        sum += c;
+    }
+    sum = dev::block_sum<uint32_t, kPB>(sum);
+    if (threadIdx.x == 0) bin_ptr[b] = sum;
+}
+
+// each block's first chunk, and the number of chunks
+__global__ void k_plan_starts(const uint32_t *tile, uint32_t nblk, uint32_t nbin, uint32_t *at) {
+    const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k <= nblk) at[k] = tile[(uint64_t)k * nbin];
+}
+
+// the bin's edges sorted by block; tile holds each tile's first chunk
+__global__ void __launch_bounds__(kPB) k_plan_fill(const uint32_t *__restrict__ in_adj, uint64_t m, uint32_t nblk,
+                                                   uint32_t nbin, const uint32_t *__restrict__ tile,
+                                                   const uint32_t *__restrict__ bin_ptr, uint16_t *src, uint16_t *pos,
+                                                   uint32_t *ptr) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    const uint32_t cap = (kBinEdges + 7 * nblk + 7) / 8 * 8;
+    uint16_t *ssrc = (uint16_t *)smem, *spos = ssrc + cap;
+    __shared__ uint32_t hist[kBlkMax], first[kBlkMax + 1], wsum[kPB / 32];
+    const uint32_t b = blockIdx.x, lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t base = (uint64_t)b * kBinEdges;
+    for (uint32_t i = threadIdx.x; i < nblk; i += kPB) hist[i] = 0;
+    __syncthreads();
+    uint32_t id[kPer], rank[kPer];
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i) {
+        const uint64_t e = base + i * kPB + threadIdx.x;
+        id[i] = e < m ? __ldcs(in_adj + e) : 0u;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i)
+        rank[i] = base + i * kPB + threadIdx.x < m ? atomicAdd(&hist[id[i] >> kBlkSrcLog], 1u) : 0u;
+    __syncthreads();
+    // exclusive prefix of the tiles' chunks: two tiles per thread
+    static_assert(kBlkMax == 2 * kPB, "two tiles per thread");
+    const uint32_t t = 2 * threadIdx.x;
+    const uint32_t c0 = t < nblk ? (hist[t] + 7) / 8 : 0u, c1 = t + 1 < nblk ? (hist[t + 1] + 7) / 8 : 0u;
+    uint32_t incl = c0 + c1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += x;
+    }
+    if (lane == 31) wsum[warp] = incl;
+    __syncthreads();
+    uint32_t before = 0;
+    for (uint32_t w = 0; w < warp; ++w) before += wsum[w];
+    first[t] = before + incl - c0 - c1;
+    first[t + 1] = before + incl - c1;
+    if (threadIdx.x == kPB - 1) first[kBlkMax] = before + incl;
+    __syncthreads();
+    const uint32_t total = first[kBlkMax];
+    for (uint32_t i = threadIdx.x; i < total; i += kPB) {
+        ((uint4 *)ssrc)[i] = make_uint4(0, 0, 0, 0);
+        ((uint4 *)spos)[i] = make_uint4(kBinEdges * 0x10001u, kBinEdges * 0x10001u, kBinEdges * 0x10001u,
+                                        kBinEdges * 0x10001u);
+    }
+    __syncthreads();
+#pragma unroll
+    for (uint32_t i = 0; i < kPer; ++i)
+        if (base + i * kPB + threadIdx.x < m) {
+            const uint32_t slot = first[id[i] >> kBlkSrcLog] * 8 + rank[i];
+            ssrc[slot] = (uint16_t)blk_slot(id[i]);
+            spos[slot] = (uint16_t)bin_slot(i * kPB + threadIdx.x);
+        }
+    __syncthreads();
+    const uint64_t list = bin_ptr[b];
+    for (uint32_t k = warp; k < nblk; k += kPB / 32) {
+        const uint32_t f = first[k], cnt = (hist[k] + 7) / 8;
+        if (!cnt) continue;
+        const uint32_t to = tile[(uint64_t)k * nbin + b];
+        for (uint32_t j = lane; j < cnt; j += 32) {
+            ((uint4 *)src)[(uint64_t)to + j] = ((const uint4 *)ssrc)[f + j];
+            ((uint4 *)pos)[(uint64_t)to + j] = ((const uint4 *)spos)[f + j];
+            ptr[list + f + j] = to + j;
+        }
+    }
+}
+
+__global__ void k_plan_ends(const uint32_t *__restrict__ list, const uint64_t *__restrict__ count,
+                            const uint64_t *__restrict__ in_off, uint32_t *ends) {
+    const uint64_t nrow = *count, stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nrow; k += stride) {
+        const uint64_t last = in_off[list[k] + 1ull] - 1;
+        atomicOr(ends + (last >> 5), 1u << (last & 31));
+    }
+}
+
+__global__ void __launch_bounds__(kBinThreads) k_plan_bin_ends(const uint32_t *__restrict__ ends, uint32_t *bin_end) {
+    const uint32_t c = dev::block_sum<uint32_t, kBinThreads>(
+        __popc(ends[(uint64_t)blockIdx.x * kBinThreads + threadIdx.x]));
+    if (threadIdx.x == 0) bin_end[blockIdx.x] = c;
+}
+
+size_t aligned(size_t b) { return (b + 255) / 256 * 256; }
+
+size_t scan_bytes(uint64_t items) {
+    size_t b = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, b, (uint32_t *)nullptr, (uint32_t *)nullptr, (int64_t)items);
+    return b;
+}
+
+// most chunks that the layout can take: each tile pads its last one
+uint64_t chunk_bound(uint64_t nblk, uint64_t nbin, uint64_t m) { return m / 8 + std::min(nblk * nbin, m); }
+
+void plan_release(PrPlan *P) {
+    cudaFree(P->base);
+    cudaFree(P->segs);
+    cudaFree(P->part_seg);
+    *P = PrPlan();
+    P->tried = true;
+}
+
+cudaError_t plan_build(gg_graph *g, PrPlan *P, void *scratch) {
+    gg_ctx *ctx = g->ctx;
+    cudaStream_t st = ctx->stream;
+#define PK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
+    const uint64_t ntile = (uint64_t)P->nblk * P->nbin, most = chunk_bound(P->nblk, P->nbin, g->m);
+    const size_t cb = aligned(most * 16), pb = aligned(most * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
+                 eb = aligned((size_t)P->nbin * kBinThreads * 4);
+    PK(cudaMalloc(&P->base, 2 * cb + pb + 2 * bb + eb));
+    char *p = (char *)P->base;
+    P->src = (uint16_t *)p;
+    P->pos = (uint16_t *)(p + cb);
+    P->ptr = (uint32_t *)(p + 2 * cb);
+    P->bin_ptr = (uint32_t *)(p + 2 * cb + pb);
+    P->bin_end = (uint32_t *)(p + 2 * cb + pb + bb);
+    P->ends = (uint32_t *)(p + 2 * cb + pb + 2 * bb);
+    // scratch: the tiles' chunks, the blocks' first chunks, the scans' own
+    uint32_t *tiles = (uint32_t *)scratch;
+    uint32_t *starts = (uint32_t *)((char *)scratch + aligned((ntile + 1) * 4));
+    void *tmp = (char *)starts + aligned(((size_t)kBlkMax + 1) * 4);
+    size_t tb = scan_bytes(ntile + 1);
+    PK(cudaMemsetAsync(P->bin_ptr, 0, 2 * bb + eb, st));
+    PK(cudaMemsetAsync(tiles + ntile, 0, 4, st));
+    k_plan_ends<<<ctx->sm_count * 8, 256, 0, st>>>(g->nonisolated, g->nonisolated_n, g->in_off, P->ends);
+    PK(cudaGetLastError());
+    k_plan_bin_ends<<<P->nbin, kBinThreads, 0, st>>>(P->ends, P->bin_end);
+    PK(cudaGetLastError());
+    k_plan_count<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, P->nblk, P->nbin, tiles, P->bin_ptr);
+    PK(cudaGetLastError());
+    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, tiles, tiles, (int64_t)ntile + 1, st));
+    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, P->bin_ptr, P->bin_ptr, (int64_t)P->nbin + 1, st));
+    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, P->bin_end, P->bin_end, (int64_t)P->nbin + 1, st));
+    k_plan_starts<<<P->nblk / 256 + 1, 256, 0, st>>>(tiles, P->nblk, P->nbin, starts);
+    PK(cudaGetLastError());
+    const size_t smem = (size_t)((kBinEdges + 7 * P->nblk + 7) / 8 * 8) * 4;
+    PK(cudaFuncSetAttribute(k_plan_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_plan_fill<<<P->nbin, kPB, smem, st>>>(g->in_adj, g->m, P->nblk, P->nbin, tiles, P->bin_ptr, P->src, P->pos,
+                                            P->ptr);
+    PK(cudaGetLastError());
+    ctx->launches += 10;
+    std::vector<uint32_t> at(P->nblk + 1);  // first chunk of each block
+    PK(cudaMemcpyAsync(at.data(), starts, at.size() * 4, cudaMemcpyDeviceToHost, st));
+    PK(cudaStreamSynchronize(st));
+    P->chunks = at[P->nblk];
+    // parts of equal work: the chunks, and for each segment the load of its
+    // block's contributions (as long as some kBlkSrc / 12 chunks)
+    const uint64_t load = kBlkSrc / 12;
+    uint64_t work = 0;
+    for (uint32_t k = 0; k < P->nblk; ++k)
+        if (at[k + 1] > at[k]) work += at[k + 1] - at[k] + load;
+    const uint64_t share = std::max<uint64_t>(work / ((uint64_t)ctx->sm_count * 8) + 1, load);
+    std::vector<uint4> segs;
+    std::vector<uint32_t> part{0};
+    uint64_t room = share;
+    for (uint32_t k = 0; k < P->nblk; ++k)
+        for (uint32_t c = at[k]; c < at[k + 1];) {
+            if (room <= load && segs.size() > part.back()) {
+                part.push_back((uint32_t)segs.size());
+                room = share;
+            }
+            const uint64_t take = std::min<uint64_t>(at[k + 1] - c, room > load ? room - load : share);
+            segs.push_back(make_uint4(k, c, (uint32_t)(c + take), 0));
+            c += (uint32_t)take;
+            room = room > take + load ? room - take - load : 0;
+        }
+    part.push_back((uint32_t)segs.size());
+    P->nparts = (uint32_t)part.size() - 1;
+    PK(cudaMalloc(&P->segs, segs.size() * sizeof(uint4)));
+    PK(cudaMalloc(&P->part_seg, part.size() * 4));
+    PK(cudaMemcpyAsync(P->segs, segs.data(), segs.size() * sizeof(uint4), cudaMemcpyHostToDevice, st));
+    PK(cudaMemcpyAsync(P->part_seg, part.data(), part.size() * 4, cudaMemcpyHostToDevice, st));
+    PK(cudaStreamSynchronize(st));
+#undef PK
+    return cudaSuccess;
+}
+
+}  // namespace
+
+static PrPlan *plan_of(gg_graph *g) {
+    if (!g->pr_plan) {
+        PrPlan *P = new PrPlan();
+        P->nblk = (uint32_t)(((uint64_t)g->n + kBlkSrc - 1) >> kBlkSrcLog);
+        P->nbin = (uint32_t)((g->m + kBinEdges - 1) / kBinEdges);
+        // (chunk numbers take 32 bits; the layout and the values, 9 bytes an
+        // edge and the padding, leave more than half of the memory)
+        size_t free_b = 0, all_b = 0;
+        P->tried = !g->m || P->nblk > kBlkMax || g->m >> 32 || cudaMemGetInfo(&free_b, &all_b) != cudaSuccess ||
+                   chunk_bound(P->nblk, P->nbin, g->m) * 150 > free_b;
+        g->pr_plan = P;
+    }
+    return (PrPlan *)g->pr_plan;
+}
+
+size_t pr_plan_bytes(gg_graph *g, size_t size) {
+    const PrPlan *P = plan_of(g);
+    if (P->tried && !P->ready) return 0;
+    const uint64_t ntile = (uint64_t)P->nblk * P->nbin;
+    const uint64_t chunks = P->ready ? P->chunks : chunk_bound(P->nblk, P->nbin, g->m);
+    const size_t use = chunks * 8 * size + (size_t)P->nbin * 16;  // values, parts of rows
+    if (P->ready) return use;
+    return std::max(use, aligned((ntile + 1) * 4) + aligned(((size_t)kBlkMax + 1) * 4) + scan_bytes(ntile + 1));
+}
+
+gg_status pr_plan(gg_graph *g, void *scratch, const PrPlan **out) {
+    *out = nullptr;
+    PrPlan *P = plan_of(g);
+    if (!P->tried) {
+        P->tried = true;
+        const cudaError_t e = plan_build(g, P, scratch);
+        if (e != cudaSuccess) {
+            plan_release(P);
+            if (e != cudaErrorMemoryAllocation) return cuda_error(g->ctx, e, "PageRank edge layout");
+            cudaGetLastError();
+            return GG_OK;
+        }
+        P->ready = true;
+    }
+    if (P->ready) *out = P;
+    return GG_OK;
+}
+
+void pr_plan_free(gg_graph *g) {
+    if (!g->pr_plan) return;
+    plan_release((PrPlan *)g->pr_plan);
+    delete (PrPlan *)g->pr_plan;
+    g->pr_plan = nullptr;
+}
+
+}  // namespace gg

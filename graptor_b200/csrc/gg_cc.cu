@@ -4,9 +4,10 @@
 //
 // CCv (bench/CCv.C:221-471) lowers labels along every edge until nothing
 // moves; its labels are the smallest id of each component, whatever the order.
-//   search : at most kSearchSteps levels of the resident BFS (gg_bfs.cu).  On
-//            a graph with hubs they reach the giant component, most of it by
-//            pulls that look at one or two edges per vertex;
+//   search : where the degrees let it reach far, at most kSearchSteps levels
+//            of the resident BFS (gg_bfs.cu).  On a graph with hubs they reach
+//            the giant component, most of it by pulls that look at one or two
+//            edges per vertex;
 //   count  : the vertices reached and their smallest id.  Where they are half
 //            of the vertices with edges, that id is their label and only the
 //            others hook their edges (gg_uf.cuh);
@@ -37,6 +38,10 @@ constexpr int kCB = 512;                   // threads per CTA, two CTAs per SM
 // The search stops early at a frontier of fewer than kSearchLeast vertices: on
 // a grid or a sparse random graph it would not reach far, on a graph with hubs
 // little is left by then.
+// For the same reason there is none where even the largest hub's neighbours,
+// each with average rows, and theirs would be fewer (with the search -> without:
+// grid 85 x 84 less a third of its edges 161 -> 133 us a call, ER of 3001
+// vertices and average degree 3 163 -> 139, of 300001 and 2 212 -> 189).
 constexpr int kSearchSteps = 10;
 constexpr unsigned long long kSearchLeast = 1024;
 
@@ -56,7 +61,8 @@ struct CcArgs {
     HeavyRows H;
     uint32_t n;
     uint64_t m;
-    const int32_t *level;  // the search's
+    int searched;          // level, cand and st's reached_v are a search's
+    const int32_t *level;
     const uint32_t *cand[2];  // its candidate lists: st->cand_cur holds the vertices the last pull left open
     uint32_t *left;        // room for the vertices outside the giant component
     uint32_t *label;
@@ -78,7 +84,7 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
     unsigned long long epoch = 0;
     const unsigned long long t0 = grid::globaltimer();
     const uint64_t nn = *A.nonisolated_n, reached = A.st->reached_v;
-    const bool giant = 2 * reached >= nn;
+    const bool giant = A.searched && 2 * reached >= nn;
     bool ok = true;
 
     // ---- label
@@ -313,7 +319,12 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
     for (uint32_t i = threadIdx.x; i < sizeof(PState) / 16; i += kCB) ((uint4 *)A.rec)[i] = src[i];
 }
 
-__global__ void k_cc_start(CcState *cs) {
+__global__ void k_cc_start(CcState *cs, PState *st, int searched) {
+    if (!searched) {
+        st->err = 0;
+        st->reached_v = 0;
+        st->exit_small = st->small_done = 0;
+    }
     cs->bar.n = 0;
     cs->bar.err = 0;
     cs->smallest = 0xFFFFFFFFu;
@@ -388,11 +399,13 @@ gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_h
     gg_prop *level;
     GG_CHECK(run_tmp_prop(g, 1, GG_I32, &level));
     A.level = (const int32_t *)level->d;
-    GG_CHECK(bfs_resident_search(g, level, g->maxdeg_v, kSearchSteps, kSearchLeast, st));
+    const double avg = (double)g->m / (double)g->n;
+    A.searched = (double)g->maxdeg * avg * avg >= (double)kSearchLeast;
+    if (A.searched) GG_CHECK(bfs_resident_search(g, level, g->maxdeg_v, kSearchSteps, kSearchLeast, st));
     A.cand[0] = g->cand.list[0];
     A.cand[1] = g->cand.list[1];
     A.left = g->tmp_front[0]->bins[0];
-    k_cc_start<<<1, 1, 0, ctx->stream>>>(r->cs);
+    k_cc_start<<<1, 1, 0, ctx->stream>>>(r->cs, st, A.searched);
     GG_LAUNCHED(ctx);
     // a CTA per 2048 vertices or 16384 edges, all that fit at most
     const uint64_t most = (uint64_t)ctx->sm_count * resident_ctas((const void *)k_cc_run, kCB);

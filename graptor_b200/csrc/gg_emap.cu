@@ -234,9 +234,8 @@ __device__ __forceinline__ void flush_counts(const EmapArgs &A, unsigned long lo
 // ---------------------------------------------------------------------------
 // Dense pull over the CSC
 // ---------------------------------------------------------------------------
-// One lane owns one destination d.  Full-scan mode walks 32-vertex words
-// (one output bitmap word per warp, plain store); candidate mode walks a
-// list of destinations (output bitmap pre-cleared, bits set with atomicOr).
+// One lane owns one destination d.  pull_body walks a list of destinations
+// (output bitmap pre-cleared, bits set with atomicOr), pull_full every vertex.
 // Loads are issued ahead of use: d's value and both offsets together, then
 // up to 4 neighbour ids, then their frontier bits and source values.
 //
@@ -265,35 +264,30 @@ struct PullSmem {
     uint32_t rest[REST ? BLOCK / 32 : 1][256];
 };
 
-template <int R, bool SRCF, bool CAND, int BLOCK, int PASS = 0, bool STAGE = false, bool REST>
+template <int R, bool SRCF, int BLOCK, int PASS = 0, bool STAGE = false, bool REST>
 __device__ __forceinline__ void pull_body(const EmapArgs &A, const Op<R> &op, PullSmem<BLOCK, REST> &sm,
                                           const uint32_t *sbits = nullptr, uint32_t sn = 0) {
     static_assert(PASS != 1 || REST, "a split pull's first pass stages its rest list");
-    static_assert(PASS == 0 || (CAND && R == GG_RELAX_MIN_PLUS1_I32), "split pull: BFS levels, candidate lists");
+    static_assert(PASS == 0 || R == GG_RELAX_MIN_PLUS1_I32, "split pull: BFS levels");
     using V = typename Op<R>::V;
     const uint32_t lane = threadIdx.x & 31u;
-    const uint64_t nitems = CAND ? *A.cand_n : (uint64_t)A.n;
+    const uint64_t nitems = *A.cand_n;
     const uint64_t nw = (gridDim.x * BLOCK) >> 5;
     const uint64_t gw = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
-    // candidate lists: grid-stride over list words; full scan: a contiguous
-    // range of vertex words of equal estimated work per warp
-    uint32_t wlo = 0, whi = 0;
-    if (!CAND) dev::balanced_range(A.word_prefix, (A.n + 31u) >> 5, gw, nw, wlo, whi);
-    const uint64_t wstep = CAND ? nw : 1;
     unsigned long long nv = 0, ne = 0, sc = 0;
     dev::WarpAppender<256> keepers{sm.cand[threadIdx.x >> 5], 0, A.cand_out, A.cand_out_n};
     dev::WarpAppender<256> rest{sm.rest[REST ? threadIdx.x >> 5 : 0], 0, A.rest_out, A.rest_out_n};
-    for (uint64_t w = CAND ? gw : wlo; CAND ? ((w << 5) < nitems) : (w < whi); w += wstep) {
+    for (uint64_t w = gw; (w << 5) < nitems; w += nw) {
         const uint64_t item = (w << 5) + lane;
         const bool valid = item < nitems;
-        const uint32_t d = CAND ? (valid ? A.cand[item] : 0u) : (uint32_t)item;
+        const uint32_t d = valid ? A.cand[item] : 0u;
         V best = Op<R>::none();
         uint64_t e = 0, end = 0;
         uint4 f2 = make_uint4(0u, 0u, 0u, 0u);
         const bool has_rec = PASS != 2 && (A.first_in || A.first1);
         const bool lazy = has_rec && A.lazy_off;
         if (valid) {
-            best = (CAND && A.fresh) ? Op<R>::none() : op.load(d);
+            best = A.fresh ? Op<R>::none() : op.load(d);
             if (has_rec) {
                 if (A.first1) {
                     const uint2 r1 = A.first1[d];
@@ -444,22 +438,17 @@ __device__ __forceinline__ void pull_body(const EmapArgs &A, const Op<R> &op, Pu
             }
         }
         if (A.out_bits) {
-            if (CAND) {
-                // lanes holding vertices of the same bitmap word combine
-                // their bits; one atomicOr per word and warp
-                const uint32_t wd = d >> 5;
-                unsigned todo = __ballot_sync(FULL, rec);
-                while (todo) {  // one round per distinct word (list is mostly ascending)
-                    const int leader = __ffs(todo) - 1;
-                    const uint32_t w0 = __shfl_sync(FULL, wd, leader);
-                    const bool mine = rec && wd == w0;
-                    const unsigned bits = __reduce_or_sync(FULL, mine ? (1u << (d & 31)) : 0u);
-                    if ((int)lane == leader) atomicOr(A.out_bits + w0, bits);
-                    todo &= ~__ballot_sync(FULL, mine);
-                }
-            } else {
-                const unsigned bits = __ballot_sync(FULL, rec);
-                if (lane == 0) A.out_bits[w] = bits;
+            // lanes holding vertices of the same bitmap word combine
+            // their bits; one atomicOr per word and warp
+            const uint32_t wd = d >> 5;
+            unsigned todo = __ballot_sync(FULL, rec);
+            while (todo) {  // one round per distinct word (list is mostly ascending)
+                const int leader = __ffs(todo) - 1;
+                const uint32_t w0 = __shfl_sync(FULL, wd, leader);
+                const bool mine = rec && wd == w0;
+                const unsigned bits = __reduce_or_sync(FULL, mine ? (1u << (d & 31)) : 0u);
+                if ((int)lane == leader) atomicOr(A.out_bits + w0, bits);
+                todo &= ~__ballot_sync(FULL, mine);
             }
         }
         if (rec) {
@@ -477,10 +466,222 @@ __device__ __forceinline__ void pull_body(const EmapArgs &A, const Op<R> &op, Pu
     if (A.out_cnt) flush_counts<BLOCK>(A, nv, ne, sc);
 }
 
+// Full scan (no candidate list): a warp walks a contiguous range of 32-vertex
+// words.  What the per-vertex record settles is settled word by word; rows
+// still open are put aside (vertex, value, edges used) and looked at 32 at a
+// time, so that a warp pays the chain of accesses of an open row, and the
+// instructions around it, once per 32 of them and not once per word.  Levels
+// of 0.81 M and 2.1 M sources of a search over edgemap, directed ER 3 M x 16:
+// 173 and 53 -> 144 and 45 us; R-MAT 20, 0.24 M and 0.40 M: 46 and 34 -> 41 and
+// 31.  What is left is the instructions (all filters and relaxations are
+// decided at run time, 54 % of the issue slots) and the open rows' gathers.
+template <int R, bool SRCF, int BLOCK>
+__device__ __forceinline__ void pull_full(const EmapArgs &A, const Op<R> &op, PullSmem<BLOCK, false> &sm,
+                                          uint4 (&s_open)[BLOCK / 32][64]) {
+    using V = typename Op<R>::V;
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint64_t nw = (gridDim.x * BLOCK) >> 5;
+    const uint64_t gw = (blockIdx.x * BLOCK + threadIdx.x) >> 5;
+    uint4 *open = s_open[threadIdx.x >> 5];
+    uint32_t nopen = 0, wlo = 0, whi = 0;
+    dev::balanced_range(A.word_prefix, (A.n + 31u) >> 5, gw, nw, wlo, whi);
+    unsigned long long nv = 0, ne = 0, sc = 0;
+    dev::WarpAppender<256> keepers{sm.cand[threadIdx.x >> 5], 0, A.cand_out, A.cand_out_n};
+    const bool has_rec = A.first_in || A.first1;
+    const bool lazy = has_rec && A.lazy_off;
+    // d's value written and recorded
+    auto settle = [&](uint32_t d, V best, bool changed, uint64_t deg) {
+        bool rec = false;
+        if (changed) {
+            op.a[d] = best;
+            if (A.record == GG_RECORD_NE_PREV) {
+                // level-synchronous: d was unvisited, so its prev equals the
+                // value replaced; prev is neither read nor written
+                if (R == GG_RELAX_MIN_PLUS1_I32 && op.level_sync) {
+                    rec = true;
+                } else if constexpr (R == GG_RELAX_OR_U32) {
+                    // prev may be the relax's source: the copy runs after the step
+                    rec = best != op.prev[d];
+                } else if (best != op.prev[d]) {
+                    op.prev[d] = best;
+                    rec = true;
+                }
+            } else if (A.record == GG_RECORD_REDUCTION) {
+                rec = true;
+            } else if (A.record == GG_RECORD_AT_FLOOR) {
+                rec = (int64_t)best == op.fk;  // COUNT_DOWN: counted down to the floor now
+            }
+        }
+        if (rec) {
+            // the output list is built from the bitmap only if a push needs it;
+            // the out-degree of a symmetric graph's vertex is its row's length
+            nv++;
+            ne += A.off == A.in_off ? deg : A.off[d + 1] - A.off[d];
+        }
+        return rec;
+    };
+    // the last cnt of the rows put aside, a lane each
+    auto drain = [&](uint32_t cnt) {
+        __syncwarp();
+        nopen -= cnt;
+        const bool have = lane < cnt;
+        uint32_t d = 0;
+        V best = Op<R>::none();
+        bool changed = false;
+        uint64_t beg = 0, e = 0, end = 0;
+        if (have) {
+            const uint4 o = open[nopen + lane];
+            d = o.x;
+            best = (V)o.y;
+            changed = o.z >> 31;
+            beg = A.in_off[d];
+            end = A.in_off[d + 1];
+            e = beg + (o.z & 0x7FFFFFFFu);
+        }
+        __syncwarp();
+        const uint64_t from = e, lim = min(end, beg + (uint64_t)A.K);
+        bool act = have;
+        while (act && e < lim) {
+            const int c = (int)min((uint64_t)4, lim - e);
+            uint32_t sv[4];
+            bool inF[4];
+            V xv[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sv[j] = j < c ? __ldg(A.in_adj + e + j) : 0u;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                inF[j] = j < c && (!SRCF || dev::bit_test(A.in_bits, sv[j]));
+                xv[j] = j < c ? op.src_val(sv[j]) : Op<R>::none();
+            }
+            int used = c;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (j < c && act && inF[j] && op.better(xv[j], best)) {
+                    best = op.combine(best, xv[j]);
+                    changed = true;
+                    if (!op.dst_ok(best)) {
+                        act = false;
+                        used = j + 1;
+                    }
+                }
+            }
+            e += used;
+        }
+        sc += e - from;
+        unsigned pend = __ballot_sync(FULL, act && e < end);
+        while (pend) {
+            const int j = __ffs(pend) - 1;
+            pend &= pend - 1;
+            const uint64_t ej = __shfl_sync(FULL, e, j);
+            const uint64_t endj = __shfl_sync(FULL, end, j);
+            V bj = __shfl_sync(FULL, best, j);
+            bool chj = false, actj = true;
+            for (uint64_t base = ej; base < endj; base += 32) {
+                const uint64_t idx = base + lane;
+                bool ok = false;
+                V x = Op<R>::none();
+                if (idx < endj) {
+                    const uint32_t s = __ldg(A.in_adj + idx);
+                    if (!SRCF || dev::bit_test(A.in_bits, s)) {
+                        x = op.src_val(s);
+                        ok = op.better(x, bj);
+                    }
+                }
+                if (lane == 0) sc += min((uint64_t)32, endj - base);
+                const unsigned okm = __ballot_sync(FULL, ok);
+                if (okm) {
+                    bj = op.warp_merge(bj, ok, x, okm);
+                    chj = true;
+                    if (!op.dst_ok(bj)) {
+                        actj = false;
+                        break;
+                    }
+                }
+            }
+            if ((int)lane == j) {
+                best = bj;
+                changed = changed || chj;
+                act = actj;
+            }
+        }
+        const bool rec = have && settle(d, best, changed, end - beg);
+        if (rec && A.out_bits) atomicOr(A.out_bits + (d >> 5), 1u << (d & 31u));
+        // still a candidate: passes the filter
+        if (A.cand_out) keepers.push(have && act, d);
+    };
+    for (uint32_t w = wlo; w < whi; ++w) {
+        const uint64_t item = ((uint64_t)w << 5) + lane;
+        const bool valid = item < A.n;
+        const uint32_t d = (uint32_t)item;
+        V best = Op<R>::none();
+        uint4 f2 = make_uint4(0u, 0u, 0u, 0u);
+        uint64_t deg = 0;
+        if (valid) {
+            best = op.load(d);
+            if (has_rec) {
+                if (A.first1) {
+                    const uint2 r1 = A.first1[d];
+                    f2 = make_uint4(r1.x, 0xFFFFFFFFu, r1.y, 0xFFFFFFFFu);
+                } else {
+                    f2 = A.first_in[d];
+                }
+            }
+            deg = lazy ? (uint64_t)f2.z : A.in_off[d + 1] - A.in_off[d];
+        }
+        bool act = valid && op.dst_ok(best);
+        if constexpr (R == GG_RELAX_OR_U32) {
+            // a bitwise-or row has no early exit: long rows go to k_or_heavy_chunks
+            if (A.heavy_T && act && deg > A.heavy_T) act = false;
+        }
+        bool changed = false;
+        uint32_t used = 0;
+        if (has_rec && act && deg) {
+            // the row's first in-neighbours, loaded beside its value: the
+            // same edges in the same order as the row's
+            const int cnt = (int)min((uint64_t)A.rec_n, min(deg, (uint64_t)A.K));
+            const uint32_t sv[3] = {f2.x, f2.y, f2.w};
+            used = cnt;
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                if (j < cnt && act && (!SRCF || dev::bit_test(A.in_bits, sv[j]))) {
+                    const V x = op.src_val(sv[j]);
+                    if (op.better(x, best)) {
+                        best = op.combine(best, x);
+                        changed = true;
+                        if (!op.dst_ok(best)) {
+                            act = false;
+                            used = j + 1;
+                        }
+                    }
+                }
+            }
+            sc += used;
+        }
+        const bool later = act && used < deg;
+        const bool rec = valid && !later && settle(d, best, changed, deg);
+        const unsigned bits = __ballot_sync(FULL, rec);
+        if (A.out_bits && lane == 0) A.out_bits[w] = bits;
+        if (A.cand_out) keepers.push(valid && act && !later && deg, d);
+        const unsigned lm = __ballot_sync(FULL, later);
+        if (later)
+            open[nopen + __popc(lm & ((1u << lane) - 1u))] = make_uint4(d, (uint32_t)best, used | (changed ? 1u << 31 : 0u), 0u);
+        nopen += __popc(lm);
+        if (nopen >= 32) drain(32);
+    }
+    if (nopen) drain(nopen);
+    if (A.cand_out) keepers.flush();
+    if (A.out_cnt) flush_counts<BLOCK>(A, nv, ne, sc);
+}
+
 template <int R, bool SRCF, bool CAND, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, 6) k_pull(EmapArgs A, Op<R> op) {
     __shared__ PullSmem<BLOCK, false> sm;
-    pull_body<R, SRCF, CAND, BLOCK>(A, op, sm);
+    if constexpr (CAND) {
+        pull_body<R, SRCF, BLOCK>(A, op, sm);
+    } else {
+        __shared__ uint4 s_open[BLOCK / 32][64];
+        pull_full<R, SRCF, BLOCK>(A, op, sm, s_open);
+    }
 }
 
 // Bitwise-or pulls over the long rows (FMv's all-source steps): a warp per
@@ -2196,13 +2397,13 @@ __global__ void __launch_bounds__(kBlock, MINB) k_g_pull(GCtl *c) {
         bool pending;
         const uint32_t sn = stage_bitmap(sA.in_bits, ((uint64_t)sA.n + 31) / 32, c->stage_words, s_stage, &s_bar,
                                          &pending);
-        if (sA.rest_out) pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock, 1, true>(sA, sOp, sm, s_stage, sn);
-        else pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock, 0, true>(sA, sOp, sm, s_stage, sn);
+        if (sA.rest_out) pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock, 1, true>(sA, sOp, sm, s_stage, sn);
+        else pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock, 0, true>(sA, sOp, sm, s_stage, sn);
         stage_finish(c, &s_bar, pending);
     } else if (sA.rest_out) {
-        pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock, 1>(sA, sOp, sm);
+        pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock, 1>(sA, sOp, sm);
     } else {
-        pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock>(sA, sOp, sm);
+        pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock>(sA, sOp, sm);
     }
     kspan_end(c, s_it, &s_done);
 }
@@ -2238,10 +2439,10 @@ __global__ void __launch_bounds__(kBlock, MINB) k_g_pull2(GCtl *c) {
         bool pending;
         const uint32_t sn = stage_bitmap(sA.in_bits, ((uint64_t)sA.n + 31) / 32, c->stage_words, s_stage, &s_bar,
                                          &pending);
-        pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock, 2, true>(sA, sOp, sm, s_stage, sn);
+        pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock, 2, true>(sA, sOp, sm, s_stage, sn);
         stage_finish(c, &s_bar, pending);
     } else {
-        pull_body<GG_RELAX_MIN_PLUS1_I32, true, true, kBlock, 2>(sA, sOp, sm);
+        pull_body<GG_RELAX_MIN_PLUS1_I32, true, kBlock, 2>(sA, sOp, sm);
     }
     kspan_end(c, s_it, &s_done);
 }
@@ -3194,7 +3395,7 @@ gg_status gg_kcore(gg_graph *g, const gg_run_opts *o, gg_prop *coreness, uint32_
     RunTimer tm(ctx);
     uint32_t *count = (uint32_t *)coreness->d;
     // every step a sparse push and no per-step records wanted: the whole peel
-    // as one resident launch (R-MAT 20: 25.1 ms below, 7.5 ms there)
+    // as one resident launch (R-MAT 20: 24.4 ms below, 6.3 ms there)
     if (g->n && opt.threshold == GG_THRESH_ALWAYS_SPARSE && opt.variant == GG_VAR_AUTO && !opt.collect_stats) {
         bool ran = false;
         uint32_t big = 0;

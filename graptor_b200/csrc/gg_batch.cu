@@ -10,11 +10,10 @@
 //    Levels are written per (vertex, root): level[v*64 + i].
 //  * Personalized PageRank for up to 128 seeds: x_s <- alpha*e_s +
 //    (1-alpha)*A^T D^-1 x_s.  The contribution matrix c[v][s] = x_s[v]/deg(v)
-//    is stored in bfloat16, one 256-byte row per vertex, so every gathered
-//    edge is one coalesced row read by a warp (lane = 4 seeds); sums are
+//    is stored in bfloat16, one row of 16, 32, 64 or 128 seeds per vertex, so
+//    every gathered edge is one coalesced row (lane = 4 seeds); sums are
 //    float32.  Hub rows are cut into chunks (HeavyRows) summed by separate
-//    warps into float32 partials.  The iteration loop is captured once into a
-//    CUDA graph and launched as one graph.
+//    warps into float32 partials.  One launch per iteration.
 //  * Disjoint union of many graphs on the device (gg_graph_union), so BFS
 //    from every part's root and CC of every part run as one traversal.
 #include <cuda_bf16.h>

@@ -690,10 +690,12 @@ static gg_status gather_launch(gg_graph *g, const typename Store<DT>::T *contrib
 // Measured per iteration, the rest of it included, by rows -> by blocks:
 // R-MAT 24 FP32 with double sums 2.02 -> 1.66 ms, directed ER 2^24 x 32 BF16
 // 2.13 -> 1.42, ER 4 M x 64 FP32 1.06 -> 0.74, R-MAT 22 BF16 0.46 -> 0.36.
-// Of it k_pr_values 0.60 ms and k_pr_bins 0.94 ms (R-MAT 24), 1.6 and 1.8
-// times their DRAM time: their accesses to shared memory, some 3.7 banks deep
-// as the ids fall, and the loads take turns, with two CTAs per SM to overlap
-// them.  Bins of 16384 edges (3 CTAs) 2.4 ms: tiles, and with them the runs
+// Of it k_pr_values 0.60 ms and k_pr_bins 0.94 ms (R-MAT 24), 1.3 and 1.8
+// times their DRAM time: the pipes of L1 and shared memory, whose accesses
+// fall into some 3 banks deep where the ids lie at random, are busy for 69 %
+// (86 % with 16-bit values) and 63 % of it, the issue slots of the second for
+// 58 %, and its loads, sums and stores take turns with two CTAs per SM to
+// overlap them.  Bins of 16384 edges (3 CTAs) 2.4 ms: tiles, and with them the runs
 // read from DRAM, get shorter.  The values written by the first kernel in
 // bin order instead, so that the second reads them in one piece: 1.9 ms, and
 // 2.0 for BF16 (runs of half sectors).

@@ -632,12 +632,14 @@ __global__ void k_pr_init(XT<DT> *x, typename Store<DT>::T *contrib, const uint6
 
 constexpr int kBlock = 256;
 
-// The gather by blocks pays from some 50 M edges on (20 iterations, by rows
-// -> by blocks: R-MAT 20 with 31 M edges 3.3 -> 5.1 ms, ER 16 M 2.0 -> 1.9,
-// ER 63 M FP16 5.9 -> 4.5, R-MAT 22 x 8 FP32 6.4 -> 5.5), and its layout takes
-// the time of some 3 (ER) to 20 (R-MAT 24) iterations' gain to build: it is
-// built once a graph has been asked for that many iterations.
-constexpr uint64_t kBlockedEdges = 3ull << 24;
+// The gather by blocks pays from some 25 M edges on (20 iterations, by rows
+// -> by blocks, the first call of a graph with the layout's building: ER 16 M
+// 2.36 -> 2.67 ms and 2.00 -> 1.71 for the next, R-MAT 20 with 31 M edges 8.7
+// -> 8.1 and 3.31 -> 2.82, ER 63 M FP16 6.4 -> 5.6 and 5.9 -> 4.2, R-MAT 22 x 8
+// FP32 6.8 -> 6.5 and 6.4 -> 5.1).  The layout takes the time of some 3 (ER) to
+// 20 (R-MAT 24) iterations' gain to build: it is built once a graph has been
+// asked for that many iterations.
+constexpr uint64_t kBlockedEdges = 3ull << 23;
 constexpr uint64_t kBlockedIters = 16;
 
 static unsigned pr_grid(gg_ctx *ctx, uint64_t work) {

@@ -14,7 +14,7 @@
  * per chunk of a hub row), blocks_per_sm (CTAs per SM of the grid-stride
  * kernels), pr_stream (0 or 1, without effect: one PageRank gather
  * serves all rows), pr_blocks_per_sm (the PageRank kernels' grid cap, 16),
- * pr_blocked (1, the default: the PageRank gather of a graph of 50 M edges
+ * pr_blocked (1, the default: the PageRank gather of a graph of 25 M edges
  * or more goes by blocks of sources once 16 iterations have been asked of
  * the graph, with a layout of about 4.7 bytes an edge kept with it; 2:
  * wherever that layout can be built; 0: never), persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as

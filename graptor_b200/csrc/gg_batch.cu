@@ -286,7 +286,8 @@ struct PprArgs {
     HeavyRows H;
     float4 *partial;    // [nchunks][L] float4 per lane
     uint32_t *arrived;  // [nheavy] chunks of the row that are done; wraps to 0
-    uint32_t tickets;   // of the chunks, 32 / L each, then of the light rows, kPprRows<L> each
+    uint32_t rows;      // light rows per ticket
+    uint32_t tickets;   // of the chunks, 32 / L each, then of the light rows
     uint32_t *ticket;   // this iteration's; the next one's is set to 0
     uint32_t *next_ticket;
 };
@@ -343,12 +344,12 @@ __device__ __forceinline__ void ppr_finish(const PprArgs &A, uint32_t d, float4 
 //     vertex in the last iteration.
 // 20 iterations, before (a warp per row, 4 rows in flight, rows of 128 seeds
 // whatever their number, three launches) -> after: 128 seeds on R-MAT 18 x 16
-// 8.49 -> 4.89 ms, R-MAT 10 1.07 -> 0.71, ER 2^18 x 32 4.99 -> 5.05; 50 seeds
+// 8.49 -> 4.89 ms, R-MAT 10 1.07 -> 0.38, ER 2^18 x 32 4.99 -> 5.05; 50 seeds
 // on R-MAT 17 4.34 -> 2.02; 5 seeds on R-MAT 18 6.72 -> 2.04; 29 and 9 seeds
 // on directed ER 200001 x 12 2.09 -> 0.79 and 2.11 -> 0.54.
 constexpr int kPprBlock = 256;
 constexpr uint32_t kPprFlight = 16;
-// light rows per ticket
+// most light rows per ticket
 template <int L> constexpr uint32_t kPprRows = L == 32 ? 8 : 4 * (32 / L);
 
 // Rows as wide as a warp.
@@ -372,8 +373,8 @@ __global__ void __launch_bounds__(kPprBlock, 4) k_ppr_wide(PprArgs A) {
             len = (uint32_t)min((uint64_t)A.H.CH, A.in_off[d0 + 1] - e0);
             ids = A.in_adj + e0;
         } else {
-            d0 = (t - (uint32_t)A.H.nchunks) * kPprRows<32>;
-            rows = min(A.n - d0, kPprRows<32>);
+            d0 = (t - (uint32_t)A.H.nchunks) * A.rows;
+            rows = min(A.n - d0, A.rows);
             const uint64_t beg = __ldg(A.in_off + d0 + min(lane, rows)), end = __shfl_down_sync(FULL, beg, 1);
             if (lane < rows && end - beg <= A.H.T) len = (uint32_t)(end - beg);
             ids = A.in_adj + beg;
@@ -463,8 +464,8 @@ __global__ void __launch_bounds__(kPprBlock, 3) k_ppr_narrow(PprArgs A) {
                 ids += e0;
             }
         } else {
-            rows = kPprRows<L>;
-            const uint64_t at = (uint64_t)(t - nct) * kPprRows<L> + wl;
+            rows = A.rows;
+            const uint64_t at = (uint64_t)(t - nct) * A.rows + wl;
             d = (uint32_t)at;
             if (wl < rows && at < A.n) {
                 const uint64_t beg = __ldg(A.in_off + at), end = __ldg(A.in_off + at + 1);
@@ -573,9 +574,15 @@ static void ppr_run(gg_ctx *ctx, PprArgs A, uint2 *c0, uint2 *c1, uint2 *x, uint
     if constexpr (L == 32) step = k_ppr_wide;
     else step = k_ppr_narrow<L>;
     constexpr uint32_t G = 32 / L;
-    A.tickets = (uint32_t)((A.H.nchunks + G - 1) / G + ((uint64_t)A.n + kPprRows<L> - 1) / kPprRows<L>);
-    const unsigned grid = (unsigned)std::min<uint64_t>(
-        (uint64_t)ctx->sm_count * resident_ctas((const void *)step, kPprBlock), ((uint64_t)A.tickets + 7) / 8);
+    const uint64_t cap = (uint64_t)ctx->sm_count * resident_ctas((const void *)step, kPprBlock);
+    // fewer rows per ticket where warps would go without any (always the most ->
+    // so: ER 1204 x 45, 99 seeds, 14 iterations 0.355 -> 0.122 ms, R-MAT 10, 128
+    // seeds, 20 iterations 0.67 -> 0.38) (ER 1204 x 45, 99
+    // seeds, 14 iterations: @@)
+    A.rows = G * (uint32_t)std::max<uint64_t>(
+                     1, std::min<uint64_t>(kPprRows<L> / G, A.n / (G * cap * (kPprBlock / 32))));
+    A.tickets = (uint32_t)((A.H.nchunks + G - 1) / G + ((uint64_t)A.n + A.rows - 1) / A.rows);
+    const unsigned grid = (unsigned)std::min<uint64_t>(cap, ((uint64_t)A.tickets + 7) / 8);
     for (int it = 0; it < iters; ++it) {
         A.cin = (it & 1) ? c1 : c0;
         A.cout = it + 1 == iters ? nullptr : (it & 1) ? c0 : c1;

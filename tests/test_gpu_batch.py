@@ -125,6 +125,20 @@ def test_ppr_row_widths(ctx, hub, k):
     G.close()
 
 
+@pytest.mark.parametrize("n", [9471, 9473, 60001])
+def test_ppr_rows_per_ticket(ctx, n):
+    # vertex counts below and above those from which a warp takes several rows
+    rng = np.random.default_rng(n)
+    g = O.from_edges(n, [(int(u), int(v)) for u, v in rng.integers(0, n, (3 * n, 2)) if u != v], symmetric=False)
+    G = upload(ctx, g, False)
+    seeds = nonisolated(g, 72, 3)
+    x = gg.ppr(G, seeds, alpha=0.15, iters=4)
+    assert np.abs(x - B.ppr_bf16(g, seeds, 0.15, 4)).sum(0).max() < PPR_L1_VS_BF16_EMUL
+    for k in (5, 20, 40):
+        assert np.array_equal(gg.ppr(G, seeds[:k], alpha=0.15, iters=4), x[:, :k])
+    G.close()
+
+
 def test_ppr_zero_iterations_is_teleport(ctx):
     g = O.rmat(8, 2000, 2)
     G = upload(ctx, g)

@@ -7,6 +7,11 @@
 // GG_ERR_TIMEOUT and the context stays usable.  Co-residency of all CTAs is
 // guaranteed by the cooperative launch, so in normal operation the deadline
 // is never reached.
+//
+// A CTA decides as one whether it goes on: its first thread reads the error
+// word, once, and the barrier that releases the others hands them what it saw
+// (read by every thread, an error set meanwhile by another CTA would send some
+// threads of a warp out and let the others on into its shuffles).
 #pragma once
 #include "gg_internal.cuh"
 
@@ -26,6 +31,7 @@ struct Barrier {
 };
 
 __device__ __forceinline__ bool sync(Barrier *b, unsigned long long timeout_ns) {
+    bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -47,9 +53,9 @@ __device__ __forceinline__ bool sync(Barrier *b, unsigned long long timeout_ns) 
             }
         }
         __threadfence();
+        ok = *(volatile unsigned int *)&b->err == 0;
     }
-    __syncthreads();
-    return *(volatile unsigned int *)&b->err == 0;
+    return __syncthreads_and(ok);
 }
 
 // Barrier on one counter of arrivals that only grows: the e-th barrier is
@@ -86,9 +92,7 @@ __device__ __forceinline__ bool arrive_and_wait(Arrivals *b, unsigned long long 
 __device__ __forceinline__ bool sync(Arrivals *b, unsigned long long &epoch, unsigned long long timeout_ns) {
     __syncthreads();
     ++epoch;
-    if (threadIdx.x == 0) arrive_and_wait(b, epoch, timeout_ns);
-    __syncthreads();
-    return *(volatile unsigned int *)&b->err == 0;
+    return __syncthreads_and(threadIdx.x != 0 || arrive_and_wait(b, epoch, timeout_ns));
 }
 
 }  // namespace grid

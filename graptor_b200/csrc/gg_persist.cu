@@ -83,8 +83,10 @@ __device__ __forceinline__ unsigned long long globaltimer() {
 template <typename T> __device__ __forceinline__ T ldcg(const T *p) { return __ldcg(p); }
 
 // Bounded grid barrier (sense = generation counter).  Returns false when any
-// CTA has flagged an error (timeout): the caller then returns.
+// CTA has flagged an error (timeout), to all threads of a CTA alike: the
+// caller then returns.
 __device__ __forceinline__ bool grid_barrier(PState *st, unsigned long long timeout_ns) {
+    bool ok = true;
     __syncthreads();
     if (threadIdx.x == 0) {
         __threadfence();
@@ -106,9 +108,9 @@ __device__ __forceinline__ bool grid_barrier(PState *st, unsigned long long time
             }
         }
         __threadfence();
+        ok = *(volatile unsigned int *)&st->err == 0;
     }
-    __syncthreads();
-    return *(volatile unsigned int *)&st->err == 0;
+    return __syncthreads_and(ok);
 }
 
 // ---- relax semantics (same table as the host-driven kernels) --------------

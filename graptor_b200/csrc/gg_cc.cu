@@ -52,6 +52,15 @@ struct CcState {
     uint32_t moved[3];  // a doubling round changed a label (three in turn)
 };
 
+// What the host reads after a run: the records, written by the first CTA at
+// its end, and a word of their own for the CTAs that gave up at a barrier (the
+// first one may have left the last barrier in time and write its records all
+// the same).
+struct CcRecord {
+    PState st;
+    unsigned int gave_up;
+};
+
 struct CcArgs {
     const uint64_t *off;
     const uint32_t *adj;
@@ -68,7 +77,7 @@ struct CcArgs {
     uint32_t *label;
     CcState *cs;
     PState *st;   // records
-    PState *rec;  // page-locked copy of them, or null
+    CcRecord *rec;  // page-locked copy of them, or null
     unsigned long long timeout_ns;
 };
 
@@ -268,7 +277,10 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
         ok = grid::sync(&A.cs->bar, epoch, A.timeout_ns);
     }
     if (!ok) {
-        if (threadIdx.x == 0) atomicOr(&A.st->err, DEV_ERR_TIMEOUT);
+        if (threadIdx.x == 0) {
+            atomicOr(&A.st->err, DEV_ERR_TIMEOUT);
+            if (A.rec) *(volatile unsigned int *)&A.rec->gave_up = 1u;
+        }
         return;
     }
     // ---- finish: every label written once, by its own thread, with its root
@@ -316,7 +328,7 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
     if (!A.rec) return;
     __syncthreads();
     const uint4 *src = (const uint4 *)A.st;
-    for (uint32_t i = threadIdx.x; i < sizeof(PState) / 16; i += kCB) ((uint4 *)A.rec)[i] = src[i];
+    for (uint32_t i = threadIdx.x; i < sizeof(PState) / 16; i += kCB) ((uint4 *)&A.rec->st)[i] = src[i];
 }
 
 __global__ void k_cc_start(CcState *cs, PState *st, int searched) {
@@ -334,7 +346,7 @@ __global__ void k_cc_start(CcState *cs, PState *st, int searched) {
 
 struct CcRes {
     CcState *cs = nullptr;
-    PState *h_rec = nullptr, *d_rec = nullptr;  // page-locked, mapped
+    CcRecord *h_rec = nullptr, *d_rec = nullptr;  // page-locked, mapped
 };
 
 void cc_resident_free(gg_graph *g) {
@@ -362,7 +374,7 @@ gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok) {
         if (!r) return GG_ERR_OOM;
         g->cc_res = r;
         if (cudaMalloc(&r->cs, sizeof(CcState)) != cudaSuccess ||
-            cudaHostAlloc(&r->h_rec, sizeof(PState), cudaHostAllocMapped) != cudaSuccess ||
+            cudaHostAlloc(&r->h_rec, sizeof(CcRecord), cudaHostAllocMapped) != cudaSuccess ||
             cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0) != cudaSuccess) {
             const cudaError_t e = cudaGetLastError();
             cc_resident_free(g);
@@ -421,11 +433,15 @@ gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *ite
     gg_ctx *ctx = g->ctx;
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
     PState *st = (PState *)g->pstate;
-    PState &hs = *((CcRes *)g->cc_res)->h_rec;
+    CcRecord &rec = *((CcRes *)g->cc_res)->h_rec;
+    PState &hs = rec.st;
     hs.iterations = -1;  // written by the run's end
+    rec.gave_up = 0;
     GG_CHECK(cc_resident_enqueue(g, label, st, true));
     GG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    if (hs.iterations < 0) return set_error(ctx, GG_ERR_TIMEOUT, "gg_cc: grid barrier timed out");
+    // (the search's error word is in the records, which follow it on the stream)
+    if (hs.iterations < 0 || rec.gave_up || (hs.err & DEV_ERR_TIMEOUT))
+        return set_error(ctx, GG_ERR_TIMEOUT, "gg_cc: grid barrier timed out");
     *iters_out = hs.iterations;
     if (stats) {
         stats->vertices_reached = hs.reached_v;

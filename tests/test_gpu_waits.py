@@ -47,3 +47,10 @@ def runs_out(ctx, short_wait, kind, call):
 @pytest.mark.parametrize("call", list(CALLS))
 def test_wait_that_runs_out_is_reported(ctx, short_wait, kind, call):
     runs_out(ctx, short_wait, kind, CALLS[call])
+
+
+@pytest.mark.parametrize("kind", ["rmat", "grid"])  # with the search, and hooking alone
+def test_cc_wait_that_runs_out_is_reported(ctx, short_wait, kind):
+    """Labels are not returned as good where any CTA of the run or of its
+    search gave up, though the first one may have come through."""
+    runs_out(ctx, short_wait, kind, lambda g: g.cc())

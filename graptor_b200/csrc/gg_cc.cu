@@ -50,6 +50,7 @@ struct CcState {
     uint32_t smallest;
     uint32_t nleft;  // vertices listed in `left`
     uint32_t moved[3];  // a doubling round changed a label (three in turn)
+    unsigned long long hooked;  // edges that the hooks looked at
 };
 
 // What the host reads after a run: the records, written by the first CTA at
@@ -164,6 +165,7 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
     }
     const unsigned long long t1 = grid::globaltimer();
     if (ok) {
+        unsigned long long looked = 0;  // edges, this thread's share
         // ---- hook.  With a giant component its vertices are done: an edge
         // that leaves the part reached is taken from its other end, and all of
         // the other vertices' edges are.  Without one, an edge is taken from
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
                     e1 = min(e0 + A.H.CH, A.off[v + 1]);
                 }
             }
+            looked += e1 - e0;
             for (unsigned todo = __ballot_sync(FULL, e0 < e1); todo; todo &= todo - 1) {
                 const int j = __ffs(todo) - 1;
                 const uint32_t vj = __shfl_sync(FULL, v, j);
@@ -247,6 +250,7 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
                     deg = A.off[v[u] + 1] - beg;
                     if (deg > A.H.T) deg = 0;  // above
                 }
+                looked += deg;
                 uint32_t incl = (uint32_t)deg;
 #pragma unroll
                 for (int o = 1; o < 32; o <<= 1) {
@@ -274,6 +278,8 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
                 }
             }
         }
+        looked = dev::block_sum<unsigned long long, kCB>(looked);
+        if (threadIdx.x == 0 && looked) atomicAdd(&A.cs->hooked, looked);
         ok = grid::sync(&A.cs->bar, epoch, A.timeout_ns);
     }
     if (!ok) {
@@ -309,6 +315,10 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
         PState *st = A.st;
         // CCv's road-network test: few zeros
         const bool road = (giant && top == 0 ? reached : 1ull) * 10 < (unsigned long long)A.n;
+        // edges examined: the search's or, without a giant component, each
+        // vertex's first one as well; then those of the hooks
+        unsigned long long first = giant ? 0ull : nn;
+        for (int i = 0; i < (A.searched ? st->iterations : 0); ++i) first += st->scanned[i];
         st->iterations = 2;
         st->reached_v = A.n;
         st->reached_e = A.m;
@@ -318,8 +328,8 @@ __global__ void __launch_bounds__(kCB, 2) k_cc_run(CcArgs A) {
             st->nactv[i] = A.n;
             st->nacte[i] = A.m;
         }
-        st->scanned[0] = A.n;
-        st->scanned[1] = giant ? A.n : A.m;
+        st->scanned[0] = first;
+        st->scanned[1] = __ldcg(&A.cs->hooked);
         st->t_ns[0] = t0;
         st->t_ns[1] = t1;
         st->t_ns[2] = st->t_end = grid::globaltimer();
@@ -342,6 +352,7 @@ __global__ void k_cc_start(CcState *cs, PState *st, int searched) {
     cs->smallest = 0xFFFFFFFFu;
     cs->nleft = 0;
     cs->moved[0] = cs->moved[1] = cs->moved[2] = 0;
+    cs->hooked = 0;
 }
 
 struct CcRes {

@@ -408,8 +408,9 @@ GG_API gg_status gg_bfs_parent(gg_graph *g, uint32_t root, const gg_run_opts *o,
  * minimum id of each component); otherwise label propagation continues.
  * By default a symmetric graph's components come from a short search from its
  * vertex of largest degree and hooking of what that did not reach (knob
- * resident); st then holds two records, the second a GG_VAR_HOOK where the
- * labels pass the road-network test.  Runs that collect per-step records, fix
+ * resident); st then holds two records: the search and the first labels, and
+ * the hooks, reported as GG_VAR_HOOK where the labels pass the road-network
+ * test and as GG_VAR_PULL_DENSE elsewhere.  Runs that collect per-step records, fix
  * a variant or take another threshold than DEFAULT or FRAC propagate labels. */
 GG_API gg_status gg_cc(gg_graph *g, const gg_run_opts *o, gg_prop *label, uint32_t *host_label,
                        gg_run_stats *st);

@@ -138,3 +138,39 @@ def test_resident_cc_exact(ctx, knobs, kind):
     assert np.array_equal(lb, want)
     assert np.array_equal(lv, np.minimum(O.bfs_level(og, 0), O.bfs_level(og, 5)))
     g.close()
+
+
+@pytest.mark.parametrize("kind", ["core_and_tail", "giant_without_0", "many", "edgeless", "star"])
+def test_resident_cc_counts_the_edges_it_examines(ctx, knobs, kind):
+    """scanned[0]: the search's edges (as a BFS of at most ten steps counts
+    them) and, where it found no giant component, every vertex's first edge;
+    scanned[1]: those of the rows that hook."""
+    if kind == "star":
+        og = O.from_edges(3001, [(7, i) for i in range(3001) if i != 7])
+    else:
+        og = cc_graph(kind)
+    g = ctx.upload(og.off, og.adj)
+    gg.tuning_set("resident", 1)
+    st, bfs = gg.RunStats(), gg.RunStats()
+    assert np.array_equal(g.cc(stats=st), O.cc(og))
+    assert st.iterations == 2
+    assert st.scanned_edges == st.scanned[0] + st.scanned[1]
+    deg = og.outdeg()
+    hub = int(np.argmax(deg))
+    level = g.bfs_level(hub, stats=bfs)
+    searched = int(deg[hub]) * (og.m / og.n) ** 2 >= 1024 if og.n else False
+    giant = 2 * int((level <= og.n).sum()) >= int((deg > 0).sum())
+    if kind == "star":  # the search reaches all of it: nothing left to hook
+        assert searched and bfs.iterations <= 10
+        assert (st.scanned[0], st.scanned[1]) == (bfs.scanned_edges, 0)
+    elif kind == "edgeless":
+        assert (st.scanned[0], st.scanned[1]) == (0, 0)
+    elif not giant:  # (the hub of giant_without_0 is a star's): every edge is looked at
+        assert st.scanned[1] == og.m
+        assert st.scanned[0] >= int((deg > 0).sum())
+    else:
+        # rows outside the part reached (the search may stop before its end)
+        out = int(deg[level > og.n].sum())
+        assert searched and out <= st.scanned[1] < og.m // 2
+        assert 0 < st.scanned[0] <= bfs.scanned_edges
+    g.close()

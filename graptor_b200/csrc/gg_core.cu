@@ -32,6 +32,7 @@ gg_status set_error(gg_ctx *ctx, gg_status s, const std::string &msg) {
 
 gg_status cuda_error(gg_ctx *ctx, cudaError_t e, const char *what) {
     std::string m = std::string(what) + ": " + cudaGetErrorString(e);
+    cudaGetLastError();  // reported here: not again by the next launch
     if (e == cudaErrorMemoryAllocation) return set_error(ctx, GG_ERR_OOM, m);
     return set_error(ctx, GG_ERR_CUDA, m);
 }

@@ -654,11 +654,7 @@ gg_status bfs_resident_prepare(gg_graph *g, bool *ok) {
         GG_CHECK(frontier_alloc_bins(f));
         GG_CHECK(frontier_alloc_bitmap(f));
     }
-    CandLists &cl = g->cand;
-    if (!cl.list[0]) {
-        for (auto &l : cl.list) GG_CUDA(ctx, cudaMalloc(&l, ((size_t)g->n + 1) * 4));
-        GG_CUDA(ctx, cudaMalloc(&cl.cnt, 2 * sizeof(uint64_t)));
-    }
+    GG_CHECK(cand_lists_alloc(g));
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
     if (!graph_items(g)) return GG_OK;
     if (!g->bfs_res) {

@@ -1523,6 +1523,23 @@ gg_status frontier_alloc_bitmap(gg_frontier *f) {
     return GG_OK;
 }
 
+// Both candidate lists and their counters, or none of them: a run takes them
+// all for there when the first one is.
+gg_status cand_lists_alloc(gg_graph *g) {
+    CandLists &c = g->cand;
+    if (c.list[0]) return GG_OK;
+    const size_t bytes = ((size_t)g->n + 1) * 4;
+    cudaError_t e = cudaMalloc(&c.list[0], bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&c.list[1], bytes);
+    if (e == cudaSuccess) e = cudaMalloc(&c.cnt, 2 * sizeof(uint64_t));
+    if (e == cudaSuccess) return GG_OK;
+    cudaFree(c.list[0]);
+    cudaFree(c.list[1]);
+    c.list[0] = c.list[1] = nullptr;
+    c.cnt = nullptr;
+    return cuda_error(g->ctx, e, "pull candidates");
+}
+
 gg_status frontier_reset_counts(gg_frontier *f) {
     GG_CUDA(f->g->ctx, cudaMemsetAsync(f->d_cnt, 0, FC_WORDS * sizeof(uint64_t), f->g->ctx->stream));
     f->host_valid = false;

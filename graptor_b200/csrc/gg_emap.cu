@@ -1849,10 +1849,7 @@ struct CandScope {
     explicit CandScope(gg_graph *gr) : g(gr) {}
     gg_status open() {
         CandLists &c = g->cand;
-        if (!c.list[0]) {
-            for (auto &l : c.list) GG_CUDA(g->ctx, cudaMalloc(&l, ((size_t)g->n + 1) * 4));
-            GG_CUDA(g->ctx, cudaMalloc(&c.cnt, 2 * sizeof(uint64_t)));
-        }
+        GG_CHECK(cand_lists_alloc(g));
         c.cur = 0;
         c.valid = false;
         c.host_n = UINT64_MAX;
@@ -2802,10 +2799,7 @@ gg_status graph_bfs_level(gg_graph *g, uint32_t root, const gg_run_opts &opt, gg
         f->has_list = f->has_bitmap = f->all = false;
     }
     CandLists &cl = g->cand;
-    if (!cl.list[0]) {
-        for (auto &l : cl.list) GG_CUDA(ctx, cudaMalloc(&l, ((size_t)g->n + 1) * 4));
-        GG_CUDA(ctx, cudaMalloc(&cl.cnt, 2 * sizeof(uint64_t)));
-    }
+    GG_CHECK(cand_lists_alloc(g));
     const Tuning &t = tuning();
     // configuration part of the control block (everything before the records)
     GCtl &h = *gb->h_up;  // the previous run's upload finished before it returned

@@ -218,6 +218,7 @@ void host_stage_free(gg_ctx *ctx);
 gg_status graph_scratch(gg_graph *g, size_t bytes, void **p);
 gg_status frontier_alloc_bins(gg_frontier *f);
 gg_status frontier_alloc_bitmap(gg_frontier *f);
+gg_status cand_lists_alloc(gg_graph *g);
 gg_status frontier_fetch_counts(gg_frontier *f);     // device -> host (syncs)
 gg_status frontier_ensure_bitmap(gg_frontier *f);    // from list
 gg_status frontier_ensure_list(gg_frontier *f);      // from bitmap / all

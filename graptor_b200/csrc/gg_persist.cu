@@ -1518,10 +1518,7 @@ gg_status persistent_enqueue(gg_graph *g, const gg_emap_desc &d, int level_k, bo
         GG_CHECK(frontier_alloc_bitmap(f));
     }
     CandLists &c = g->cand;
-    if (!c.list[0]) {
-        for (auto &l : c.list) GG_CUDA(ctx, cudaMalloc(&l, ((size_t)g->n + 1) * 4));
-        GG_CUDA(ctx, cudaMalloc(&c.cnt, 2 * sizeof(uint64_t)));
-    }
+    GG_CHECK(cand_lists_alloc(g));
     PState *st = (PState *)state;
     const size_t words = ((size_t)g->n + 31) / 32 + 1;
     std::memset(&P, 0, sizeof(P));
@@ -1798,11 +1795,7 @@ gg_status batch_bfs_cc(gg_graph *g, const uint32_t *roots, uint32_t k, gg_prop *
         GG_CHECK(frontier_alloc_bins(f));
         GG_CHECK(frontier_alloc_bitmap(f));
     }
-    CandLists &c = g->cand;
-    if (!c.list[0]) {
-        for (auto &l : c.list) GG_CUDA(ctx, cudaMalloc(&l, ((size_t)g->n + 1) * 4));
-        GG_CUDA(ctx, cudaMalloc(&c.cnt, 2 * sizeof(uint64_t)));
-    }
+    GG_CHECK(cand_lists_alloc(g));
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
     if (!g->pstate2) GG_CUDA(ctx, cudaMalloc(&g->pstate2, sizeof(PState)));
     void *merge;

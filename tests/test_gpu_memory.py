@@ -53,3 +53,36 @@ def test_an_error_is_reported_once(ctx):
         assert e.value.status == gg.GG_ERR_OOM
         assert np.array_equal(g.bfs_level(0), want)
     g.close()
+
+
+@pytest.mark.parametrize("resident", [0])
+def test_buffers_that_fit_in_part(ctx, resident):
+    """First calls with room for ever more of their buffers: the levels or
+    GG_ERR_OOM, and the levels from the next call, whichever buffer was the
+    one that did not fit (two frontiers of 50 MiB, two candidate lists, level
+    and prev of 17 MiB each, 34 MiB of items)."""
+    n = 1 << 22
+    old = gg.tuning_get("resident")
+    gg.tuning_set("resident", resident)
+    try:
+        want, kept = None, 0
+        for left in range(4, 232, 12):
+            g = ctx.rmat(22, n, seed=2)
+            with Fill(left * MB):
+                try:
+                    kept = g.bfs_level(0)
+                except gg.GGError as e:
+                    assert e.status == gg.GG_ERR_OOM
+                    kept = None
+            got = g.bfs_level(0)
+            want = got if want is None else want
+            assert np.array_equal(got, want)
+            assert kept is None or np.array_equal(kept, want), left
+            g.close()
+        assert kept is not None
+        g = ctx.rmat(22, n, seed=2)
+        off, adj = g.download()
+        assert np.array_equal(want, O.bfs_level(O.Graph(n, off, adj), 0))
+        g.close()
+    finally:
+        gg.tuning_set("resident", old)

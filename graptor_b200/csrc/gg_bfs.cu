@@ -643,11 +643,8 @@ void bfs_resident_free(gg_graph *g) {
     g->bfs_res = nullptr;
 }
 
-// Buffers for a run on g.  *ok = false (and nothing kept) where they do not
-// fit in memory: the caller takes another driver.
-gg_status bfs_resident_prepare(gg_graph *g, bool *ok) {
+static gg_status bfs_resident_buffers(gg_graph *g) {
     gg_ctx *ctx = g->ctx;
-    *ok = false;
     for (auto &f : g->tmp_front)
         if (!f) GG_CHECK(gg_frontier_create(g, &f));
     for (auto *f : g->tmp_front) {
@@ -656,22 +653,38 @@ gg_status bfs_resident_prepare(gg_graph *g, bool *ok) {
     }
     GG_CHECK(cand_lists_alloc(g));
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
-    if (!graph_items(g)) return GG_OK;
-    if (!g->bfs_res) {
-        BfsRes *r = new (std::nothrow) BfsRes;
-        if (!r) return GG_ERR_OOM;
-        g->bfs_res = r;
-        const size_t nw4 = ((size_t)g->n + 127) / 128;
-        if (cudaMalloc(&r->bs, sizeof(BState)) != cudaSuccess || cudaMalloc(&r->bits, 3 * nw4 * 16) != cudaSuccess ||
-            cudaHostAlloc(&r->h_rec, sizeof(PState), cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0) != cudaSuccess) {
-            cudaGetLastError();
-            bfs_resident_free(g);
-            return GG_OK;
-        }
-    }
-    *ok = true;
+    GG_CHECK(graph_items(g));
+    if (g->bfs_res) return GG_OK;
+    BfsRes *r = new (std::nothrow) BfsRes;
+    if (!r) return GG_ERR_OOM;
+    g->bfs_res = r;
+    const size_t nw4 = ((size_t)g->n + 127) / 128;
+    cudaError_t e = cudaMalloc(&r->bs, sizeof(BState));
+    if (e == cudaSuccess) e = cudaMalloc(&r->bits, 3 * nw4 * 16);
+    if (e == cudaSuccess) e = cudaHostAlloc(&r->h_rec, sizeof(PState), cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0);
+    if (e == cudaSuccess) return GG_OK;
+    bfs_resident_free(g);
+    return cuda_error(ctx, e, "resident BFS");
+}
+
+// What the resident runs of g allocated for themselves goes back: the drivers
+// taken instead need room too (their frontiers and candidate lists are the same).
+gg_status resident_give_up(gg_graph *g, gg_status s) {
+    if (s != GG_ERR_OOM) return s;
+    bfs_resident_free(g);
+    cc_resident_free(g);
+    cudaFree(g->items);
+    g->items = nullptr;
     return GG_OK;
+}
+
+// Buffers for a run on g.  *ok = false (and nothing kept but what other
+// drivers use) where they do not fit in memory: the caller takes another one.
+gg_status bfs_resident_prepare(gg_graph *g, bool *ok) {
+    const gg_status s = bfs_resident_buffers(g);
+    *ok = s == GG_OK;
+    return resident_give_up(g, s);
 }
 
 static gg_status bfs_args(gg_graph *g, gg_prop *level, const gg_run_opts &opt, PState *st, BArgs &A) {
@@ -688,7 +701,7 @@ static gg_status bfs_args(gg_graph *g, gg_prop *level, const gg_run_opts &opt, P
     A.m = g->m;
     A.level = (int32_t *)level->d;
     for (int i = 0; i < 3; ++i) A.bits[i] = r->bits + (size_t)i * A.nw4 * 4;
-    A.items = item_lists(g, graph_items(g));
+    A.items = item_lists(g, (unsigned long long *)g->items);
     A.cand[0] = g->cand.list[0];
     A.cand[1] = g->cand.list[1];
     A.nonisolated = g->nonisolated;

@@ -369,34 +369,40 @@ void cc_resident_free(gg_graph *g) {
     g->cc_res = nullptr;
 }
 
+// The run's own buffers, and those of the search, its levels among them.
+static gg_status cc_resident_buffers(gg_graph *g) {
+    if (!g->cc_res) {
+        CcRes *r = new (std::nothrow) CcRes;
+        if (!r) return GG_ERR_OOM;
+        g->cc_res = r;
+        cudaError_t e = cudaMalloc(&r->cs, sizeof(CcState));
+        if (e == cudaSuccess) e = cudaHostAlloc(&r->h_rec, sizeof(CcRecord), cudaHostAllocMapped);
+        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0);
+        if (e != cudaSuccess) {
+            cc_resident_free(g);
+            return cuda_error(g->ctx, e, "resident CC");
+        }
+    }
+    bool search;
+    GG_CHECK(bfs_resident_prepare(g, &search));
+    if (!search) return GG_ERR_OOM;
+    gg_prop *level;
+    return run_tmp_prop(g, 1, GG_I32, &level);
+}
+
 // Whether CC of g with these options runs here, its buffers made: symmetric
 // graphs with the threshold's choice of variants (which no pass here takes)
-// and no per-step records wanted.
+// and no per-step records wanted.  Not where the buffers do not fit in memory.
 gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok) {
-    gg_ctx *ctx = g->ctx;
     const Tuning &t = tuning();
     *ok = false;
     if (!g->symmetric || g->n == 0 || !t.resident || !(t.persistent & 4) || t.cc_hook != 1 || (t.fusion & 4) ||
         g->force_iter >= 0 || opt.variant != GG_VAR_AUTO || opt.collect_stats ||
         (opt.threshold != GG_THRESH_DEFAULT && opt.threshold != GG_THRESH_FRAC))
         return GG_OK;
-    if (!g->cc_res) {
-        CcRes *r = new (std::nothrow) CcRes;
-        if (!r) return GG_ERR_OOM;
-        g->cc_res = r;
-        if (cudaMalloc(&r->cs, sizeof(CcState)) != cudaSuccess ||
-            cudaHostAlloc(&r->h_rec, sizeof(CcRecord), cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0) != cudaSuccess) {
-            const cudaError_t e = cudaGetLastError();
-            cc_resident_free(g);
-            return cuda_error(ctx, e, "gg_cc");
-        }
-    }
-    // the search's buffers, its levels among them
-    GG_CHECK(bfs_resident_prepare(g, ok));
-    gg_prop *level;
-    if (*ok) GG_CHECK(run_tmp_prop(g, 1, GG_I32, &level));
-    return GG_OK;
+    const gg_status s = cc_resident_buffers(g);
+    *ok = s == GG_OK;
+    return resident_give_up(g, s);
 }
 
 // Enqueues the run with its records in `st` (and, with to_host, copied to the

@@ -252,6 +252,7 @@ gg_status bfs_resident_multi(gg_graph *g, gg_prop *level, const uint32_t *d_root
 gg_status bfs_resident_search(gg_graph *g, gg_prop *level, uint32_t root, int steps, unsigned long long give_up,
                               PState *st);
 void bfs_resident_free(gg_graph *g);
+gg_status resident_give_up(gg_graph *g, gg_status s);
 gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok);
 gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *iters_out);
 gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_host);

@@ -24,9 +24,8 @@ inline uint64_t items_cap(const gg_graph *g, int kind) {
     default: return 2 * (g->m / kHuge) + 2;
     }
 }
-// The graph's item buffer, kind by kind (allocated on first use; null where
-// it does not fit in memory).
-unsigned long long *graph_items(gg_graph *g);
+// The graph's item buffer g->items, kind by kind, allocated on first use.
+gg_status graph_items(gg_graph *g);
 
 struct ItemLists {
     unsigned long long *p[IT_KINDS];

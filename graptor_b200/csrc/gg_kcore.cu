@@ -235,24 +235,25 @@ __global__ void __launch_bounds__(256) k_kc_start(const uint64_t *__restrict__ o
     if (threadIdx.x == 0 && k) atomicAdd(&st->many, k);
 }
 
-unsigned long long *graph_items(gg_graph *g) {
+gg_status graph_items(gg_graph *g) {
     const size_t total = items_cap(g, IT_SHORT) + items_cap(g, IT_LONG) + items_cap(g, IT_HUGE);
-    if (!g->items && cudaMalloc(&g->items, total * 8) != cudaSuccess) {
-        cudaGetLastError();
-        g->items = nullptr;
-    }
-    return (unsigned long long *)g->items;
+    if (!g->items) GG_CUDA(g->ctx, cudaMalloc(&g->items, total * 8));
+    return GG_OK;
 }
 
 // The whole peel of g into count[] (g->n entries, alive lists allocated).
-// *ran = false, and nothing done, where the item arrays do not fit in memory.
+// *ran = false, and nothing done, where its buffers do not fit in memory.
 gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *largest, int *steps, int *floors) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     *ran = false;
-    unsigned long long *items = graph_items(g);
-    if (!items) return GG_OK;
-    if (!g->kc_state) GG_CUDA(ctx, cudaMalloc(&g->kc_state, sizeof(KcState)));
+    auto buffers = [&]() -> gg_status {
+        GG_CHECK(graph_items(g));
+        if (!g->kc_state) GG_CUDA(ctx, cudaMalloc(&g->kc_state, sizeof(KcState)));
+        return GG_OK;
+    };
+    const gg_status fit = buffers();
+    if (fit != GG_OK) return resident_give_up(g, fit);
     KcState *st = (KcState *)g->kc_state;
     KcArgs A;
     A.off = g->off;
@@ -261,7 +262,7 @@ gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *larg
     A.count = count;
     A.alive[0] = g->kc_alive[0];
     A.alive[1] = g->kc_alive[1];
-    A.items = item_lists(g, items);
+    A.items = item_lists(g, (unsigned long long *)g->items);
     A.st = st;
     A.timeout_ns = tuning().barrier_timeout_ns;
     KcState init;

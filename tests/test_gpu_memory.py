@@ -55,7 +55,7 @@ def test_an_error_is_reported_once(ctx):
     g.close()
 
 
-@pytest.mark.parametrize("resident", [0])
+@pytest.mark.parametrize("resident", [0, 1])
 def test_buffers_that_fit_in_part(ctx, resident):
     """First calls with room for ever more of their buffers: the levels or
     GG_ERR_OOM, and the levels from the next call, whichever buffer was the
@@ -86,3 +86,25 @@ def test_buffers_that_fit_in_part(ctx, resident):
         g.close()
     finally:
         gg.tuning_set("resident", old)
+
+
+@pytest.mark.parametrize("extra", [-30, 2, 8, 40])  # no items; no bitmaps or levels of the search; all of it
+def test_cc_takes_the_other_driver_where_its_buffers_do_not_fit(ctx, extra):
+    """A CC that had run in this memory runs in it still: the search's levels
+    (17 MiB) or items (34 MiB) do not fit, label propagation does."""
+    n = 1 << 22
+    g = ctx.rmat(22, n, seed=3)
+    old = gg.tuning_get("resident")
+    try:
+        gg.tuning_set("resident", 0)
+        want = g.cc()
+        gg.tuning_set("resident", 1)
+        items = 8 * (n + g.m // 32 + g.m // 256 + 2 * (g.m // 4096) + 5)
+        with Fill(items + 3 * n // 8 + extra * MB):
+            for _ in range(2):
+                assert np.array_equal(g.cc(), want)
+        assert np.array_equal(g.cc(), want)
+        assert np.array_equal(gg.batch_bfs_cc(g, np.array([0], dtype=np.uint32))[1], want)
+    finally:
+        gg.tuning_set("resident", old)
+    g.close()

@@ -1206,14 +1206,14 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     if (!staged) g->pr_iters += p->maxiter;
     const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
                          (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && g->pr_iters >= kBlockedIters));
-    // (the values' space also serves the building of the plan)
-    const size_t vb = blocked ? pr_plan_bytes(g, dt == GG_F32 ? 4 : 2) : 0;
-    gg_status s = graph_scratch(g, 2 * nb + sb + ab + pb + vb, &base);
-    if (s != GG_OK && vb) {  // without the blocked gather, then
-        cudaGetLastError();
-        s = graph_scratch(g, 2 * nb + sb + ab + pb, &base);
-    } else if (vb) {
-        s = pr_plan(g, (char *)base + 2 * nb + sb + ab + pb, &plan);
+    gg_status s = blocked ? pr_plan(g, &plan) : GG_OK;
+    if (s == GG_OK) {
+        const size_t own = 2 * nb + sb + ab + pb;
+        s = graph_scratch(g, own + (plan ? pr_plan_bytes(plan, dt == GG_F32 ? 4 : 2) : 0), &base);
+        if (s == GG_ERR_OOM && plan) {  // without the blocked gather, then
+            plan = nullptr;
+            s = graph_scratch(g, own, &base);
+        }
     }
     if (s != GG_OK) { if (tmpx) gg_prop_destroy(tmpx); return s; }
     float *y = (float *)base;

@@ -140,9 +140,6 @@ size_t scan_bytes(uint64_t items) {
     return b;
 }
 
-// most chunks that the layout can take: each tile pads its last one
-uint64_t chunk_bound(uint64_t nblk, uint64_t nbin, uint64_t m) { return m / 8 + std::min(nblk * nbin, m); }
-
 void plan_release(PrPlan *P) {
     cudaFree(P->base);
     cudaFree(P->segs);
@@ -151,12 +148,49 @@ void plan_release(PrPlan *P) {
     P->tried = true;
 }
 
-cudaError_t plan_build(gg_graph *g, PrPlan *P, void *scratch) {
+// What the building needs beside the layout: every tile's chunks, every bin's,
+// the blocks' first chunks, and the scans' own.
+struct PlanTmp {
+    void *base = nullptr, *scan = nullptr;
+    uint32_t *tiles = nullptr, *bins = nullptr, *starts = nullptr;
+    size_t scan_b = 0;
+    ~PlanTmp() { cudaFree(base); }
+};
+
+#define PK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
+
+// Counts the chunks of every tile; at[k]: block k's first one, of P->chunks.
+cudaError_t plan_count(gg_graph *g, PrPlan *P, PlanTmp &T, std::vector<uint32_t> &at) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
-#define PK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
-    const uint64_t ntile = (uint64_t)P->nblk * P->nbin, most = chunk_bound(P->nblk, P->nbin, g->m);
-    const size_t cb = aligned(most * 16), pb = aligned(most * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
+    const uint64_t ntile = (uint64_t)P->nblk * P->nbin;
+    const size_t tb = aligned((ntile + 1) * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
+                 sb = aligned(((size_t)P->nblk + 1) * 4);
+    T.scan_b = std::max(scan_bytes(ntile + 1), scan_bytes((uint64_t)P->nbin + 1));
+    PK(cudaMalloc(&T.base, tb + bb + sb + T.scan_b));
+    T.tiles = (uint32_t *)T.base;
+    T.bins = (uint32_t *)((char *)T.base + tb);
+    T.starts = (uint32_t *)((char *)T.base + tb + bb);
+    T.scan = (char *)T.base + tb + bb + sb;
+    PK(cudaMemsetAsync(T.tiles + ntile, 0, 4, st));
+    PK(cudaMemsetAsync(T.bins + P->nbin, 0, 4, st));
+    k_plan_count<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, P->nblk, P->nbin, T.tiles, T.bins);
+    PK(cudaGetLastError());
+    PK(cub::DeviceScan::ExclusiveSum(T.scan, T.scan_b, T.tiles, T.tiles, (int64_t)ntile + 1, st));
+    k_plan_starts<<<P->nblk / 256 + 1, 256, 0, st>>>(T.tiles, P->nblk, P->nbin, T.starts);
+    PK(cudaGetLastError());
+    ctx->launches += 3;
+    at.resize((size_t)P->nblk + 1);
+    PK(cudaMemcpyAsync(at.data(), T.starts, at.size() * 4, cudaMemcpyDeviceToHost, st));
+    PK(cudaStreamSynchronize(st));
+    P->chunks = at[P->nblk];
+    return cudaSuccess;
+}
+
+cudaError_t plan_build(gg_graph *g, PrPlan *P, PlanTmp &T, const std::vector<uint32_t> &at) {
+    gg_ctx *ctx = g->ctx;
+    cudaStream_t st = ctx->stream;
+    const size_t cb = aligned(P->chunks * 16), pb = aligned(P->chunks * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
                  eb = aligned((size_t)P->nbin * kBinThreads * 4);
     PK(cudaMalloc(&P->base, 2 * cb + pb + 2 * bb + eb));
     char *p = (char *)P->base;
@@ -166,34 +200,19 @@ cudaError_t plan_build(gg_graph *g, PrPlan *P, void *scratch) {
     P->bin_ptr = (uint32_t *)(p + 2 * cb + pb);
     P->bin_end = (uint32_t *)(p + 2 * cb + pb + bb);
     P->ends = (uint32_t *)(p + 2 * cb + pb + 2 * bb);
-    // scratch: the tiles' chunks, the blocks' first chunks, the scans' own
-    uint32_t *tiles = (uint32_t *)scratch;
-    uint32_t *starts = (uint32_t *)((char *)scratch + aligned((ntile + 1) * 4));
-    void *tmp = (char *)starts + aligned(((size_t)kBlkMax + 1) * 4);
-    size_t tb = scan_bytes(ntile + 1);
-    PK(cudaMemsetAsync(P->bin_ptr, 0, 2 * bb + eb, st));
-    PK(cudaMemsetAsync(tiles + ntile, 0, 4, st));
+    PK(cudaMemsetAsync(P->bin_end, 0, bb + eb, st));
     k_plan_ends<<<ctx->sm_count * 8, 256, 0, st>>>(g->nonisolated, g->nonisolated_n, g->in_off, P->ends);
     PK(cudaGetLastError());
     k_plan_bin_ends<<<P->nbin, kBinThreads, 0, st>>>(P->ends, P->bin_end);
     PK(cudaGetLastError());
-    k_plan_count<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, P->nblk, P->nbin, tiles, P->bin_ptr);
-    PK(cudaGetLastError());
-    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, tiles, tiles, (int64_t)ntile + 1, st));
-    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, P->bin_ptr, P->bin_ptr, (int64_t)P->nbin + 1, st));
-    PK(cub::DeviceScan::ExclusiveSum(tmp, tb, P->bin_end, P->bin_end, (int64_t)P->nbin + 1, st));
-    k_plan_starts<<<P->nblk / 256 + 1, 256, 0, st>>>(tiles, P->nblk, P->nbin, starts);
-    PK(cudaGetLastError());
+    PK(cub::DeviceScan::ExclusiveSum(T.scan, T.scan_b, T.bins, P->bin_ptr, (int64_t)P->nbin + 1, st));
+    PK(cub::DeviceScan::ExclusiveSum(T.scan, T.scan_b, P->bin_end, P->bin_end, (int64_t)P->nbin + 1, st));
     const size_t smem = (size_t)((kBinEdges + 7 * P->nblk + 7) / 8 * 8) * 4;
     PK(cudaFuncSetAttribute(k_plan_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_plan_fill<<<P->nbin, kPB, smem, st>>>(g->in_adj, g->m, P->nblk, P->nbin, tiles, P->bin_ptr, P->src, P->pos,
+    k_plan_fill<<<P->nbin, kPB, smem, st>>>(g->in_adj, g->m, P->nblk, P->nbin, T.tiles, P->bin_ptr, P->src, P->pos,
                                             P->ptr);
     PK(cudaGetLastError());
-    ctx->launches += 10;
-    std::vector<uint32_t> at(P->nblk + 1);  // first chunk of each block
-    PK(cudaMemcpyAsync(at.data(), starts, at.size() * 4, cudaMemcpyDeviceToHost, st));
-    PK(cudaStreamSynchronize(st));
-    P->chunks = at[P->nblk];
+    ctx->launches += 5;
     // parts of equal work: the chunks, and for each segment the load of its
     // block's contributions (as long as some kBlkSrc / 12 chunks); eight a SM,
     // fewer where loads would then take more than an eighth of a part (as many
@@ -231,37 +250,30 @@ cudaError_t plan_build(gg_graph *g, PrPlan *P, void *scratch) {
 
 }  // namespace
 
-static PrPlan *plan_of(gg_graph *g) {
+size_t pr_plan_bytes(const PrPlan *P, size_t size) {
+    return P->chunks * 8 * size + (size_t)P->nbin * 16;  // values, parts of rows
+}
+
+gg_status pr_plan(gg_graph *g, const PrPlan **out) {
+    *out = nullptr;
     if (!g->pr_plan) {
         PrPlan *P = new PrPlan();
         P->nblk = (uint32_t)(((uint64_t)g->n + kBlkSrc - 1) >> kBlkSrcLog);
         P->nbin = (uint32_t)((g->m + kBinEdges - 1) / kBinEdges);
-        // (chunk numbers take 32 bits; the layout and the values, 9 bytes an
-        // edge and the padding, leave more than half of the memory)
-        size_t free_b = 0, all_b = 0;
-        P->tried = !g->m || P->nblk > kBlkMax || g->m >> 32 || cudaMemGetInfo(&free_b, &all_b) != cudaSuccess ||
-                   chunk_bound(P->nblk, P->nbin, g->m) * 150 > free_b;
+        P->tried = !g->m || P->nblk > kBlkMax || g->m >> 32;  // (chunk numbers take 32 bits)
         g->pr_plan = P;
     }
-    return (PrPlan *)g->pr_plan;
-}
-
-size_t pr_plan_bytes(gg_graph *g, size_t size) {
-    const PrPlan *P = plan_of(g);
-    if (P->tried && !P->ready) return 0;
-    const uint64_t ntile = (uint64_t)P->nblk * P->nbin;
-    const uint64_t chunks = P->ready ? P->chunks : chunk_bound(P->nblk, P->nbin, g->m);
-    const size_t use = chunks * 8 * size + (size_t)P->nbin * 16;  // values, parts of rows
-    if (P->ready) return use;
-    return std::max(use, aligned((ntile + 1) * 4) + aligned(((size_t)kBlkMax + 1) * 4) + scan_bytes(ntile + 1));
-}
-
-gg_status pr_plan(gg_graph *g, void *scratch, const PrPlan **out) {
-    *out = nullptr;
-    PrPlan *P = plan_of(g);
+    PrPlan *P = (PrPlan *)g->pr_plan;
     if (!P->tried) {
         P->tried = true;
-        const cudaError_t e = plan_build(g, P, scratch);
+        PlanTmp T;
+        std::vector<uint32_t> at;
+        cudaError_t e = plan_count(g, P, T, at);
+        size_t free_b = 0, all_b = 0;
+        if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &all_b);
+        // a chunk's layout and values, 36 and up to 40 bytes, leave half of the memory
+        if (e == cudaSuccess && P->chunks * 152 > free_b) e = cudaErrorMemoryAllocation;
+        if (e == cudaSuccess) e = plan_build(g, P, T, at);
         if (e != cudaSuccess) {
             plan_release(P);
             if (e != cudaErrorMemoryAllocation) return cuda_error(g->ctx, e, "PageRank edge layout");

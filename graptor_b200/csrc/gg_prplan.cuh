@@ -48,13 +48,12 @@ struct PrPlan {
     uint32_t *part_seg = nullptr;
 };
 
-// Bytes of scratch that a gather of values of `size` bytes takes, and with it
-// the building of the plan; 0 where the graph does not fit the layout's limits
-// or the layout the memory.
-size_t pr_plan_bytes(gg_graph *g, size_t size);
-// The graph's plan, built when first asked for, in scratch of pr_plan_bytes;
-// null where there is not the memory.
-gg_status pr_plan(gg_graph *g, void *scratch, const PrPlan **out);
+// The graph's plan, built when first asked for; null where the graph does not
+// fit the layout's limits, or the layout and the values not half of the free
+// memory.
+gg_status pr_plan(gg_graph *g, const PrPlan **out);
+// Bytes of scratch that a gather of values of `size` bytes takes.
+size_t pr_plan_bytes(const PrPlan *P, size_t size);
 void pr_plan_free(gg_graph *g);
 
 }  // namespace gg

@@ -126,6 +126,7 @@ gg_status gg_graph_retune(gg_graph *g) {
     cudaFree(g->nonisolated_n);
     g->nonisolated = nullptr;
     g->nonisolated_n = nullptr;
+    pr_plan_free(g);  // (built again when next asked for)
     return build_heavy_rows(g);
 }
 

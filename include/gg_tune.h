@@ -54,7 +54,9 @@ GG_API gg_status gg_tuning_set(const char *name, int64_t value);
 GG_API gg_status gg_tuning_get(const char *name, int64_t *value);
 
 /* Rebuild the graph's tuning-dependent tables (chunked heavy rows, per-word
- * cost prefixes) with the current heavy_deg / heavy_chunk. */
+ * cost prefixes) with the current heavy_deg / heavy_chunk.  Gives back the
+ * memory of the blocked PageRank gather's layout (built again when a run next
+ * takes that gather). */
 GG_API gg_status gg_graph_retune(gg_graph *g);
 
 /* Autotuner.  Coordinate descent over the knobs above on graph g: each knob

@@ -756,7 +756,7 @@ gg_status gg_ppr(gg_graph *g, const uint32_t *seeds, int k, float alpha, int ite
     return GG_OK;
 }
 
-gg_status gg_graph_union(gg_ctx *ctx, gg_graph *const *parts, int k, gg_graph **out, uint32_t *vertex_base) {
+static gg_status graph_union_once(gg_ctx *ctx, gg_graph *const *parts, int k, gg_graph **out, uint32_t *vertex_base) {
     if (!ctx || !parts || k < 1 || !out) return GG_ERR_ARG;
     uint64_t n = 0, m = 0;
     int sym = 1;
@@ -791,6 +791,11 @@ gg_status gg_graph_union(gg_ctx *ctx, gg_graph *const *parts, int k, gg_graph **
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { cudaFree(uoff); cudaFree(uadj); return cuda_error(ctx, e, "gg_graph_union"); }
     return graph_adopt_device_csr(ctx, (uint32_t)n, m, uoff, uadj, sym, sorted, out);
+}
+
+gg_status gg_graph_union(gg_ctx *ctx, gg_graph *const *parts, int k, gg_graph **out, uint32_t *vertex_base) {
+    if (!ctx) return GG_ERR_ARG;
+    return with_room(ctx, [&] { return graph_union_once(ctx, parts, k, out, vertex_base); });
 }
 
 }  // extern "C"

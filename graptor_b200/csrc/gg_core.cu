@@ -522,6 +522,10 @@ gg_status graph_ensure_first1(gg_graph *g) {
 static gg_status graph_finish(gg_graph *g) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
+    g->next_graph = ctx->graphs;
+    g->at_graph = &ctx->graphs;
+    if (ctx->graphs) ctx->graphs->at_graph = &g->next_graph;
+    ctx->graphs = g;
     if (g->symmetric) {
         g->in_off = g->off;
         g->in_adj = g->adj;
@@ -560,8 +564,29 @@ static gg_status graph_finish(gg_graph *g) {
     return build_heavy_rows(g);
 }
 
+// Memory that graphs keep between calls for their next ones (the blocked
+// gather's layout, scratch, the resident runs' buffers): given back, to be
+// allocated again when a call next needs it.  Not while a call that uses it
+// runs.  False: there was none.
+bool graphs_give_back(gg_ctx *ctx) {
+    bool any = false;
+    for (gg_graph *g = ctx->graphs; g; g = g->next_graph) {
+        any = any || g->pr_plan || g->scratch || g->items;
+        pr_plan_free(g);
+        resident_give_up(g, GG_ERR_OOM);
+        cudaFree(g->scratch);
+        g->scratch = nullptr;
+        g->scratch_bytes = 0;
+    }
+    return any;
+}
+
 static void graph_free(gg_graph *g) {
     if (!g) return;
+    if (g->at_graph) {
+        *g->at_graph = g->next_graph;
+        if (g->next_graph) g->next_graph->at_graph = g->at_graph;
+    }
     delete[] g->sel_h;
     cudaFree(g->sel_d);
     if (g->in_off && g->in_off != g->off) cudaFree(g->in_off);
@@ -910,7 +935,7 @@ gg_status gg_tuning_get(const char *name, int64_t *v) {
 // ---------------------------------------------------------------------------
 // Graphs
 // ---------------------------------------------------------------------------
-gg_status gg_graph_upload(gg_ctx *ctx, uint32_t n, uint64_t m, const uint64_t *off,
+static gg_status graph_upload_once(gg_ctx *ctx, uint32_t n, uint64_t m, const uint64_t *off,
                           const uint32_t *adj, int symmetric, gg_graph **out) {
     if (!ctx || !out || !off || (m && !adj) || n == 0xFFFFFFFFu) return set_error(ctx, GG_ERR_ARG, "gg_graph_upload: bad arguments");
     *out = nullptr;
@@ -943,6 +968,12 @@ gg_status gg_graph_upload(gg_ctx *ctx, uint32_t n, uint64_t m, const uint64_t *o
     if (s != GG_OK) { graph_free(g); return s; }
     *out = g;
     return GG_OK;
+}
+
+gg_status gg_graph_upload(gg_ctx *ctx, uint32_t n, uint64_t m, const uint64_t *off,
+                          const uint32_t *adj, int symmetric, gg_graph **out) {
+    if (!ctx) return GG_ERR_ARG;
+    return with_room(ctx, [&] { return graph_upload_once(ctx, n, m, off, adj, symmetric, out); });
 }
 
 }  // extern "C"
@@ -1023,7 +1054,7 @@ static gg_status graph_from_keys(gg_ctx *ctx, uint32_t n, uint64_t *keys, uint64
     return graph_adopt_device_csr(ctx, n, m, off, adj, sym, true, out);  // keys sorted: rows ascending
 }
 
-gg_status gg_graph_from_edges(gg_ctx *ctx, uint32_t n, uint64_t nedges, const uint32_t *src, const uint32_t *dst,
+static gg_status graph_from_edges_once(gg_ctx *ctx, uint32_t n, uint64_t nedges, const uint32_t *src, const uint32_t *dst,
                               int flags, gg_graph **out) {
     if (!ctx || !out || (nedges && (!src || !dst)) || n == 0xFFFFFFFFu || (flags & ~3)) return GG_ERR_ARG;
     *out = nullptr;
@@ -1069,7 +1100,13 @@ gg_status gg_graph_from_edges(gg_ctx *ctx, uint32_t n, uint64_t nedges, const ui
     return graph_from_keys(ctx, n, keys, nk, sym, out);
 }
 
-gg_status gg_graph_read_bin_clean(gg_ctx *ctx, const char *path, int flags, gg_graph **out) {
+gg_status gg_graph_from_edges(gg_ctx *ctx, uint32_t n, uint64_t nedges, const uint32_t *src, const uint32_t *dst,
+                              int flags, gg_graph **out) {
+    if (!ctx) return GG_ERR_ARG;
+    return with_room(ctx, [&] { return graph_from_edges_once(ctx, n, nedges, src, dst, flags, out); });
+}
+
+static gg_status graph_read_bin_clean_once(gg_ctx *ctx, const char *path, int flags, gg_graph **out) {
     if (!ctx || !path || !out || (flags & ~GG_INGEST_SYMMETRISE)) return GG_ERR_ARG;
     *out = nullptr;
     FILE *f = fopen(path, "rb");
@@ -1131,6 +1168,11 @@ gg_status gg_graph_read_bin_clean(gg_ctx *ctx, const char *path, int flags, gg_g
     return graph_from_keys(ctx, n, keys, nk, sym, out);
 }
 
+gg_status gg_graph_read_bin_clean(gg_ctx *ctx, const char *path, int flags, gg_graph **out) {
+    if (!ctx) return GG_ERR_ARG;
+    return with_room(ctx, [&] { return graph_read_bin_clean_once(ctx, path, flags, out); });
+}
+
 gg_status gg_graph_write_bin(gg_graph *g, const char *path) {
     if (!g || !path) return GG_ERR_ARG;
     std::vector<uint64_t> off((size_t)g->n + 1);
@@ -1146,7 +1188,7 @@ gg_status gg_graph_write_bin(gg_graph *g, const char *path) {
     return ok ? GG_OK : set_error(g->ctx, GG_ERR_IO, "write failed");
 }
 
-gg_status gg_graph_generate(gg_ctx *ctx, const gg_gen_params *p, gg_graph **out) {
+static gg_status graph_generate_once(gg_ctx *ctx, const gg_gen_params *p, gg_graph **out) {
     if (!ctx || !p || !out) return GG_ERR_ARG;
     *out = nullptr;
     GG_CUDA(ctx, cudaSetDevice(ctx->device));
@@ -1210,6 +1252,11 @@ gg_status gg_graph_generate(gg_ctx *ctx, const gg_gen_params *p, gg_graph **out)
     if (s != GG_OK) { graph_free(g); return s; }
     *out = g;
     return GG_OK;
+}
+
+gg_status gg_graph_generate(gg_ctx *ctx, const gg_gen_params *p, gg_graph **out) {
+    if (!ctx) return GG_ERR_ARG;
+    return with_room(ctx, [&] { return graph_generate_once(ctx, p, out); });
 }
 
 gg_status gg_graph_info(gg_graph *g, uint32_t *n, uint64_t *m, int *symmetric) {

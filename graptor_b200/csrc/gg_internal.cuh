@@ -49,6 +49,8 @@ enum : uint32_t {
 // ---------------------------------------------------------------------------
 // Handles
 // ---------------------------------------------------------------------------
+struct gg_graph;
+
 struct gg_ctx {
     int device = 0;
     int sm_count = 148;
@@ -66,6 +68,7 @@ struct gg_ctx {
     // events that mark them filled, created on first use
     void *stage = nullptr;
     cudaEvent_t stage_ev[16] = {};
+    gg_graph *graphs = nullptr;  // those alive, linked by next_graph
 };
 
 // Frontier counters live on the device in this layout.
@@ -176,6 +179,7 @@ struct gg_graph {
     void *items = nullptr;     // work items of the resident kernels (gg_items.cuh)
     void *bfs_res = nullptr;   // resident BFS: buffers
     void *cc_res = nullptr;    // resident CC: buffers
+    gg_graph *next_graph = nullptr, **at_graph = nullptr;  // in the context's list; the link that points here
     void *pr_plan = nullptr;   // blocked PageRank gather: edge layout (gg_prplan.cuh)
     uint64_t pr_iters = 0;     // PageRank iterations asked for so far
     CandLists cand;               // pull candidate lists (driver runs)
@@ -219,6 +223,15 @@ gg_status graph_scratch(gg_graph *g, size_t bytes, void **p);
 gg_status frontier_alloc_bins(gg_frontier *f);
 gg_status frontier_alloc_bitmap(gg_frontier *f);
 gg_status cand_lists_alloc(gg_graph *g);
+bool graphs_give_back(gg_ctx *ctx);
+
+// A graph made by make(), a second time with the memory that the context's
+// other graphs can do without where the first found too little.
+template <typename F> gg_status with_room(gg_ctx *ctx, F make) {
+    const gg_status s = make();
+    return s == GG_ERR_OOM && graphs_give_back(ctx) ? make() : s;
+}
+
 gg_status frontier_fetch_counts(gg_frontier *f);     // device -> host (syncs)
 gg_status frontier_ensure_bitmap(gg_frontier *f);    // from list
 gg_status frontier_ensure_list(gg_frontier *f);      // from bitmap / all

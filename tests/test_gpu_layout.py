@@ -48,3 +48,26 @@ def test_layout_takes_its_chunks_and_goes_with_a_retune(ctx, knob):
     np.testing.assert_allclose(g.pagerank(maxiter=2), want, rtol=1e-6, atol=0)
     assert abs(held - free()) <= 2 * MB
     g.close()
+
+
+def test_a_new_graph_gets_the_memory_that_others_can_do_without(ctx, knob):
+    """A graph that fits in what a layout and its values hold: they go, the
+    ranks come back the same, and the layout once there is room again."""
+    from test_gpu_memory import Fill
+    g = ctx.er(1 << 16, 256.0, seed=4, symmetric=False)  # 75 MB of layout, 84 of values
+    run = dict(maxiter=2, accum_f64=True)
+    knob(0)
+    rows = g.pagerank(**run)
+    knob(2)
+    st = gg.RunStats()
+    want = g.pagerank(stats=st, **run)
+    assert st.kernels >= BLOCKS * 2
+    n = 1 << 20  # keys 17 MB, sorted 17, rows: 60 MB at its most
+    src = np.arange(n, dtype=np.uint32)
+    with Fill(16 * MB):
+        h = ctx.from_edges(n, src, (src + 1) % n, symmetrise=False)
+        assert h.m == n
+        h.close()
+    np.testing.assert_allclose(g.pagerank(**run), want, rtol=1e-6, atol=0)
+    np.testing.assert_allclose(want, rows, rtol=1e-6, atol=0)
+    g.close()

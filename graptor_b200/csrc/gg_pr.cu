@@ -1206,7 +1206,7 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     if (!staged) g->pr_iters += p->maxiter;
     const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
                          (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && g->pr_iters >= kBlockedIters));
-    gg_status s = blocked ? pr_plan(g, &plan) : GG_OK;
+    gg_status s = blocked ? pr_plan(g, dt == GG_F32 ? 4 : 2, tuning().pr_blocked == 2, &plan) : GG_OK;
     if (s == GG_OK) {
         const size_t own = 2 * nb + sb + ab + pb;
         s = graph_scratch(g, own + (plan ? pr_plan_bytes(plan, dt == GG_F32 ? 4 : 2) : 0), &base);

@@ -19,6 +19,24 @@ constexpr uint32_t kBlkSrcLog = 15, kBlkSrc = 1u << kBlkSrcLog;
 constexpr uint32_t kBinThreads = 768, kBinEdges = 32 * kBinThreads;  // (32 edges per thread of k_pr_bins)
 constexpr uint32_t kBlkMax = 2048;  // source blocks (a bin's tiles are sorted in shared memory)
 
+// What the gather by rows takes depends on the ids: values that many edges in
+// a row share, or whose sectors they share, are found in L1.  The blocked gather
+// takes the same time whatever they are.  So it pays where 1024 consecutive edges
+// (the work of one warp) have their values in at least kSpreadLeast * 1024 sectors
+// of 32 bytes.  Time by rows over time by blocks, FP32 with double sums / BF16,
+// at that share: grid 4096^2 0.90 / 0.97 (0.10, 0.05), star 2^25 0.63 / 0.75 (0.06,
+// 0.03), sources within 1000 ids 0.79 / 0.77 (0.13, 0.06), 2000 1.00 / 0.90 (0.25,
+// 0.13), 4000 1.16 / 1.05 (0.43, 0.24), 8000 1.28 / 1.20 (0.63, 0.43), R-MAT 20 to
+// 24 and ER 1.14 to 2.9 (0.82 to 0.94).
+constexpr float kSpreadLeast = 0.24f;
+// L1 also holds the values of a graph of up to 2 source blocks whatever the
+// order of its edges (ER of 50,000 vertices and 50 M edges 0.79 / 0.61, 60,000
+// 0.98 / 0.73, 80,000 1.14 / 1.09), and those of the hubs up to 4 (R-MAT 17
+// with 41 M edges 0.92 / 0.93 at 0.62 / 0.50, R-MAT 18 1.00 / 1.08, ER of 100,000 to
+// 300,000 1.15 to 2.1 at 0.9).
+constexpr uint32_t kBlkInL1 = 2, kBlkHubsInL1 = 4;
+constexpr float kSpreadLeastHubs = 0.75f;
+
 // Place of a block's source in shared memory: its low bits mixed with the
 // others, for in an R-MAT graph the sources of most edges have the same low
 // bits and with them the same bank.
@@ -33,7 +51,8 @@ __host__ __device__ __forceinline__ uint32_t blk_slot(uint32_t v) {
 __host__ __device__ __forceinline__ uint32_t bin_slot(uint32_t p) { return p ^ ((p >> 5) & 31u); }
 
 struct PrPlan {
-    bool tried = false, ready = false;
+    bool counted = false, tried = false, ready = false;
+    float spread[2] = {0, 0};  // sectors per edge of 4- and 2-byte values
     uint32_t nblk = 0, nbin = 0, nparts = 0;
     uint64_t chunks = 0;
     void *base = nullptr;  // one allocation for the arrays below
@@ -48,10 +67,11 @@ struct PrPlan {
     uint32_t *part_seg = nullptr;
 };
 
-// The graph's plan, built when first asked for; null where the graph does not
-// fit the layout's limits, or the layout and the values not half of the free
-// memory.
-gg_status pr_plan(gg_graph *g, const PrPlan **out);
+// The graph's plan for a gather of values of `size` bytes, built when first
+// asked for; null where the graph does not fit the layout's limits, or the
+// layout and the values not half of the free memory, or (unless `always`) the
+// gather by rows is the faster one (kSpreadLeast).
+gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out);
 // Bytes of scratch that a gather of values of `size` bytes takes.
 size_t pr_plan_bytes(const PrPlan *P, size_t size);
 void pr_plan_free(gg_graph *g);

@@ -71,3 +71,39 @@ def test_a_new_graph_gets_the_memory_that_others_can_do_without(ctx, knob):
     np.testing.assert_allclose(g.pagerank(**run), want, rtol=1e-6, atol=0)
     np.testing.assert_allclose(want, rows, rtol=1e-6, atol=0)
     g.close()
+
+
+def star(ctx, n):
+    leaves = np.arange(1, n, dtype=np.uint32)
+    return ctx.from_edges(n, np.zeros_like(leaves), leaves)
+
+
+FROM = 3 << 23  # edges from which the default asks for the blocked gather
+GRAPHS = {  # what the rule looks at: shared sectors, few vertices, few edges
+    "er": (lambda ctx: ctx.er(1 << 20, 26.0, seed=3, symmetric=False), True),
+    "rmat": (lambda ctx: ctx.rmat(20, 15 << 20, seed=3), True),
+    "grid": (lambda ctx: ctx.grid(2600, 2600, seed=3), False),
+    "star": (lambda ctx: star(ctx, (FROM >> 1) + 10), False),
+    "dense": (lambda ctx: ctx.er(50000, 520.0, seed=3, symmetric=False), False),
+    "fewer": (lambda ctx: ctx.er(1 << 20, 23.0, seed=3, symmetric=False), False),
+}
+
+
+@pytest.mark.parametrize("kind", list(GRAPHS))
+@pytest.mark.parametrize("fmt,acc64", [(gg.F32, True), (gg.BF16, False)])
+def test_default_takes_the_faster_gather(ctx, knob, kind, fmt, acc64):
+    make, blocks = GRAPHS[kind]
+    g = make(ctx)
+    assert (g.m >= FROM) == (kind != "fewer")
+    k, st = 16, gg.RunStats()
+    run = dict(maxiter=k, tol=-1.0, contrib=fmt, accum_f64=acc64)
+    knob(0)
+    rows = g.pagerank(stats=st, **run)
+    by_rows = st.kernels
+    knob(1)
+    g.pagerank(**run)
+    got = g.pagerank(stats=st, **run)
+    assert st.kernels - by_rows == (k * (BLOCKS - ROWS[0 if by_rows > 2.5 * k else 1]) if blocks else 0)
+    # double sums: eight roundings an iteration; float ones of 16-bit values: those of a step of the format
+    np.testing.assert_allclose(got, rows, rtol=k * 8 * 2.0 ** -24 if acc64 else 2.0 ** -8, atol=0)
+    g.close()

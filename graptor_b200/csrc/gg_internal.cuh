@@ -181,7 +181,7 @@ struct gg_graph {
     void *cc_res = nullptr;    // resident CC: buffers
     gg_graph *next_graph = nullptr, **at_graph = nullptr;  // in the context's list; the link that points here
     void *pr_plan = nullptr;   // blocked PageRank gather: edge layout (gg_prplan.cuh)
-    uint64_t pr_iters = 0;     // PageRank iterations asked for so far
+    uint64_t pr_iters = 0;     // PageRank iterations run so far
     CandLists cand;               // pull candidate lists (driver runs)
     bool cand_active = false;     // a driver run uses them for its pull steps
     // released frontier buffers, reused in stream order

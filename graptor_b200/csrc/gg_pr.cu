@@ -637,8 +637,9 @@ constexpr int kBlock = 256;
 // 2.36 -> 2.67 ms and 2.00 -> 1.71 for the next, R-MAT 20 with 31 M edges 8.7
 // -> 8.1 and 3.31 -> 2.82, ER 63 M FP16 6.4 -> 5.6 and 5.9 -> 4.2, R-MAT 22 x 8
 // FP32 6.8 -> 6.5 and 6.4 -> 5.1).  The layout takes the time of some 3 (ER) to
-// 20 (R-MAT 24) iterations' gain to build: it is built once a graph has been
-// asked for that many iterations.
+// 20 (R-MAT 24) iterations' gain to build: it is built once a graph has run that
+// many, those counted that the coming run is sure to take (no tolerance to meet:
+// with one it may end after a few, however many it is allowed).
 constexpr uint64_t kBlockedEdges = 3ull << 23;
 constexpr uint64_t kBlockedIters = 16;
 
@@ -1203,9 +1204,9 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     const size_t ab = p->average_last > 0 ? (((size_t)g->n + 1) * 4 + 255) / 256 * 256 : 0;
     const size_t pb = ((g->heavy.nchunks + 1) * 8 + 255) / 256 * 256;
     const PrPlan *plan = nullptr;
-    if (!staged) g->pr_iters += p->maxiter;
+    const uint64_t iters = g->pr_iters + (p->tol <= 0 ? (uint64_t)p->maxiter : 0ull);
     const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
-                         (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && g->pr_iters >= kBlockedIters));
+                         (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && iters >= kBlockedIters));
     gg_status s = blocked ? pr_plan(g, dt == GG_F32 ? 4 : 2, tuning().pr_blocked == 2, &plan) : GG_OK;
     if (s == GG_OK) {
         const size_t own = 2 * nb + sb + ab + pb;
@@ -1263,6 +1264,7 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
         if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
         if (e != cudaSuccess) s = cuda_error(ctx, e, "gg_pagerank");
     }
+    if (s == GG_OK && !staged) g->pr_iters += (uint64_t)fin.iters;
     if (s == GG_OK && stats) {
         memset(stats, 0, sizeof(*stats));
         float ms = 0;

@@ -16,10 +16,11 @@
  * serves all rows), pr_blocks_per_sm (the PageRank kernels' grid cap, 16),
  * pr_blocked (1, the default: the PageRank gather of a graph of 25 M edges
  * or more whose neighbours' values lie far apart goes by blocks of sources
- * once 16 iterations have been asked of the graph, with a layout of 36 bytes
- * for every 8 edges kept with it (about 4.7 bytes an edge; more where there
- * are few edges for each 24576 edges x 32768 vertices); 2: wherever that
- * layout can be built; 0: never), persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
+ * once the graph has run 16 iterations (those counted that a run without a
+ * tolerance is sure to take), with a layout of 36 bytes for every 8 edges
+ * kept with it (about 4.7 bytes an edge; more where there are few edges for
+ * each 24576 edges x 32768 vertices); 2: wherever that layout can be built;
+ * 0: never), persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
  * one device-driven cooperative launch; otherwise one launch per iteration
 resident (1, the default (1, the default: BFS levels run as one resident
  * cooperative launch where the CUDA graph below would be taken, from many

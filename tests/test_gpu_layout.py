@@ -107,3 +107,40 @@ def test_default_takes_the_faster_gather(ctx, knob, kind, fmt, acc64):
     # double sums: eight roundings an iteration; float ones of 16-bit values: those of a step of the format
     np.testing.assert_allclose(got, rows, rtol=k * 8 * 2.0 ** -24 if acc64 else 2.0 ** -8, atol=0)
     g.close()
+
+
+def test_layout_waits_for_iterations_that_are_run(ctx, knob):
+    """A tolerance met after a few of the iterations allowed does not build the
+    layout; runs do, once they have come to 16 iterations together, and a run
+    without a tolerance that takes as many."""
+    g = ctx.er(1 << 20, 26.0, seed=3, symmetric=False)
+    st = gg.RunStats()
+
+    def kernels(k, **run):
+        g.pagerank(stats=st, host=False, **run)
+        g.pagerank_iters = st.iterations
+        return (st.kernels - 3) / k  # per iteration enqueued
+
+    knob(0)
+    assert kernels(100, maxiter=100, tol=1e-2) < BLOCKS
+    few = g.pagerank_iters
+    assert few < 8
+    knob(1)
+    gg.graph_retune(g)
+    done = few
+    while done < 16:
+        assert kernels(100, maxiter=100, tol=1e-2) < BLOCKS
+        done += few
+    assert kernels(100, maxiter=100, tol=1e-2) >= BLOCKS
+    g.close()
+
+    for parts in ((8, 7, 8), (15, 1), (16,)):
+        g = ctx.er(1 << 20, 26.0, seed=3, symmetric=False)
+        for k in parts[:-1]:
+            assert kernels(k, maxiter=k, tol=0.0) < BLOCKS, parts
+        assert kernels(parts[-1], maxiter=parts[-1], tol=0.0) >= BLOCKS, parts
+        x = g.pagerank(maxiter=10, tol=0.0)
+        knob(0)
+        np.testing.assert_allclose(x, g.pagerank(maxiter=10, tol=0.0), rtol=80 * 2.0 ** -24, atol=0)
+        knob(1)
+        g.close()

@@ -1207,6 +1207,9 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     const uint64_t iters = g->pr_iters + (p->tol <= 0 ? (uint64_t)p->maxiter : 0ull);
     const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
                          (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && iters >= kBlockedIters));
+    // (the run's time and kernels: with the layout's, where it is built)
+    const uint64_t k0 = ctx->launches;
+    cudaEventRecord(ctx->ev0, ctx->stream);
     gg_status s = blocked ? pr_plan(g, dt == GG_F32 ? 4 : 2, tuning().pr_blocked == 2, &plan) : GG_OK;
     if (s == GG_OK) {
         const size_t own = 2 * nb + sb + ab + pb;
@@ -1237,8 +1240,6 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     }
     init.sr = p->stochastic ? 1 : 0;
     init.avg_from = p->average_last > 0 ? std::max(0, p->maxiter - p->average_last) : -1;
-    uint64_t k0 = ctx->launches;
-    cudaEventRecord(ctx->ev0, ctx->stream);
     cudaError_t e = cudaMemcpyAsync(st, &init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(pr_ticket(g, partial), 0, 8, ctx->stream);
     if (e == cudaSuccess && acc) e = cudaMemsetAsync(acc, 0, (size_t)g->n * 4, ctx->stream);

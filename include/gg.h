@@ -458,7 +458,11 @@ typedef struct gg_pr_params {
     int stochastic;
     int average_last;
 } gg_pr_params;
-/* PageRank power iteration (PRv / PR_vary run_prec); x receives the ranks. */
+/* PageRank power iteration (PRv / PR_vary run_prec); x receives the ranks.
+ * A large graph that has run 16 iterations takes another gather from then on
+ * (knob pr_blocked, gg_tune.h), which adds a row's terms in another order: the
+ * last bits of float sums can differ from an earlier call's.  st->total_ms and
+ * st->kernels of the call that builds that gather's layout include it. */
 GG_API gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x, float *host_x,
                              gg_run_stats *st);
 

@@ -144,3 +144,15 @@ def test_layout_waits_for_iterations_that_are_run(ctx, knob):
         np.testing.assert_allclose(x, g.pagerank(maxiter=10, tol=0.0), rtol=80 * 2.0 ** -24, atol=0)
         knob(1)
         g.close()
+
+
+def test_run_that_builds_the_layout_reports_it(ctx, knob):
+    g = ctx.er(1 << 20, 26.0, seed=3, symmetric=False)
+    knob(2)
+    first, next_ = gg.RunStats(), gg.RunStats()
+    g.pagerank(maxiter=2, host=False, stats=first)
+    g.pagerank(maxiter=2, host=False, stats=next_)
+    assert next_.kernels == 3 + 2 * BLOCKS
+    assert first.kernels >= next_.kernels + 5  # counts, scans, row ends, the sorting pass
+    assert first.total_ms > next_.total_ms
+    g.close()

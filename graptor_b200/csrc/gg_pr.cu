@@ -917,21 +917,58 @@ k_pr_bins(PrPlan P, const typename Store<DT>::T *__restrict__ vals, const uint32
     }
 }
 
-// Totals of the rows that end in a later bin than they begin in: a thread
-// per bin, its first row's parts in the order of the bins.
+// Totals of the rows that end in a later bin than they begin in: a lane per
+// bin in which such a row ends, rows over more than kSpanLane bins by the warp,
+// 128 bins at a time from their last one back to the one they begin in (a star
+// of 2^25 vertices, a row over 1365 bins, all of it by one lane: 1.03 ms an
+// iteration with FP32 and 0.88 with BF16 -> 0.81 and 0.73).
+constexpr uint32_t kSpanLane = 4;
+
 template <int DT, bool ACC64>
 __global__ void __launch_bounds__(256)
 k_pr_spans(PrPlan P, const uint32_t *__restrict__ list, float *y_f32, PrState *st,
            const typename std::conditional<ACC64, double, float>::type *parts) {
     using Acc = typename std::conditional<ACC64, double, float>::type;
     if (pr_idle(st, -1)) return;
-    const uint32_t b = blockIdx.x * 256 + threadIdx.x;
-    double ysum = 0;
-    if (b && b < P.nbin && P.bin_end[b + 1] > P.bin_end[b] && !(P.ends[(uint64_t)b * kBinThreads - 1] >> 31)) {
+    const uint32_t b = blockIdx.x * 256 + threadIdx.x, lane = threadIdx.x & 31u;
+    const bool need =
+        b && b < P.nbin && P.bin_end[b + 1] > P.bin_end[b] && !(P.ends[(uint64_t)b * kBinThreads - 1] >> 31);
+    const auto begins = [&](uint32_t x) { return x == 0 || P.bin_end[x + 1] != P.bin_end[x]; };
+    Acc acc = 0;
+    bool wide = false;
+    if (need) {
         uint32_t x = b - 1;
-        while (x && P.bin_end[x + 1] == P.bin_end[x]) --x;
-        Acc acc = 0;
-        for (; x < b; ++x) acc += parts[2 * (uint64_t)x + 1];
+        while (b - x < kSpanLane && !begins(x)) --x;
+        wide = !begins(x);
+        if (!wide)
+            for (; x < b; ++x) acc += parts[2 * (uint64_t)x + 1];
+    }
+    for (unsigned pend = __ballot_sync(FULL, wide); pend; pend &= pend - 1) {
+        const int j = __ffs(pend) - 1;
+        Acc part = 0;
+        bool on = true;
+        for (int64_t at = (int64_t)__shfl_sync(FULL, b, j) - 1; on; at -= 128) {
+            Acc v[4];
+            bool first[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int64_t x = at - 32 * u - lane;
+                first[u] = x < 0 || begins((uint32_t)x);
+                v[u] = x < 0 ? Acc(0) : parts[2 * x + 1];
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const unsigned f = __ballot_sync(FULL, first[u]);
+                // up to the bin that the row begins in, and none of the next 32 after it
+                if (on && (!f || (int)lane < __ffs(f))) part += v[u];
+                on = on && !f;
+            }
+        }
+        part = dev::warp_sum(part);
+        if ((int)lane == j) acc = part;
+    }
+    double ysum = 0;
+    if (need) {
         acc += parts[2 * (uint64_t)b];
         ysum = pr_store_row<DT, false>(y_f32, nullptr, list[P.bin_end[b]], acc, st->scale_inv);
     }

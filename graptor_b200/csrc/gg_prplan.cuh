@@ -24,7 +24,7 @@ constexpr uint32_t kBlkMax = 2048;  // source blocks (a bin's tiles are sorted i
 // takes the same time whatever they are.  So it pays where 1024 consecutive edges
 // (the work of one warp) have their values in at least kSpreadLeast * 1024 sectors
 // of 32 bytes.  Time by rows over time by blocks, FP32 with double sums / BF16,
-// at that share: grid 4096^2 0.90 / 0.97 (0.10, 0.05), star 2^25 0.63 / 0.75 (0.06,
+// at that share: grid 4096^2 0.90 / 0.97 (0.10, 0.05), star 2^25 0.81 / 0.93 (0.06,
 // 0.03), sources within 1000 ids 0.79 / 0.77 (0.13, 0.06), 2000 1.00 / 0.90 (0.25,
 // 0.13), 4000 1.16 / 1.05 (0.43, 0.24), 8000 1.28 / 1.20 (0.63, 0.43), R-MAT 20 to
 // 24 and ER 1.14 to 2.9 (0.82 to 0.94).

@@ -69,3 +69,35 @@ def test_blocked_equals_row_gather(ctx, knob, kind, fmt, acc64):
     rel = {gg.F32: 5 * 400 * eps, gg.BF16: 2.0 ** -8, gg.F16: 2.0 ** -10}[fmt]
     np.testing.assert_allclose(g.pagerank(maxiter=5, **run), again, rtol=rel, atol=0)
     g.close()
+
+
+@pytest.mark.parametrize("fmt,acc64", [(gg.F32, True), (gg.F32, False), (gg.BF16, False)])
+def test_rows_over_many_bins(ctx, knob, fmt, acc64):
+    """Rows over 2 to 6 bins (summed by a lane up to 4) and over 33, 34, 129,
+    130 and 300 (by a warp, 128 bins at a time), the first one from bin 0, with
+    short rows before, between and after them."""
+    rng = np.random.default_rng(11)
+    n = 1 << 23
+    bins = [300, 2, 3, 4, 5, 6, 33, 34, 129, 130]
+    deg = np.zeros(n, dtype=np.int64)
+    at = 0
+    for k in bins:  # k - 1 whole bins and some edges before and after them
+        deg[at] = (k - 1) * 24576 + 7
+        deg[at + 1: at + 40] = rng.integers(1, 5, 39)
+        at += 60
+    dst = np.repeat(np.arange(n, dtype=np.int64), deg)
+    first = np.repeat(np.cumsum(deg) - deg, deg)
+    src = (dst + 1 + (np.arange(len(dst)) - first)) % n  # distinct within a row
+    g = ctx.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32), symmetrise=False)
+    assert g.m == len(dst)
+    run = dict(contrib=fmt, accum_f64=acc64, tol=0.0, maxiter=1)
+    gg.tuning_set(KNOB, 0)
+    want = g.pagerank(**run).astype(np.float64)
+    gg.tuning_set(KNOB, 2)
+    got = g.pagerank(**run)
+    # the same terms in another order: double sums round once, float sums take
+    # at most 32 + 5 + 24 + 4 + 300 / 32 + 5 + 1 additions one after the other by
+    # blocks, and 1024 / 32 + 5 + 7200 / 32 + 5 by rows
+    eps = 2.0 ** -24
+    assert np.all(np.abs(got - want) <= want * eps * (8 if acc64 else 400))
+    g.close()

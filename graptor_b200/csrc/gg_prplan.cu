@@ -6,6 +6,7 @@
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <new>
 #include <vector>
 
 #include "gg_prplan.cuh"
@@ -276,8 +277,7 @@ size_t pr_plan_bytes(const PrPlan *P, size_t size) {
     return P->chunks * 8 * size + (size_t)P->nbin * 16;  // values, parts of rows
 }
 
-gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out) {
-    *out = nullptr;
+static gg_status plan_of(gg_graph *g, size_t size, bool always, const PrPlan **out) {
     if (!g->pr_plan) {
         PrPlan *P = new PrPlan();
         P->nblk = (uint32_t)(((uint64_t)g->n + kBlkSrc - 1) >> kBlkSrcLog);
@@ -311,6 +311,16 @@ gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out) {
     }
     if (P->ready && pays()) *out = P;
     return GG_OK;
+}
+
+gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out) {
+    *out = nullptr;
+    try {
+        return plan_of(g, size, always, out);
+    } catch (const std::bad_alloc &) {  // of the host: no layout either
+        if (g->pr_plan) plan_release((PrPlan *)g->pr_plan);
+        return GG_OK;
+    }
 }
 
 void pr_plan_free(gg_graph *g) {

@@ -31,6 +31,20 @@ void host_stage_free(gg_ctx *ctx) {
     ctx->stage = nullptr;
 }
 
+// The context's device as the calling thread's current one, whose own comes
+// back at the end: the slots' events belong to it, and a download leaves the
+// caller's device as it is.
+struct CurrentDevice {
+    int before = -1;
+    explicit CurrentDevice(int device) {
+        if (cudaGetDevice(&before) != cudaSuccess || before == device) before = -1;
+        else cudaSetDevice(device);
+    }
+    ~CurrentDevice() {
+        if (before >= 0) cudaSetDevice(before);
+    }
+};
+
 static bool host_stage(gg_ctx *ctx) {
     if (ctx->stage) return true;
     bool ok = cudaHostAlloc(&ctx->stage, 2 * kMaxCopiers * kPiece, cudaHostAllocDefault) == cudaSuccess;
@@ -51,6 +65,7 @@ static gg_status direct(gg_ctx *ctx, void *dst, const void *src, size_t bytes) {
 // bytes of device memory to host memory, after the work on the context's
 // stream; returns when they are there.
 gg_status host_download(gg_ctx *ctx, void *dst, const void *src, size_t bytes) {
+    const CurrentDevice device(ctx->device);
     if (bytes == 0) return direct(ctx, dst, src, 0);
     cudaPointerAttributes at;
     const bool known = cudaPointerGetAttributes(&at, dst) == cudaSuccess;

@@ -32,3 +32,21 @@ def test_msbfs_rows_packed(ctx, k):
     for i in (0, k - 1):
         assert np.array_equal(lv[:, i], g.bfs_level(int(roots[i])))
     g.close()
+
+
+def test_download_leaves_the_current_device(ctx):
+    """From a context on another device than the thread's current one."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.device_count() < 2:
+        pytest.skip("two devices")
+    c = gg.Context(1)
+    n = 6 << 20
+    g = c.from_edges(n, np.zeros(0, np.uint32), np.zeros(0, np.uint32))
+    p = g.prop(gg.U8)
+    a = np.random.default_rng(n).integers(0, 256, n, dtype=np.uint8)
+    p.upload(a)
+    torch.cuda.set_device(0)
+    for _ in range(2):
+        assert np.array_equal(p.download(), a)
+        assert torch.cuda.current_device() == 0
+    c.close()

@@ -632,17 +632,6 @@ __global__ void k_pr_init(XT<DT> *x, typename Store<DT>::T *contrib, const uint6
 
 constexpr int kBlock = 256;
 
-// The gather by blocks pays from some 25 M edges on (20 iterations, by rows
-// -> by blocks, the first call of a graph with the layout's building: ER 16 M
-// 2.36 -> 2.67 ms and 2.00 -> 1.71 for the next, R-MAT 20 with 31 M edges 8.7
-// -> 8.1 and 3.31 -> 2.82, ER 63 M FP16 6.4 -> 5.6 and 5.9 -> 4.2, R-MAT 22 x 8
-// FP32 6.8 -> 6.5 and 6.4 -> 5.1).  The layout takes the time of some 3 (ER) to
-// 20 (R-MAT 24) iterations' gain to build: it is built once a graph has run that
-// many, those counted that the coming run is sure to take (no tolerance to meet:
-// with one it may end after a few, however many it is allowed).
-constexpr uint64_t kBlockedEdges = 3ull << 23;
-constexpr uint64_t kBlockedIters = 16;
-
 static unsigned pr_grid(gg_ctx *ctx, uint64_t work) {
     uint64_t b = (work + kBlock - 1) / kBlock;
     uint64_t cap = (uint64_t)ctx->sm_count * tuning().pr_blocks_per_sm;

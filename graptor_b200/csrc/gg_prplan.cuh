@@ -19,6 +19,17 @@ constexpr uint32_t kBlkSrcLog = 15, kBlkSrc = 1u << kBlkSrcLog;
 constexpr uint32_t kBinThreads = 768, kBinEdges = 32 * kBinThreads;  // (32 edges per thread of k_pr_bins)
 constexpr uint32_t kBlkMax = 2048;  // source blocks (a bin's tiles are sorted in shared memory)
 
+// The gather by blocks pays from some 25 M edges on (20 iterations, by rows
+// -> by blocks, the first call of a graph with the layout's building: ER 16 M
+// 2.36 -> 2.67 ms and 2.00 -> 1.71 for the next, R-MAT 20 with 31 M edges 8.7
+// -> 8.1 and 3.31 -> 2.82, ER 63 M FP16 6.4 -> 5.6 and 5.9 -> 4.2, R-MAT 22 x 8
+// FP32 6.8 -> 6.5 and 6.4 -> 5.1).  The layout takes the time of some 3 (ER) to
+// 20 (R-MAT 24) iterations' gain to build: it is built once a graph has run that
+// many, those counted that the coming run is sure to take (no tolerance to meet:
+// with one it may end after a few, however many it is allowed).
+constexpr uint64_t kBlockedEdges = 3ull << 23;
+constexpr uint64_t kBlockedIters = 16;
+
 // What the gather by rows takes depends on the ids: values that many edges in
 // a row share, or whose sectors they share, are found in L1.  The blocked gather
 // takes the same time whatever they are.  So it pays where 1024 consecutive edges

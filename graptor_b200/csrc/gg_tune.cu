@@ -6,7 +6,7 @@
 #include <string>
 #include <vector>
 
-#include "gg_internal.cuh"
+#include "gg_prplan.cuh"
 
 namespace gg {
 
@@ -37,6 +37,23 @@ std::vector<Knob> knob_space(int analytics) {
     return k;
 }
 
+// Whether a run that the objective times reads the knob, with the others as
+// they are now: a knob that none reads would be set by the noise of the clock.
+bool read_by_runs(const gg_graph *g, int analytics, const std::string &knob) {
+    const Tuning &t = tuning();
+    const bool bfs = analytics & GG_TUNE_BFS, cc = analytics & GG_TUNE_CC, pr = analytics & GG_TUNE_PR;
+    const bool graph_bfs = bfs && (t.graph & 1) && !(t.persistent & 1);  // or its resident form
+    const bool bfs_res = graph_bfs && t.resident;
+    const bool cc_res = cc && g->symmetric && t.resident && (t.persistent & 4) && t.cc_hook == 1 && !(t.fusion & 4);
+    const bool other = (bfs && !bfs_res) || (cc && !cc_res);  // by lists of vertices, host- or device-driven
+    if (knob == "pull_k") return bfs || cc;                   // (the resident CC searches by BFS)
+    if (knob == "heavy_deg" || knob == "heavy_chunk") return cc || pr;
+    if (knob == "persistent") return bfs || cc;
+    if (knob == "pull_split") return graph_bfs && !bfs_res;
+    if (knob == "pr_blocks_per_sm") return pr;
+    return other;
+}
+
 struct Objective {
     gg_graph *g;
     int analytics;
@@ -46,6 +63,17 @@ struct Objective {
     std::vector<uint32_t> cc0, cc;
     bool have_ref = false;
     int evals = 0;
+
+    gg_status pagerank(int iters, gg_run_stats *st) {
+        gg_pr_params p;
+        std::memset(&p, 0, sizeof(p));
+        p.maxiter = iters;
+        p.tol = 0;
+        p.damping = 0.85f;
+        p.contrib_dtype = GG_F32;
+        p.accum_f64 = 0;
+        return gg_pagerank(g, &p, nullptr, nullptr, st);
+    }
 
     // sum over analytics of the fastest of `reps` runs; false on a result mismatch
     gg_status eval(double *ms_out) {
@@ -72,16 +100,9 @@ struct Objective {
             total += best;
         }
         if (analytics & GG_TUNE_PR) {
-            gg_pr_params p;
-            std::memset(&p, 0, sizeof(p));
-            p.maxiter = 5;
-            p.tol = 0;
-            p.damping = 0.85f;
-            p.contrib_dtype = GG_F32;
-            p.accum_f64 = 0;
             double best = 1e30;
             for (int r = 0; r < reps; ++r) {
-                GG_CHECK(gg_pagerank(g, &p, nullptr, nullptr, &st));
+                GG_CHECK(pagerank(5, &st));
                 best = std::min(best, st.total_ms);
             }
             total += best;
@@ -126,7 +147,7 @@ gg_status gg_graph_retune(gg_graph *g) {
     cudaFree(g->nonisolated_n);
     g->nonisolated = nullptr;
     g->nonisolated_n = nullptr;
-    pr_plan_free(g);  // (built again when next asked for)
+    if (!tuning().pr_blocked) pr_plan_free(g);
     return build_heavy_rows(g);
 }
 
@@ -145,10 +166,14 @@ gg_status gg_autotune(gg_graph *g, int analytics, const uint32_t *roots, int nro
     obj.lv.assign((analytics & GG_TUNE_BFS) ? g->n : 0, 0);
     obj.cc.assign((analytics & GG_TUNE_CC) ? g->n : 0, 0);
     std::vector<Knob> space = knob_space(analytics);
+    std::vector<bool> swept(space.size(), false);
     std::vector<int64_t> cur(space.size());
     for (size_t i = 0; i < space.size(); ++i) GG_CHECK(gg_tuning_get(space[i].name, &cur[i]));
-    // a warm-up evaluation (first-use allocations), then the reference one
+    // a warm-up evaluation (first-use allocations, and iterations enough for
+    // PageRank to have changed over to the gather it stays with), then the
+    // reference one
     double best;
+    if (analytics & GG_TUNE_PR) GG_CHECK(obj.pagerank((int)kBlockedIters, nullptr));
     GG_CHECK(obj.eval(&best));
     GG_CHECK(obj.eval(&best));
     out->initial_ms = best;
@@ -156,6 +181,8 @@ gg_status gg_autotune(gg_graph *g, int analytics, const uint32_t *roots, int nro
         bool changed = false;
         for (size_t i = 0; i < space.size(); ++i) {
             const Knob &k = space[i];
+            if (!read_by_runs(g, analytics, k.name)) continue;
+            swept[i] = true;
             int64_t keep = cur[i];
             for (int64_t v : k.values) {
                 if (v == cur[i]) continue;
@@ -188,8 +215,9 @@ gg_status gg_autotune(gg_graph *g, int analytics, const uint32_t *roots, int nro
     out->evaluations = obj.evals;
     std::string s;
     for (size_t i = 0; i < space.size(); ++i) {
+        if (!swept[i]) continue;
         char buf[64];
-        std::snprintf(buf, sizeof(buf), "%s%s=%lld", i ? "," : "", space[i].name, (long long)cur[i]);
+        std::snprintf(buf, sizeof(buf), "%s%s=%lld", s.empty() ? "" : ",", space[i].name, (long long)cur[i]);
         s += buf;
     }
     std::snprintf(out->best, sizeof(out->best), "%s", s.c_str());

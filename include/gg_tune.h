@@ -57,16 +57,16 @@ GG_API gg_status gg_tuning_set(const char *name, int64_t value);
 GG_API gg_status gg_tuning_get(const char *name, int64_t *value);
 
 /* Rebuild the graph's tuning-dependent tables (chunked heavy rows, per-word
- * cost prefixes) with the current heavy_deg / heavy_chunk.  Gives back the
- * memory of the blocked PageRank gather's layout (built again when a run next
- * takes that gather). */
+ * cost prefixes) with the current heavy_deg / heavy_chunk.  With pr_blocked
+ * 0, also give back the memory of the blocked PageRank gather's layout. */
 GG_API gg_status gg_graph_retune(gg_graph *g);
 
 /* Autotuner.  Coordinate descent over the knobs above on graph g: each knob
  * in turn takes each of its candidate values while the others stay at their
  * best so far; a candidate is kept when the objective (the sum of the
  * analytics' device times, each the minimum of `reps` runs) drops by more
- * than 1%.  `passes` sweeps over all knobs.  Every candidate's BFS levels
+ * than 1%.  A knob that none of the timed runs reads, with the others as they
+ * are, is left alone.  `passes` sweeps over all knobs.  Every candidate's BFS levels
  * and CC labels are compared with the first run's and must be identical
  * (GG_ERR_STATE otherwise).  On return the best values are set. */
 enum { GG_TUNE_BFS = 1, GG_TUNE_CC = 2, GG_TUNE_PR = 4 };
@@ -74,7 +74,7 @@ typedef struct gg_tune_result {
     double initial_ms;   /* objective with the values on entry */
     double best_ms;      /* objective with the chosen values */
     int evaluations;     /* objective evaluations */
-    char best[512];      /* "name=value,..." of every knob tuned */
+    char best[512];      /* "name=value,..." of every knob swept */
 } gg_tune_result;
 GG_API gg_status gg_autotune(gg_graph *g, int analytics, const uint32_t *roots, int nroots, int passes, int reps,
                              gg_tune_result *out);

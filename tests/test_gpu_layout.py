@@ -39,8 +39,10 @@ def test_layout_takes_its_chunks_and_goes_with_a_retune(ctx, knob):
     knob(2)
     want = g.pagerank(maxiter=2)
     held = free()
+    knob(0)
     gg.graph_retune(g)
     layout = free() - held
+    knob(2)
     bins = -(-g.m // 24576)
     chunks = g.m // 8 + bins
     bound = 36 * chunks + bins * (768 * 4 + 8)
@@ -126,7 +128,6 @@ def test_layout_waits_for_iterations_that_are_run(ctx, knob):
     few = g.pagerank_iters
     assert few < 8
     knob(1)
-    gg.graph_retune(g)
     done = few
     while done < 16:
         assert kernels(100, maxiter=100, tol=1e-2) < BLOCKS

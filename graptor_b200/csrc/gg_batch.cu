@@ -577,8 +577,7 @@ static void ppr_run(gg_ctx *ctx, PprArgs A, uint2 *c0, uint2 *c1, uint2 *x, uint
     const uint64_t cap = (uint64_t)ctx->sm_count * resident_ctas((const void *)step, kPprBlock);
     // fewer rows per ticket where warps would go without any (always the most ->
     // so: ER 1204 x 45, 99 seeds, 14 iterations 0.355 -> 0.122 ms, R-MAT 10, 128
-    // seeds, 20 iterations 0.67 -> 0.38) (ER 1204 x 45, 99
-    // seeds, 14 iterations: @@)
+    // seeds, 20 iterations 0.67 -> 0.38)
     A.rows = G * (uint32_t)std::max<uint64_t>(
                      1, std::min<uint64_t>(kPprRows<L> / G, A.n / (G * cap * (kPprBlock / 32))));
     A.tickets = (uint32_t)((A.H.nchunks + G - 1) / G + ((uint64_t)A.n + A.rows - 1) / A.rows);

@@ -10,22 +10,24 @@
  * Names: bin_small_max, bin_medium_max (sparse-push degree bins),
  * pull_k, push_k (edges a lane scans alone before its warp helps),
  * heavy_deg, heavy_chunk (CSC rows chunked for gathers; apply to graphs
- * created afterwards or after gg_graph_retune), large_chunk (push: edges
+ * created afterwards or after gg_graph_retune; a heavy_deg above 2^26 acts as
+ * 2^26), large_chunk (push: edges
  * per chunk of a hub row), blocks_per_sm (CTAs per SM of the grid-stride
  * kernels), pr_stream (0 or 1, without effect: one PageRank gather
  * serves all rows), pr_blocks_per_sm (the PageRank kernels' grid cap, 16),
- * pr_blocked (1, the default: the PageRank gather of a graph of 25 M edges
- * or more whose neighbours' values lie far apart goes by blocks of sources
- * once the graph has run 16 iterations (those counted that a run without a
- * tolerance is sure to take), with a layout of 36 bytes for every 8 edges
- * kept with it (about 4.7 bytes an edge; more where there are few edges for
- * each 24576 edges x 32768 vertices); 2: wherever that layout can be built;
- * 0: never), persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
+ * pr_blocked (1, the default: the PageRank gather of a graph of 25 M edges or
+ * more, and more than 65536 vertices, whose neighbours' values lie far apart
+ * goes by blocks of sources once the graph has run 16 iterations (those
+ * counted that a run without a tolerance is sure to take), with a layout of 36
+ * bytes for every 8 edges kept with it (about 4.7 bytes an edge; more where
+ * there are few edges for each 24576 edges x 32768 vertices); 2: wherever that
+ * layout can be built; 0: never),
+ * persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
  * one device-driven cooperative launch; otherwise one launch per iteration
-resident (1, the default (1, the default: BFS levels run as one resident
+ * from the host), resident (1, the default: BFS levels run as one resident
  * cooperative launch where the CUDA graph below would be taken, from many
- * roots too, and CC of symmetric graphs as two; 0: not), graph (1, the default: BFS levels run as one CUDA graph
- * whose conditional nodes take each step's push/pull decision on the
+ * roots too, and CC of symmetric graphs as two; 0: not),
+ * graph (1, the default: BFS levels run as one CUDA graph whose conditional nodes take each step's push/pull decision on the
  * device; 0: one host round trip per iteration), graph_handoff (32, the
  * default: a graph-driven BFS still running after that many iterations
  * continues as one device-driven cooperative launch from its current

@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 
 from graptor_b200 import gg
+from oracle import oracle as O
 
 pytestmark = pytest.mark.gpu
 
@@ -100,4 +101,43 @@ def test_rows_over_many_bins(ctx, knob, fmt, acc64):
     # blocks, and 1024 / 32 + 5 + 7200 / 32 + 5 by rows
     eps = 2.0 ** -24
     assert np.all(np.abs(got - want) <= want * eps * (8 if acc64 else 400))
+    g.close()
+
+
+@pytest.mark.parametrize("kind", ["short", "lengths", "full", "small"])
+def test_knob_decides_which_gather_runs(ctx, knob, kind):
+    """Told apart by their kernels: four per iteration by blocks, two or three
+    (heavy rows) by rows."""
+    n, src, dst = edges(kind, np.random.default_rng(len(kind)))
+    g = ctx.from_edges(n, src, dst, symmetrise=False)
+    st = gg.RunStats()
+    for fmt, acc64 in ((gg.F32, True), (gg.F32, False), (gg.BF16, False), (gg.F16, False), (gg.CFP_6_10, False),
+                       (gg.BF16_TRUNC, False)):
+        for value, kernels in ((2, {4}), (0, {2, 3})):
+            gg.tuning_set(KNOB, value)
+            for _ in range(2):  # (the first also builds the layout)
+                g.pagerank(maxiter=3, tol=0.0, contrib=fmt, accum_f64=acc64, host=False, stats=st)
+            assert st.kernels - 3 in {3 * k for k in kernels}, (fmt, value)
+    for fmt, acc64 in ((gg.F64, True), (gg.FP8E4M3, False)):  # never by blocks
+        gg.tuning_set(KNOB, 2)
+        g.pagerank(maxiter=3, tol=0.0, contrib=fmt, accum_f64=acc64, host=False, stats=st)
+        assert st.kernels - 3 in (6, 9)
+    g.close()
+
+
+@pytest.mark.parametrize("blocked", [0, 2])
+def test_both_gathers_give_the_references_ranks(ctx, knob, blocked):
+    """PRv's answer by rows and by blocks, and PR_vary's with customfp<6,10>
+    storage, as the row gather's tests have it."""
+    og = O.rmat(15, 16 << 15, seed=9)
+    g = ctx.upload(og.off, og.adj)
+    gg.tuning_set(KNOB, blocked)
+    st = gg.RunStats()
+    xo, _, _ = O.pagerank(og, maxiter=20, tol=0)
+    x = g.pagerank(maxiter=20, tol=0, stats=st)
+    assert (st.kernels >= 3 + 20 * 4) == (blocked == 2)
+    assert np.abs(x.astype(np.float64) - xo).sum() <= 1e-6
+    xo, _, _ = O.pagerank_vary(og, O.CFP_6_10, accum_f64=False, maxiter=20, tol=0)
+    x = g.pagerank(maxiter=20, tol=0, contrib=gg.CFP_6_10, accum_f64=False, renorm_f32=False)
+    assert np.abs(x.astype(np.float64) - xo).sum() <= 1e-5
     g.close()

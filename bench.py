@@ -218,14 +218,13 @@ def pick_roots(deg: np.ndarray) -> np.ndarray:
     return rng.choice(nz, size=NROOTS, replace=False).astype(np.uint32)
 
 
-# DRAM bytes (read + write) per dense-pull launch, from one ncu capture of
-# k_pull with the three-neighbour records (4 launches of R-MAT scale 23 BFS,
-# 245.0 MB each on average) scaled by the vertex count to scale 24
-K_PULL_TRAFFIC_PER_LAUNCH = 490.0e6
-# DRAM bytes of one 128-seed PPR iteration at R-MAT 22 (m = 128,311,324):
-# ncu's 3.03 GB read + 2.08 GB written by k_ppr_light, less the 1.07 GB of
-# rank rows that only the last iteration writes now
-PPR_DRAM_BYTES_PER_ITER = 4.04e9
+# DRAM bytes (read + write) of one resident BFS (k_bfs_run) from ncu captures
+# at R-MAT scale 23 (two roots, 734 and 374 MB), their mean scaled by the
+# vertex count to scale 24
+K_BFS_TRAFFIC_PER_RUN = 1.108e9
+# DRAM bytes of one 128-seed PPR iteration (k_ppr_wide) at R-MAT 22
+# (m = 128,311,324) from ncu: 8.58 GB read, 1.20 GB written
+PPR_DRAM_BYTES_PER_ITER = 9.78e9
 
 
 def bfs_bytes(n: int, st, it: int) -> float:
@@ -244,7 +243,8 @@ def cc_bytes(n: int, m: int, st, it: int) -> float:
     """Algorithmic bytes of CC iteration `it`: a dense pull reads offsets,
     labels, the scanned in-edges and their sources' labels (8(n+1) + 4n + 8S
     + 4N + 2n/8); a sparse push 4F + 16F + 4E + 4E + 4N; the hooking step
-    (road-like graphs) one pass over the CSR and the labels (8(n+1) + 4m + 8n)."""
+    (road-like graphs) offsets, labels and the scanned edges' ids (8(n+1) + 4S + 8n).
+    The default run's two records, the search and the hooks, count as pulls."""
     from graptor_b200 import gg
     F, E, S = st.nactv[it], st.nacte[it], st.scanned[it]
     N = st.nactv[it + 1] if it + 1 < st.iterations else 0
@@ -252,7 +252,7 @@ def cc_bytes(n: int, m: int, st, it: int) -> float:
     if v == gg.VAR_PULL_DENSE:
         return 8.0 * (n + 1) + 4.0 * n + 8.0 * S + 4.0 * N + 2.0 * n / 8
     if v == gg.VAR_HOOK:
-        return 8.0 * (n + 1) + 4.0 * m + 8.0 * n
+        return 8.0 * (n + 1) + 4.0 * S + 8.0 * n
     return 20.0 * F + 8.0 * E + 4.0 * N
 
 
@@ -439,8 +439,9 @@ def selector_eval(ctx, graphs):
     from graptor_b200 import gg
     from graptor_b200.selector_train import load_selector
     sel = load_selector(ctx)
-    old = gg.tuning_get("persistent")
+    old = {k: gg.tuning_get(k) for k in ("persistent", "resident")}
     gg.tuning_set("persistent", 7)
+    gg.tuning_set("resident", 0)  # (the resident CC makes no choice: not for one policy only)
     out = {"weights": "graptor_b200/data/selector.npz" if sel else None,
            "oracle": "per root, the smaller of: the threshold run with one iteration forced to each variant "
                      "in turn on the same state (BFS sums the per-iteration gains, CC takes the best single "
@@ -505,9 +506,10 @@ def selector_eval(ctx, graphs):
             if sel:
                 gg.attach_selector(g, None)
     finally:
-        gg.tuning_set("persistent", old)
-    # the default BFS driver (one CUDA graph per run, device decisions): the
-    # network picks between its push and pull
+        for k, v in old.items():
+            gg.tuning_set(k, v)
+    # the default BFS driver (one resident launch per run): the network picks
+    # between its push and pull
     if sel:
         for name, g, roots in graphs:
             gg.attach_selector(g, sel)
@@ -521,8 +523,8 @@ def selector_eval(ctx, graphs):
                     g.bfs_level(r, host=False, opts=opts, stats=st)
                     t += st.total_ms
                 tot[mode] = t / len(roots)
-            out[name]["bfs_graph_driver"] = {k: round(v, 4) for k, v in tot.items()}
-            out[name]["bfs_graph_driver"]["learned_vs_threshold"] = round(tot["threshold"] / tot["learned"], 3)
+            out[name]["bfs_default_driver"] = {k: round(v, 4) for k, v in tot.items()}
+            out[name]["bfs_default_driver"]["learned_vs_threshold"] = round(tot["threshold"] / tot["learned"], 3)
             gg.attach_selector(g, None)
     return out
 
@@ -685,17 +687,14 @@ def batch_eval(ctx, g, roots, hbm_peak, n_small):
     # contribution rows (the ranks are written by the last iteration only).
     # Most of those row reads hit L2 (R-MAT hubs' rows are read again and
     # again), so this is a work figure, not DRAM traffic; the DRAM fraction
-    # uses the bytes ncu counted for one light-row launch at this size (3.03
-    # GB read + 2.08 GB written with the ranks written every iteration; 4.0
-    # GB with the ranks written by the last one only)
+    # uses the bytes ncu counted for one iteration's launch at this size
     ppr_bytes = m * (256.0 + 4.0) + 8.0 * (n + 1) + n * 256.0
     ppr_dram = PPR_DRAM_BYTES_PER_ITER * m / 128311324.0
     out["ppr128"] = {"ms_per_iter": round(t, 3), "gedges_per_s_per_iter": round(m / (t / 1e3) / 1e9, 3),
                      "seed_edges_per_s": round(128 * m / (t / 1e3) / 1e9, 1),
                      "dram_frac_of_hbm": round(ppr_dram / (t / 1e3) / 1e9 / hbm_peak, 4),
                      "dram_bytes_per_iter": ppr_dram,
-                     "dram_bytes_source": "ncu dram__bytes_read+write of k_ppr_light at R-MAT 22, less the rank "
-                                          "rows no longer written every iteration, scaled by m",
+                     "dram_bytes_source": "ncu dram__bytes_read+write of k_ppr_wide at R-MAT 22, scaled by m",
                      "work_bytes_per_iter": ppr_bytes,
                      "work_bytes_over_time_frac": round(ppr_bytes / (t / 1e3) / 1e9 / hbm_peak, 4),
                      "storage": "bf16 rows of 128 seeds, fp32 sums"}
@@ -856,10 +855,11 @@ def run_ours(args, ws, rank, local):
         value_threshold = total_half_edges / (t_thr / 1e3) / 1e9
     per_root = [st.edges_reached / 2.0 / (st.total_ms / 1e3) / 1e9 for st in stats]
 
-    # roofline of the dominant traversal kernel (by summed kernel time): each
-    # step's traversal kernel span (first CTA start to last CTA end, stamped
-    # by the kernel) and, beside it, the whole step (launch gaps, list/bitmap
-    # conversions and the next step's decision included)
+    # roofline of the traversal kernel.  By default a BFS is one launch of
+    # k_bfs_run, whose steps (their barrier and the next step's decision
+    # included) are listed by kind beside it; other drivers launch a kernel per
+    # step, whose span (first CTA start to last CTA end) is stamped by the
+    # kernel, and the dominant one by summed time is taken
     ktime = {}
     kbytes = {}
     stime = {}
@@ -869,11 +869,18 @@ def run_ours(args, ws, rank, local):
             ktime[v] = ktime.get(v, 0.0) + st.kernel_ms[it]
             stime[v] = stime.get(v, 0.0) + st.iter_ms[it]
             kbytes[v] = kbytes.get(v, 0.0) + bfs_bytes(n, st, it)
-    dom = max(ktime, key=ktime.get)
-    nlaunch = sum(1 for st in stats for it in range(st.iterations) if st.variant[it] == dom)
-    achieved = kbytes[dom] / (ktime[dom] / 1e3) / 1e9
-    kernel_names = {gg.VAR_PULL_DENSE: "k_pull", gg.VAR_PUSH_SPARSE: "k_push_binned",
-                    gg.VAR_PUSH_MERGE: "k_push_merge", gg.VAR_PUSH_DENSE: "k_push_dense"}
+    resident = all(st.kernels == 2 for st in stats)  # k_bfs_start and k_bfs_run
+    if resident:
+        dom_name, nlaunch = "k_bfs_run", len(stats)
+        dom_ms, dom_bytes = sum(ktime.values()), sum(kbytes.values())
+        kernel_names = {gg.VAR_PULL_DENSE: "k_bfs_run: pull steps", gg.VAR_PUSH_SPARSE: "k_bfs_run: push steps"}
+    else:
+        kernel_names = {gg.VAR_PULL_DENSE: "k_pull", gg.VAR_PUSH_SPARSE: "k_push_binned",
+                        gg.VAR_PUSH_MERGE: "k_push_merge", gg.VAR_PUSH_DENSE: "k_push_dense"}
+        dom = max(ktime, key=ktime.get)
+        nlaunch = sum(1 for st in stats for it in range(st.iterations) if st.variant[it] == dom)
+        dom_name, dom_ms, dom_bytes = kernel_names[dom], ktime[dom], kbytes[dom]
+    achieved = dom_bytes / (dom_ms / 1e3) / 1e9
     bfs_iter_total_ms = sum(ktime.values())
     bfs_pass_bytes = 8.0 * (n + 1) + 4.0 * m + 8.0 * n
     # whole-run roofline: the algorithmic bytes of every iteration of every
@@ -921,9 +928,6 @@ def run_ours(args, ws, rank, local):
             cc_ms.append(st.total_ms)
             cst = st
         cc_best = float(np.median(cc_ms))
-        # per-iteration records (variant, counts) of one more run
-        cst = gg.RunStats()
-        g.cc(label=lab, host=False, opts=gg.default_opts(gg.THRESH_FRAC, 5, collect=True), stats=cst)
         # one pass over the CSC and the labels, as the BFS line's one-pass fraction
         cc_pass = 8.0 * (n + 1) + 4.0 * m + 8.0 * n
         cc_all = sum(cc_bytes(n, m, cst, it) for it in range(min(cst.iterations, gg.MAX_ITERS)))
@@ -1076,16 +1080,16 @@ def run_ours(args, ws, rank, local):
                        "variant_selection": "learned" if sel is not None else "threshold",
                        "l2": "graph 2.3 GB > 126 MB L2, no flush between steps",
                        "graph_build_s": round(gen_s, 2)},
-            "roofline": {"bound": "hbm", "kernel": kernel_names[dom], "achieved": round(achieved, 1),
+            "roofline": {"bound": "hbm", "kernel": dom_name, "achieved": round(achieved, 1),
                          "peak": hbm_peak, "unit": "GB/s", "frac": round(achieved / hbm_peak, 4),
-                         "traffic": (K_PULL_TRAFFIC_PER_LAUNCH * n / (1 << 24)
-                                     if kernel_names[dom] == "k_pull" else None),
-                         "traffic_source": "ncu dram__bytes_read+write of k_pull, scale-23 capture scaled by n",
+                         "traffic": K_BFS_TRAFFIC_PER_RUN * n / (1 << 24) if resident else None,
+                         "traffic_source": "ncu dram__bytes_read+write of k_bfs_run, scale-23 capture scaled by n",
                          "peak_kind": peak_kind, "launches": nlaunch,
-                         "bytes_per_launch": round(kbytes[dom] / max(nlaunch, 1)),
-                         "ms_per_launch": round(ktime[dom] / max(nlaunch, 1), 4),
-                         "duration": "kernel span per launch (first CTA start to last CTA end, stamped by the "
-                                     "kernel inside the graph-driven run)"},
+                         "bytes_per_launch": round(dom_bytes / max(nlaunch, 1)),
+                         "ms_per_launch": round(dom_ms / max(nlaunch, 1), 4),
+                         "duration": "from the run's first step to its end, stamped by the kernel" if resident else
+                                     "kernel span per launch (first CTA start to last CTA end, stamped by the "
+                                     "kernel)"},
             "clocks": clocks, "gpu_launches": launches,
             "e2e": e2e, "cpu_baseline": cpu, "parity": parity, "wall_s": wall,
         }
@@ -1170,7 +1174,7 @@ def run_case(a):
         ts = []
         for _ in range(a.reps):
             st = gg.RunStats()
-            g.cc(host=False, opts=gg.default_opts(gg.THRESH_FRAC, 5, collect=True), stats=st)
+            g.cc(host=False, opts=gg.default_opts(gg.THRESH_FRAC, 5), stats=st)
             ts.append(st.total_ms)
         out.update(ms=round(float(np.median(ts)), 4), iterations=iter_table(st))
     elif a.case == "kc":
@@ -1179,7 +1183,9 @@ def run_case(a):
         ts = []
         for _ in range(a.reps):
             st = gg.RunStats()
-            _, largest = g.kcore(host=False, opts=gg.default_opts(collect=a.reps == 1), stats=st)
+            # (records per step: the host-driven peel)
+            opts = gg.default_opts(gg.THRESH_ALWAYS_SPARSE, collect=True) if a.reps == 1 else None
+            _, largest = g.kcore(host=False, opts=opts, stats=st)
             ts.append(st.total_ms)
         out.update(ms=round(float(np.median(ts)), 4), largest_core=largest, peel_steps=st.iterations,
                    floors=int(st.vertices_reached), kernels=int(st.kernels),

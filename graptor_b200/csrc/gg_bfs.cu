@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kBB, 2) k_bfs_run(BArgs A) {
     // staging of a push (items) and of a pull (kept candidates, open rows):
     // never in use at the same time
     __shared__ union {
-        unsigned long long items[kBW][IT_KINDS][ItemAppender::CAP];
+        unsigned long long items[kBW][ItemLister::STAGED][ItemAppender::CAP];
         struct {
             uint32_t keep[kBW][kKeepCap], rest[kBW][kRestCap];
         } pull;

@@ -60,7 +60,7 @@ struct KcArgs {
 
 __global__ void __launch_bounds__(kKcBlock, 2) k_kc_run(KcArgs A) {
     constexpr unsigned FULL = 0xffffffffu;
-    __shared__ unsigned long long s_items[kKcBlock / 32][IT_KINDS][ItemAppender::CAP];
+    __shared__ unsigned long long s_items[kKcBlock / 32][ItemLister::STAGED][ItemAppender::CAP];
     __shared__ uint32_t s_alive[kKcBlock / 32][128];
     KcState *st = A.st;
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;

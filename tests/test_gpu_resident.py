@@ -198,3 +198,21 @@ def test_huge_rows_are_listed_together(ctx, knobs):
     assert np.array_equal(core, want) and largest == wl
     assert np.array_equal(g.cc(), O.cc(og))
     g.close()
+
+
+@pytest.mark.parametrize("width,deg", [(20, 3), (1000, 8), (7000, 1)])
+def test_resident_cc_local_ids(ctx, knobs, width, deg):
+    """Chains of trees that many edges merge at once: neighbours within `width`
+    ids, components cut every 9973 vertices."""
+    n = 60000
+    rng = np.random.default_rng(width)
+    src = np.repeat(np.arange(n), deg)
+    dst = np.minimum(src + rng.integers(1, width, len(src)), (src // 9973 + 1) * 9973 - 1).clip(max=n - 1)
+    g = ctx.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32))
+    off, adj = g.download()
+    want = O.cc(O.Graph(n, off, adj))
+    for res in (1, 0):
+        gg.tuning_set("resident", res)
+        for _ in range(5):
+            assert np.array_equal(g.cc(), want), res
+    g.close()

@@ -452,7 +452,17 @@ gg_status build_heavy_rows(gg_graph *g) {
             HK(cub::DeviceScan::InclusiveSum(tmp, tb, H.light_prefix, H.light_prefix, (int64_t)nwords, st));
             HK(cub::DeviceScan::InclusiveSum(tmp, tb, H.pull_prefix, H.pull_prefix, (int64_t)nwords, st));
             ctx->launches += 2;
-            H.ncut = std::min(nwords, kLightCuts);
+            // no more ranges than their work allows, one per resident warp of the
+            // gather's 5 CTAs per SM at least: a warp overlaps its range's words, not
+            // its tickets (a word per ticket -> so, BF16, us an iteration: grid 30 x
+            // 60000 65.1 -> 48.8, directed star of 2^21 67.4 -> 48.8, ER 1 M x 2 46.9
+            // -> 39.1; least work of 1024 instead of 512: R-MAT 19 relabelled 65.1 ->
+            // 72.6, of 256: grid 65.2)
+            uint64_t work = 0;
+            HK(cudaMemcpyAsync(&work, H.light_prefix + nwords - 1, 8, cudaMemcpyDeviceToHost, st));
+            HK(cudaStreamSynchronize(st));
+            H.ncut = (uint32_t)std::min<uint64_t>(std::min(nwords, kLightCuts),
+                                                  std::max<uint64_t>(work / 512 + 1, (uint64_t)ctx->sm_count * 40));
             HK(cudaMalloc(&H.light_cut, ((size_t)H.ncut + 1) * 4));
             k_light_cuts<<<grid_for(ctx, (uint64_t)H.ncut + 1), 256, 0, st>>>(H.light_prefix, nwords, H.light_cut,
                                                                               H.ncut);

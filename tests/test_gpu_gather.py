@@ -56,3 +56,26 @@ def test_gather_rows(ctx, kind, dtype, acc64):
     tol = want * eps * (np.maximum(deg, 1) if dtype == gg.F64 or not acc64 else 1.001)
     assert np.all(np.abs(got - want) <= tol)
     g.close()
+
+
+@pytest.mark.parametrize("n", [5920 * 32 - 1, 5920 * 32 + 1, 400003, 2200001])
+@pytest.mark.parametrize("deg", [0, 1, 3])
+def test_gather_ranges_of_several_words(ctx, n, deg):
+    """Sparse rows, whose ranges are of several words: up to and beyond a word
+    per warp, none and few edges, and a stretch of longer rows."""
+    rng = np.random.default_rng(n + deg)
+    degs = np.full(n, deg, dtype=np.int64)
+    degs[n // 3: n // 3 + 2000] = 40
+    dst = np.repeat(np.arange(n), degs)
+    src = (dst + 1 + np.arange(len(dst)) % 977) % n
+    g = ctx.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32), symmetrise=False)
+    assert g.m == len(dst)
+    c = rng.uniform(0.5, 1.5, n)
+    contrib, y = g.prop(gg.F64), g.prop(gg.F64)
+    contrib.upload(c)
+    y.fill(0)
+    g.edgemap(gg.EmapDesc(relax=gg.RELAX_ADD_GATHER, a=y.h, src=contrib.h, accum_f64=1, record=gg.RECORD_NONE,
+                          variant=gg.VAR_AUTO))
+    want = np.bincount(dst, weights=c[src], minlength=n)
+    assert np.all(np.abs(y.download() - want) <= want * 2.0 ** -52 * np.maximum(degs, 1))
+    g.close()

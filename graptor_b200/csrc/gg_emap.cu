@@ -68,6 +68,7 @@ struct EmapArgs {
     uint32_t large_ch;            // edges per large-bin chunk
     int merge_med;                // push: medium bin chunked with the large one (small frontiers)
     int large_as_med;             // push: large bin walked a warp per row with the medium one
+    uint32_t small_least;         // push: small-bin sources that a warp takes at least
     // pull candidate lists (drivers only): the destinations that can still
     // pass the (monotone) dst filter.  cand == nullptr: scan all vertices.
     const uint32_t *cand;
@@ -797,6 +798,8 @@ __device__ __forceinline__ void push_edges(const EmapArgs &A, const Op<R> &op, t
     }
 }
 
+constexpr uint32_t kSmallWarps = 4096;
+
 template <int R, int BLOCK>
 __device__ __forceinline__ void push_binned_body(const EmapArgs &A, const Op<R> &op, uint32_t nb_large,
                                                  uint32_t nb_med) {
@@ -864,11 +867,15 @@ __device__ __forceinline__ void push_binned_body(const EmapArgs &A, const Op<R> 
         // flattened; fewer where the bin would leave warps without any (each
         // 128 edges of a warp are a chain of six or more dependent accesses.
         // Levels of 243, 3880 and 60878 sources of a search over edgemap,
-        // directed ER 3 M x 16: 55, 58 and 70 -> 12, 15 and 56 us)
+        // directed ER 3 M x 16: 55, 58 and 70 -> 12, 15 and 56 us).  Beyond
+        // kSmallWarps warps, no fewer than fill a warp: their appends to the
+        // output's counters, one address each, cost more than the shorter
+        // chains give (84 k sources of a 2048^2 grid, ER 4 M x 2, a binary tree:
+        // 28, 25 and 23 us with 32 a warp, 36, 34 and 30 with 9, 28, 26 and 24 so)
         const uint32_t wpb = BLOCK / 32;
         const uint32_t nws = (gridDim.x - nb_large - nb_med) * wpb;
         const uint32_t wid = (blockIdx.x - nb_large - nb_med) * wpb + (threadIdx.x >> 5);
-        const uint32_t per = min(32u, (A.c0 + nws - 1) / nws);
+        const uint32_t per = min(32u, max((A.c0 + nws - 1) / nws, min(A.small_least, (A.c0 + kSmallWarps - 1) / kSmallWarps)));
         for (uint64_t base = (uint64_t)wid * per; base < A.c0; base += (uint64_t)nws * per) {
             const uint64_t i = base + lane;
             const bool have = lane < per && i < A.c0;
@@ -1120,6 +1127,12 @@ static gg_status pull_records(gg_graph *g, const Tuning &t, const uint4 **fi, co
     return GG_OK;
 }
 
+// Sources of the small bin that fill the 128 edges a warp has in flight, going by
+// the graph's average degree.
+static uint32_t small_least(const gg_graph *g) {
+    return (uint32_t)std::min<uint64_t>(32, std::max<uint64_t>(1, g->m ? 128 * (uint64_t)g->n / g->m : 32));
+}
+
 template <int R>
 static gg_status launch_variant(gg_graph *g, const gg_emap_desc *d, gg_frontier *in,
                                 gg_frontier *out, int variant) {
@@ -1145,6 +1158,7 @@ static gg_status launch_variant(gg_graph *g, const gg_emap_desc *d, gg_frontier 
     A.smax = t.bin_small_max;
     A.mmax = t.bin_medium_max;
     A.K = variant == GG_VAR_PULL_DENSE ? t.pull_k : t.push_k;
+    A.small_least = small_least(g);
     A.word_prefix = g->heavy.pull_prefix;
     GG_CHECK(pull_records(g, t, &A.first_in, &A.first1, &A.rec_n, &A.lazy_off));
     const bool have_out = out != nullptr && d->record != GG_RECORD_NONE;
@@ -1937,6 +1951,7 @@ struct GCtl {
     int sel_iter, sel_push, sel_valid;
     uint32_t smax, mmax, large_ch, sm_count;
     int pull_k, push_k;
+    uint32_t small_least;
     const uint64_t *off, *in_off, *word_prefix;
     const uint32_t *adj, *in_adj;
     const uint4 *first_in;
@@ -2142,6 +2157,7 @@ __device__ void decide_step(GCtl *c, GCtl *h, const mlp::LaneWeights *lw) {
     A.smax = h->smax;
     A.mmax = h->mmax;
     A.K = push ? h->push_k : h->pull_k;
+    A.small_least = h->small_least;
     A.word_prefix = h->word_prefix;
     A.first_in = push ? nullptr : h->first_in;
     A.first1 = push ? nullptr : h->first1;
@@ -2838,6 +2854,7 @@ gg_status graph_bfs_level(gg_graph *g, uint32_t root, const gg_run_opts &opt, gg
     h.sm_count = (uint32_t)ctx->sm_count;
     h.pull_k = t.pull_k;
     h.push_k = t.push_k;
+    h.small_least = small_least(g);
     h.off = g->off;
     h.in_off = g->in_off;
     h.word_prefix = g->heavy.pull_prefix;

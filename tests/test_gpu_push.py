@@ -37,3 +37,33 @@ def test_push_from_small_sources(ctx, k):
     assert np.array_equal(np.sort(fout.download()), np.flatnonzero(reached))
     assert fout.counts() == (int(reached.sum()), int(deg[reached].sum()))
     G.close()
+
+
+@pytest.mark.parametrize("deg", [1, 5, 40])
+@pytest.mark.parametrize("k", [4095, 4096, 4097, 8193, 131073])
+def test_push_where_warps_take_several(ctx, k, deg):
+    """Sources per warp by what fills it: graphs of few edges, some and many a
+    vertex, around the 4096 warps beyond which they count."""
+    n = 140003
+    src = np.repeat(np.arange(n), deg)
+    dst = (src + 1 + np.arange(len(src)) % (deg * 7 + 1) * 3) % n
+    G = ctx.from_edges(n, src.astype(np.uint32), dst.astype(np.uint32), symmetrise=False)
+    rng = np.random.default_rng(k)
+    active = np.zeros(n, dtype=bool)
+    active[rng.choice(n, k, replace=False)] = True
+    a, prev = G.prop(gg.U32), G.prop(gg.U32)
+    fin, fout = G.frontier(), G.frontier()
+    fin.set_list(np.flatnonzero(active))
+    lab = rng.integers(0, 1 << 30, n).astype(np.uint32)
+    a.upload(lab)
+    prev.upload(lab)
+    G.edgemap(gg.EmapDesc(relax=gg.RELAX_OR_U32, a=a.h, src=prev.h, prev=prev.h, record=gg.RECORD_NE_PREV,
+                          variant=gg.VAR_PUSH_SPARSE), fin, fout)
+    want = lab.copy()
+    on = active[src]
+    np.bitwise_or.at(want, dst[on], lab[src[on]])
+    changed = np.flatnonzero(want != lab)
+    assert np.array_equal(a.download(), want)
+    assert np.array_equal(np.sort(fout.download()), changed)
+    assert fout.counts() == (len(changed), int(np.bincount(src, minlength=n)[changed].sum()))
+    G.close()

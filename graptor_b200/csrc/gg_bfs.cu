@@ -625,23 +625,7 @@ timed_out:
 
 const void *selector_weights(gg_graph *g);
 
-// Per-graph buffers of the resident BFS.
-struct BfsRes {
-    BState *bs = nullptr;
-    uint32_t *bits = nullptr;
-    PState *h_rec = nullptr, *d_rec = nullptr;  // page-locked, mapped
-    PFront fr[2];                               // hand-over lists (the scratch frontiers' buffers)
-};
-
-void bfs_resident_free(gg_graph *g) {
-    BfsRes *r = (BfsRes *)g->bfs_res;
-    if (!r) return;
-    cudaFree(r->bs);
-    cudaFree(r->bits);
-    cudaFreeHost(r->h_rec);
-    delete r;
-    g->bfs_res = nullptr;
-}
+static_assert(sizeof(PState) <= kRunRecord && sizeof(BState) <= kRunState, "records and state block");
 
 static gg_status bfs_resident_buffers(gg_graph *g) {
     gg_ctx *ctx = g->ctx;
@@ -653,29 +637,16 @@ static gg_status bfs_resident_buffers(gg_graph *g) {
     }
     GG_CHECK(cand_lists_alloc(g));
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
-    GG_CHECK(graph_items(g));
-    if (g->bfs_res) return GG_OK;
-    BfsRes *r = new (std::nothrow) BfsRes;
-    if (!r) return GG_ERR_OOM;
-    g->bfs_res = r;
-    const size_t nw4 = ((size_t)g->n + 127) / 128;
-    cudaError_t e = cudaMalloc(&r->bs, sizeof(BState));
-    if (e == cudaSuccess) e = cudaMalloc(&r->bits, 3 * nw4 * 16);
-    if (e == cudaSuccess) e = cudaHostAlloc(&r->h_rec, sizeof(PState), cudaHostAllocMapped);
-    if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0);
-    if (e == cudaSuccess) return GG_OK;
-    bfs_resident_free(g);
-    return cuda_error(ctx, e, "resident BFS");
+    GG_CHECK(run_record(ctx));
+    return resident_memory(g);
 }
 
 // What the resident runs of g allocated for themselves goes back: the drivers
 // taken instead need room too (their frontiers and candidate lists are the same).
 gg_status resident_give_up(gg_graph *g, gg_status s) {
     if (s != GG_ERR_OOM) return s;
-    bfs_resident_free(g);
-    cc_resident_free(g);
-    cudaFree(g->items);
-    g->items = nullptr;
+    cudaFree(g->resident);
+    g->resident = nullptr;
     return GG_OK;
 }
 
@@ -689,7 +660,6 @@ gg_status bfs_resident_prepare(gg_graph *g, bool *ok) {
 
 static gg_status bfs_args(gg_graph *g, gg_prop *level, const gg_run_opts &opt, PState *st, BArgs &A) {
     const Tuning &t = tuning();
-    BfsRes *r = (BfsRes *)g->bfs_res;
     std::memset(&A, 0, sizeof(A));
     A.off = g->off;
     A.in_off = g->in_off;
@@ -697,16 +667,17 @@ static gg_status bfs_args(gg_graph *g, gg_prop *level, const gg_run_opts &opt, P
     A.in_adj = g->in_adj;
     A.first_in = g->first_in;
     A.n = g->n;
-    A.nw4 = (uint32_t)(((uint64_t)g->n + 127) / 128);
+    A.nw4 = (uint32_t)bitmap_words4(g);
     A.m = g->m;
     A.level = (int32_t *)level->d;
-    for (int i = 0; i < 3; ++i) A.bits[i] = r->bits + (size_t)i * A.nw4 * 4;
-    A.items = item_lists(g, (unsigned long long *)g->items);
+    uint32_t *bits = (uint32_t *)((char *)g->resident + resident_bits_at(g));
+    for (int i = 0; i < 3; ++i) A.bits[i] = bits + (size_t)i * A.nw4 * 4;
+    A.items = item_lists(g);
     A.cand[0] = g->cand.list[0];
     A.cand[1] = g->cand.list[1];
     A.nonisolated = g->nonisolated;
     A.nonisolated_n = (const unsigned long long *)g->nonisolated_n;
-    A.bs = r->bs;
+    A.bs = (BState *)resident_state(g, RUN_BFS);
     A.st = st;
     for (int i = 0; i < 2; ++i) {
         gg_frontier *f = g->tmp_front[i];
@@ -790,15 +761,14 @@ gg_status bfs_resident(gg_graph *g, gg_prop *level, uint32_t root, const gg_run_
     gg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     const Tuning &t = tuning();
-    BfsRes *r = (BfsRes *)g->bfs_res;
     PState *ds = (PState *)g->pstate;
     BArgs A;
     GG_CHECK(bfs_args(g, level, opt, ds, A));
     A.root = root;
-    A.rec = r->d_rec;
+    A.rec = (PState *)ctx->d_run;
     A.small_ok = t.small_frontier;
     A.small_from = t.graph_handoff > 0 ? t.graph_handoff : 32;
-    PState &hs = *r->h_rec;
+    PState &hs = *(PState *)ctx->h_run;
     while (true) {
         hs.small_done = -1;  // written by the run's end
         GG_CHECK(bfs_launch(g, A));

@@ -30,6 +30,7 @@
 
 #include "gg_grid.cuh"
 #include "gg_internal.cuh"
+#include "gg_items.cuh"
 #include "gg_persist.cuh"
 #include "gg_uf.cuh"
 
@@ -62,6 +63,7 @@ struct CcRecord {
     PState st;
     unsigned int gave_up;
 };
+static_assert(sizeof(CcRecord) <= kRunRecord && sizeof(CcState) <= kRunState, "records and state block");
 
 struct CcArgs {
     const uint64_t *off;
@@ -356,34 +358,8 @@ __global__ void k_cc_start(CcState *cs, PState *st, int searched) {
     cs->hooked = 0;
 }
 
-struct CcRes {
-    CcState *cs = nullptr;
-    CcRecord *h_rec = nullptr, *d_rec = nullptr;  // page-locked, mapped
-};
-
-void cc_resident_free(gg_graph *g) {
-    CcRes *r = (CcRes *)g->cc_res;
-    if (!r) return;
-    cudaFree(r->cs);
-    cudaFreeHost(r->h_rec);
-    delete r;
-    g->cc_res = nullptr;
-}
-
-// The run's own buffers, and those of the search, its levels among them.
+// The search's buffers, its levels among them, and with them this run's.
 static gg_status cc_resident_buffers(gg_graph *g) {
-    if (!g->cc_res) {
-        CcRes *r = new (std::nothrow) CcRes;
-        if (!r) return GG_ERR_OOM;
-        g->cc_res = r;
-        cudaError_t e = cudaMalloc(&r->cs, sizeof(CcState));
-        if (e == cudaSuccess) e = cudaHostAlloc(&r->h_rec, sizeof(CcRecord), cudaHostAllocMapped);
-        if (e == cudaSuccess) e = cudaHostGetDevicePointer((void **)&r->d_rec, r->h_rec, 0);
-        if (e != cudaSuccess) {
-            cc_resident_free(g);
-            return cuda_error(g->ctx, e, "resident CC");
-        }
-    }
     bool search;
     GG_CHECK(bfs_resident_prepare(g, &search));
     if (!search) return GG_ERR_OOM;
@@ -410,7 +386,7 @@ gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok) {
 // host); may be captured.
 gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_host) {
     gg_ctx *ctx = g->ctx;
-    CcRes *r = (CcRes *)g->cc_res;
+    CcState *cs = (CcState *)resident_state(g, RUN_CC);
     CcArgs A;
     std::memset(&A, 0, sizeof(A));
     A.off = g->off;
@@ -422,9 +398,9 @@ gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_h
     A.n = g->n;
     A.m = g->m;
     A.label = (uint32_t *)label->d;
-    A.cs = r->cs;
+    A.cs = cs;
     A.st = st;
-    A.rec = to_host ? r->d_rec : nullptr;
+    A.rec = to_host ? (CcRecord *)ctx->d_run : nullptr;
     A.timeout_ns = tuning().barrier_timeout_ns;
     gg_prop *level;
     GG_CHECK(run_tmp_prop(g, 1, GG_I32, &level));
@@ -435,7 +411,7 @@ gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_h
     A.cand[0] = g->cand.list[0];
     A.cand[1] = g->cand.list[1];
     A.left = g->tmp_front[0]->bins[0];
-    k_cc_start<<<1, 1, 0, ctx->stream>>>(r->cs, st, A.searched);
+    k_cc_start<<<1, 1, 0, ctx->stream>>>(cs, st, A.searched);
     GG_LAUNCHED(ctx);
     // a CTA per 2048 vertices or 16384 edges, all that fit at most
     const uint64_t most = (uint64_t)ctx->sm_count * resident_ctas((const void *)k_cc_run, kCB);
@@ -451,7 +427,7 @@ gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *ite
     gg_ctx *ctx = g->ctx;
     if (!g->pstate) GG_CUDA(ctx, cudaMalloc(&g->pstate, sizeof(PState)));
     PState *st = (PState *)g->pstate;
-    CcRecord &rec = *((CcRes *)g->cc_res)->h_rec;
+    CcRecord &rec = *(CcRecord *)ctx->h_run;
     PState &hs = rec.st;
     hs.iterations = -1;  // written by the run's end
     rec.gave_up = 0;

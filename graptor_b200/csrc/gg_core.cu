@@ -581,7 +581,7 @@ static gg_status graph_finish(gg_graph *g) {
 bool graphs_give_back(gg_ctx *ctx) {
     bool any = false;
     for (gg_graph *g = ctx->graphs; g; g = g->next_graph) {
-        any = any || g->pr_plan || g->scratch || g->items;
+        any = any || g->pr_plan || g->scratch || g->resident;
         pr_plan_free(g);
         resident_give_up(g, GG_ERR_OOM);
         cudaFree(g->scratch);
@@ -615,10 +615,7 @@ static void graph_free(gg_graph *g) {
     cudaFree(g->kc_alive[0]);
     cudaFree(g->kc_alive[1]);
     cudaFree(g->kc_cnt);
-    cudaFree(g->kc_state);
-    cudaFree(g->items);
-    bfs_resident_free(g);
-    cc_resident_free(g);
+    cudaFree(g->resident);
     pr_plan_free(g);
     cudaFree(g->pstate2);
     for (int i = 0; i < 2; ++i) {
@@ -810,6 +807,7 @@ gg_status gg_ctx_destroy(gg_ctx *ctx) {
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->h_pinned) cudaFreeHost(ctx->h_pinned);
     host_stage_free(ctx);
+    cudaFreeHost(ctx->h_run);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     if (ctx->evk0) cudaEventDestroy(ctx->evk0);
@@ -1578,6 +1576,16 @@ gg_status frontier_alloc_bitmap(gg_frontier *f) {
     size_t words = ((size_t)g->n + 31) / 32 + 1;
     GG_CUDA(g->ctx, cudaMalloc(&f->bitmap, words * 4));
     return GG_OK;
+}
+
+gg_status run_record(gg_ctx *ctx) {
+    if (ctx->h_run) return GG_OK;
+    cudaError_t e = cudaHostAlloc(&ctx->h_run, kRunRecord, cudaHostAllocMapped);
+    if (e == cudaSuccess) e = cudaHostGetDevicePointer(&ctx->d_run, ctx->h_run, 0);
+    if (e == cudaSuccess) return GG_OK;
+    cudaFreeHost(ctx->h_run);
+    ctx->h_run = nullptr;
+    return cuda_error(ctx, e, "run records");
 }
 
 // Both candidate lists and their counters, or none of them: a run takes them

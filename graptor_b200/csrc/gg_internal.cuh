@@ -69,6 +69,9 @@ struct gg_ctx {
     void *stage = nullptr;
     cudaEvent_t stage_ev[16] = {};
     gg_graph *graphs = nullptr;  // those alive, linked by next_graph
+    // page-locked memory that a resident run writes its records to, and its
+    // device address: one for all graphs, whose runs wait for their ends
+    void *h_run = nullptr, *d_run = nullptr;
 };
 
 // Frontier counters live on the device in this layout.
@@ -85,6 +88,8 @@ enum {
 enum { NBINS = 3 };
 
 struct gg_graph;
+
+constexpr size_t kRunRecord = 16384;  // bytes of gg_ctx::h_run
 
 // Upper bound of HeavyRows::T (knob heavy_deg): the light rows of a 32-vertex
 // word then hold fewer than 2^32 edges.
@@ -175,10 +180,7 @@ struct gg_graph {
     // each) and their counters {count A, count B, smallest count left}
     uint32_t *kc_alive[2] = {nullptr, nullptr};
     unsigned long long *kc_cnt = nullptr;
-    void *kc_state = nullptr;  // gg_kcore's resident peel
-    void *items = nullptr;     // work items of the resident kernels (gg_items.cuh)
-    void *bfs_res = nullptr;   // resident BFS: buffers
-    void *cc_res = nullptr;    // resident CC: buffers
+    void *resident = nullptr;  // work items, bitmaps and state of the resident runs (gg_items.cuh)
     gg_graph *next_graph = nullptr, **at_graph = nullptr;  // in the context's list; the link that points here
     void *pr_plan = nullptr;   // blocked PageRank gather: edge layout (gg_prplan.cuh)
     uint64_t pr_iters = 0;     // PageRank iterations run so far
@@ -223,6 +225,7 @@ gg_status graph_scratch(gg_graph *g, size_t bytes, void **p);
 gg_status frontier_alloc_bins(gg_frontier *f);
 gg_status frontier_alloc_bitmap(gg_frontier *f);
 gg_status cand_lists_alloc(gg_graph *g);
+gg_status run_record(gg_ctx *ctx);
 bool graphs_give_back(gg_ctx *ctx);
 
 // A graph made by make(), a second time with the memory that the context's
@@ -264,12 +267,10 @@ gg_status bfs_resident_multi(gg_graph *g, gg_prop *level, const uint32_t *d_root
                              const gg_run_opts &opt, gg_run_stats *stats, int *iters_out);
 gg_status bfs_resident_search(gg_graph *g, gg_prop *level, uint32_t root, int steps, unsigned long long give_up,
                               PState *st);
-void bfs_resident_free(gg_graph *g);
 gg_status resident_give_up(gg_graph *g, gg_status s);
 gg_status cc_resident_prepare(gg_graph *g, const gg_run_opts &opt, bool *ok);
 gg_status cc_resident(gg_graph *g, gg_prop *label, gg_run_stats *stats, int *iters_out);
 gg_status cc_resident_enqueue(gg_graph *g, gg_prop *label, PState *st, bool to_host);
-void cc_resident_free(gg_graph *g);
 void pr_plan_free(gg_graph *g);
 gg_status enqueue_bfs_start(gg_graph *g, gg_prop *level, gg_prop *prev, const uint32_t *d_roots, uint32_t k);
 gg_status enqueue_cc_start(gg_graph *g, gg_prop *label, gg_prop *prev);

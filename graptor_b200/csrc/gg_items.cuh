@@ -24,13 +24,27 @@ inline uint64_t items_cap(const gg_graph *g, int kind) {
     default: return 2 * (g->m / kHuge) + 2;
     }
 }
-// The graph's item buffer g->items, kind by kind, allocated on first use.
-gg_status graph_items(gg_graph *g);
+// One allocation per graph, g->resident, holds what its resident runs keep: the
+// items, kind by kind, three frontier bitmaps, and a state block for each run.
+// (An allocation of its own for each cost a graph's first CC some 0.3 ms apiece.)
+constexpr size_t kRunState = 1024;
+enum { RUN_BFS = 0, RUN_CC = 1, RUN_KCORE = 2, RUN_KINDS = 3 };
+inline size_t resident_bits_at(const gg_graph *g) {
+    const uint64_t items = items_cap(g, IT_SHORT) + items_cap(g, IT_LONG) + items_cap(g, IT_HUGE);
+    return (items * 8 + kRunState - 1) / kRunState * kRunState;
+}
+inline size_t bitmap_words4(const gg_graph *g) { return ((size_t)g->n + 127) / 128; }  // 16-byte words
+inline size_t resident_state_at(const gg_graph *g, int run) {
+    return (resident_bits_at(g) + 3 * bitmap_words4(g) * 16 + kRunState - 1) / kRunState * kRunState + run * kRunState;
+}
+inline void *resident_state(const gg_graph *g, int run) { return (char *)g->resident + resident_state_at(g, run); }
+gg_status resident_memory(gg_graph *g);
 
 struct ItemLists {
     unsigned long long *p[IT_KINDS];
 };
-inline ItemLists item_lists(const gg_graph *g, unsigned long long *items) {
+inline ItemLists item_lists(const gg_graph *g) {
+    unsigned long long *items = (unsigned long long *)g->resident;
     ItemLists l;
     for (int k = 0; k < IT_KINDS; ++k) {
         l.p[k] = items;

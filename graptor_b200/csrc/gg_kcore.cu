@@ -47,6 +47,8 @@ struct KcState {
     uint32_t floors, steps, largest;
 };
 
+static_assert(sizeof(KcState) <= kRunState, "state block");
+
 struct KcArgs {
     const uint64_t *off;
     const uint32_t *adj;
@@ -235,9 +237,8 @@ __global__ void __launch_bounds__(256) k_kc_start(const uint64_t *__restrict__ o
     if (threadIdx.x == 0 && k) atomicAdd(&st->many, k);
 }
 
-gg_status graph_items(gg_graph *g) {
-    const size_t total = items_cap(g, IT_SHORT) + items_cap(g, IT_LONG) + items_cap(g, IT_HUGE);
-    if (!g->items) GG_CUDA(g->ctx, cudaMalloc(&g->items, total * 8));
+gg_status resident_memory(gg_graph *g) {
+    if (!g->resident) GG_CUDA(g->ctx, cudaMalloc(&g->resident, resident_state_at(g, RUN_KINDS)));
     return GG_OK;
 }
 
@@ -247,14 +248,9 @@ gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *larg
     gg_ctx *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
     *ran = false;
-    auto buffers = [&]() -> gg_status {
-        GG_CHECK(graph_items(g));
-        if (!g->kc_state) GG_CUDA(ctx, cudaMalloc(&g->kc_state, sizeof(KcState)));
-        return GG_OK;
-    };
-    const gg_status fit = buffers();
+    const gg_status fit = resident_memory(g);
     if (fit != GG_OK) return resident_give_up(g, fit);
-    KcState *st = (KcState *)g->kc_state;
+    KcState *st = (KcState *)resident_state(g, RUN_KCORE);
     KcArgs A;
     A.off = g->off;
     A.adj = g->adj;
@@ -262,7 +258,7 @@ gg_status kcore_resident(gg_graph *g, uint32_t *count, bool *ran, uint32_t *larg
     A.count = count;
     A.alive[0] = g->kc_alive[0];
     A.alive[1] = g->kc_alive[1];
-    A.items = item_lists(g, (unsigned long long *)g->items);
+    A.items = item_lists(g);
     A.st = st;
     A.timeout_ns = tuning().barrier_timeout_ns;
     KcState init;

@@ -1231,19 +1231,23 @@ extern "C" gg_status gg_pagerank(gg_graph *g, const gg_pr_params *p, gg_prop *x,
     const size_t pb = ((g->heavy.nchunks + 1) * 8 + 255) / 256 * 256;
     const PrPlan *plan = nullptr;
     const uint64_t iters = g->pr_iters + (p->tol <= 0 ? (uint64_t)p->maxiter : 0ull);
-    const bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
-                         (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && iters >= kBlockedIters));
+    const size_t vsize = dt == GG_F32 ? 4 : 2, own = 2 * nb + sb + ab + pb;
+    bool blocked = !staged && dt != GG_F64 && dt != GG_FP8E4M3 && tuning().pr_blocked &&
+                   (tuning().pr_blocked == 2 || (g->m >= kBlockedEdges && iters >= kBlockedIters));
     // (the run's time and kernels: with the layout's, where it is built)
     const uint64_t k0 = ctx->launches;
     cudaEventRecord(ctx->ev0, ctx->stream);
-    gg_status s = blocked ? pr_plan(g, dt == GG_F32 ? 4 : 2, tuning().pr_blocked == 2, &plan) : GG_OK;
-    if (s == GG_OK) {
-        const size_t own = 2 * nb + sb + ab + pb;
-        s = graph_scratch(g, own + (plan ? pr_plan_bytes(plan, dt == GG_F32 ? 4 : 2) : 0), &base);
-        if (s == GG_ERR_OOM && plan) {  // without the blocked gather, then
-            plan = nullptr;
-            s = graph_scratch(g, own, &base);
-        }
+    gg_status s = blocked ? pr_plan_wanted(g, vsize, tuning().pr_blocked == 2, &blocked) : GG_OK;
+    if (s == GG_OK) s = graph_scratch(g, own + (blocked ? pr_plan_scratch(g, vsize) : 0), &base);
+    if (s == GG_OK && blocked) {
+        // (the values' space serves the building too; where it turns out too
+        // small, for tiles of few edges, it grows)
+        s = pr_plan(g, (char *)base + own, &plan);
+        if (s == GG_OK && plan) s = graph_scratch(g, own + pr_plan_scratch(g, vsize), &base);
+    }
+    if (s == GG_ERR_OOM && blocked) {  // without the blocked gather, then
+        plan = nullptr;
+        s = graph_scratch(g, own, &base);
     }
     if (s != GG_OK) { if (tmpx) gg_prop_destroy(tmpx); return s; }
     float *y = (float *)base;

@@ -19,26 +19,38 @@ constexpr int kPB = 1024;
 constexpr uint32_t kPer = kBinEdges / kPB;
 static_assert(kBinEdges % kPB == 0 && kBinEdges < 65536, "places within a bin take 16 bits");
 
-// chunks of every tile, and of every bin; sectors[0 / 1]: 32-byte sectors that
-// the 4- / 2-byte values of each bin's first kPB edges lie in, those of a bin
-// told apart by 13 bits of a hash (1000 of them count as 940)
-__global__ void __launch_bounds__(kPB) k_plan_count(const uint32_t *__restrict__ in_adj, uint64_t m, uint32_t nblk,
-                                                    uint32_t nbin, uint32_t *tile, uint32_t *bin_ptr,
-                                                    uint32_t *sectors) {
-    __shared__ uint32_t hist[kBlkMax], seen[2][256];
-    const uint32_t b = blockIdx.x;
-    const uint64_t base = (uint64_t)b * kBinEdges;
-    for (uint32_t i = threadIdx.x; i < nblk; i += kPB) hist[i] = 0;
+// sectors[0 / 1]: 32-byte sectors that the 4- / 2-byte values of each bin's first
+// kPB edges lie in, those of a bin told apart by 13 bits of a hash (1000 of them
+// count as 940)
+__global__ void __launch_bounds__(kPB) k_plan_spread(const uint32_t *__restrict__ in_adj, uint64_t m,
+                                                     uint32_t *sectors) {
+    __shared__ uint32_t seen[2][256];
+    const uint64_t e = (uint64_t)blockIdx.x * kBinEdges + threadIdx.x;
     if (threadIdx.x < 512) seen[threadIdx.x >> 8][threadIdx.x & 255u] = 0;
     __syncthreads();
-    if (base + threadIdx.x < m) {
-        const uint32_t v = __ldg(in_adj + base + threadIdx.x);
+    if (e < m) {
+        const uint32_t v = __ldg(in_adj + e);
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
             const uint32_t h = (v >> (3 + k)) * 2654435761u >> 19;
             atomicOr(&seen[k][h >> 5], 1u << (h & 31u));
         }
     }
+    __syncthreads();
+    if (threadIdx.x < 512) {  // (a counter's bits lie in whole warps)
+        const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(seen[threadIdx.x >> 8][threadIdx.x & 255u]));
+        if (dev::lane_id() == 0) atomicAdd(sectors + (threadIdx.x >> 8), c);
+    }
+}
+
+// chunks of every tile, and of every bin
+__global__ void __launch_bounds__(kPB) k_plan_count(const uint32_t *__restrict__ in_adj, uint64_t m, uint32_t nblk,
+                                                    uint32_t nbin, uint32_t *tile, uint32_t *bin_ptr) {
+    __shared__ uint32_t hist[kBlkMax];
+    const uint32_t b = blockIdx.x;
+    const uint64_t base = (uint64_t)b * kBinEdges;
+    for (uint32_t i = threadIdx.x; i < nblk; i += kPB) hist[i] = 0;
+    __syncthreads();
 #pragma unroll 4
     for (uint32_t i = 0; i < kPer; ++i) {
         const uint64_t e = base + i * kPB + threadIdx.x;
@@ -53,10 +65,6 @@ __global__ void __launch_bounds__(kPB) k_plan_count(const uint32_t *__restrict__
     }
     sum = dev::block_sum<uint32_t, kPB>(sum);
     if (threadIdx.x == 0) bin_ptr[b] = sum;
-    if (threadIdx.x < 512) {  // (a counter's bits lie in whole warps)
-        const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(seen[threadIdx.x >> 8][threadIdx.x & 255u]));
-        if (dev::lane_id() == 0) atomicAdd(sectors + (threadIdx.x >> 8), c);
-    }
 }
 
 // each block's first chunk, and the number of chunks
@@ -165,48 +173,66 @@ void plan_release(PrPlan *P) {
     P->tried = true;
 }
 
-// What the building needs beside the layout: every tile's chunks, every bin's,
-// the blocks' first chunks, and the scans' own.
+// What the building needs beside the layout, in scratch: every tile's chunks,
+// every bin's, the blocks' first chunks, and the scans' own.
 struct PlanTmp {
-    void *base = nullptr, *scan = nullptr;
-    uint32_t *tiles = nullptr, *bins = nullptr, *starts = nullptr;
-    size_t scan_b = 0;
-    ~PlanTmp() { cudaFree(base); }
+    uint32_t *tiles, *bins, *starts;
+    void *scan;
+    size_t scan_b, bytes;
+    PlanTmp(const PrPlan *P, void *scratch) {
+        const uint64_t ntile = (uint64_t)P->nblk * P->nbin;
+        const size_t tb = aligned((ntile + 1) * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
+                     sb = aligned(((size_t)P->nblk + 1) * 4);
+        scan_b = std::max(scan_bytes(ntile + 1), scan_bytes((uint64_t)P->nbin + 1));
+        bytes = tb + bb + sb + scan_b;
+        char *p = (char *)scratch;
+        tiles = (uint32_t *)p;
+        bins = (uint32_t *)(p + tb);
+        starts = (uint32_t *)(p + tb + bb);
+        scan = p + tb + bb + sb;
+    }
 };
 
 #define PK(expr) do { cudaError_t _e = (expr); if (_e != cudaSuccess) return _e; } while (0)
 
-// Counts the chunks of every tile (at[k]: block k's first one, of P->chunks) and
-// the sectors that the sampled edges' values lie in.
+// The share of sectors that a sample of the edges lies in.
+cudaError_t plan_spread(gg_graph *g, PrPlan *P) {
+    cudaStream_t st = g->ctx->stream;
+    uint32_t *d = nullptr, h[2] = {0, 0};
+    PK(cudaMalloc(&d, sizeof(h)));
+    cudaError_t e = cudaMemsetAsync(d, 0, sizeof(h), st);
+    if (e == cudaSuccess) {
+        k_plan_spread<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, d);
+        g->ctx->launches++;
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFree(d);
+    PK(e);
+    const double sampled = (double)(g->m / kBinEdges) * kPB + (double)std::min<uint64_t>(g->m % kBinEdges, kPB);
+    for (int k = 0; k < 2; ++k) P->spread[k] = (float)(h[k] / sampled);
+    P->sampled = true;
+    return cudaSuccess;
+}
+
+// Counts the chunks of every tile; at[k]: block k's first one, of P->chunks.
 cudaError_t plan_count(gg_graph *g, PrPlan *P, PlanTmp &T, std::vector<uint32_t> &at) {
     gg_ctx *ctx = g->ctx;
     cudaStream_t st = ctx->stream;
     const uint64_t ntile = (uint64_t)P->nblk * P->nbin;
-    const size_t tb = aligned((ntile + 1) * 4), bb = aligned(((size_t)P->nbin + 1) * 4),
-                 sb = aligned(((size_t)P->nblk + 3) * 4);  // (and the sector counts)
-    T.scan_b = std::max(scan_bytes(ntile + 1), scan_bytes((uint64_t)P->nbin + 1));
-    PK(cudaMalloc(&T.base, tb + bb + sb + T.scan_b));
-    T.tiles = (uint32_t *)T.base;
-    T.bins = (uint32_t *)((char *)T.base + tb);
-    T.starts = (uint32_t *)((char *)T.base + tb + bb);
-    T.scan = (char *)T.base + tb + bb + sb;
     PK(cudaMemsetAsync(T.tiles + ntile, 0, 4, st));
     PK(cudaMemsetAsync(T.bins + P->nbin, 0, 4, st));
-    uint32_t *sectors = T.starts + P->nblk + 1;
-    PK(cudaMemsetAsync(sectors, 0, 8, st));
-    k_plan_count<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, P->nblk, P->nbin, T.tiles, T.bins, sectors);
+    k_plan_count<<<P->nbin, kPB, 0, st>>>(g->in_adj, g->m, P->nblk, P->nbin, T.tiles, T.bins);
     PK(cudaGetLastError());
     PK(cub::DeviceScan::ExclusiveSum(T.scan, T.scan_b, T.tiles, T.tiles, (int64_t)ntile + 1, st));
     k_plan_starts<<<P->nblk / 256 + 1, 256, 0, st>>>(T.tiles, P->nblk, P->nbin, T.starts);
     PK(cudaGetLastError());
     ctx->launches += 3;
-    at.resize((size_t)P->nblk + 3);
+    at.resize((size_t)P->nblk + 1);
     PK(cudaMemcpyAsync(at.data(), T.starts, at.size() * 4, cudaMemcpyDeviceToHost, st));
     PK(cudaStreamSynchronize(st));
     P->chunks = at[P->nblk];
-    const double sampled = (double)(g->m / kBinEdges) * kPB + (double)std::min<uint64_t>(g->m % kBinEdges, kPB);
-    for (int k = 0; k < 2; ++k) P->spread[k] = (float)(at[P->nblk + 1 + k] / sampled);
-    P->counted = true;
     return cudaSuccess;
 }
 
@@ -273,54 +299,68 @@ cudaError_t plan_build(gg_graph *g, PrPlan *P, PlanTmp &T, const std::vector<uin
 
 }  // namespace
 
-size_t pr_plan_bytes(const PrPlan *P, size_t size) {
-    return P->chunks * 8 * size + (size_t)P->nbin * 16;  // values, parts of rows
-}
-
-static gg_status plan_of(gg_graph *g, size_t size, bool always, const PrPlan **out) {
+gg_status pr_plan_wanted(gg_graph *g, size_t size, bool always, bool *yes) {
+    *yes = false;
     if (!g->pr_plan) {
-        PrPlan *P = new PrPlan();
+        PrPlan *P = new (std::nothrow) PrPlan();
+        if (!P) return GG_OK;
         P->nblk = (uint32_t)(((uint64_t)g->n + kBlkSrc - 1) >> kBlkSrcLog);
         P->nbin = (uint32_t)((g->m + kBinEdges - 1) / kBinEdges);
         P->tried = !g->m || P->nblk > kBlkMax || g->m >> 32;  // (chunk numbers take 32 bits)
         g->pr_plan = P;
     }
     PrPlan *P = (PrPlan *)g->pr_plan;
-    if (!always && P->nblk <= kBlkInL1) return GG_OK;
-    const auto pays = [&]() {
-        return always || P->spread[size == 4 ? 0 : 1] >= (P->nblk <= kBlkHubsInL1 ? kSpreadLeastHubs : kSpreadLeast);
-    };
-    if (!P->tried && (!P->counted || pays())) {
-        PlanTmp T;
-        std::vector<uint32_t> at;
-        cudaError_t e = plan_count(g, P, T, at);
-        if (e == cudaSuccess && pays()) {
-            size_t free_b = 0, all_b = 0;
-            e = cudaMemGetInfo(&free_b, &all_b);
-            // a chunk's layout and values, 36 and up to 40 bytes, leave half of the memory
-            if (e == cudaSuccess && P->chunks * 152 > free_b) e = cudaErrorMemoryAllocation;
-            if (e == cudaSuccess) e = plan_build(g, P, T, at);
-            P->tried = P->ready = e == cudaSuccess;
-        }
-        if (e != cudaSuccess) {
-            plan_release(P);
-            if (e != cudaErrorMemoryAllocation) return cuda_error(g->ctx, e, "PageRank edge layout");
+    if ((P->tried && !P->ready) || (!always && P->nblk <= kBlkInL1)) return GG_OK;
+    if (!always && !P->sampled) {
+        const cudaError_t e = plan_spread(g, P);
+        if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
             return GG_OK;
         }
+        if (e != cudaSuccess) return cuda_error(g->ctx, e, "PageRank edge layout");
     }
-    if (P->ready && pays()) *out = P;
+    *yes = always || P->spread[size == 4 ? 0 : 1] >= (P->nblk <= kBlkHubsInL1 ? kSpreadLeastHubs : kSpreadLeast);
     return GG_OK;
 }
 
-gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out) {
+size_t pr_plan_scratch(gg_graph *g, size_t size) {
+    const PrPlan *P = (const PrPlan *)g->pr_plan;
+    const size_t parts = (size_t)P->nbin * 16;  // of rows
+    if (P->ready) return P->chunks * 8 * size + parts;
+    return std::max(g->m * size + parts, PlanTmp(P, nullptr).bytes);
+}
+
+static gg_status plan_make(gg_graph *g, void *scratch) {
+    PrPlan *P = (PrPlan *)g->pr_plan;
+    P->tried = true;
+    PlanTmp T(P, scratch);
+    std::vector<uint32_t> at;
+    cudaError_t e = plan_count(g, P, T, at);
+    size_t free_b = 0, all_b = 0;
+    if (e == cudaSuccess) e = cudaMemGetInfo(&free_b, &all_b);
+    // the layout, 36 bytes a chunk, leaves half of the memory beside the values
+    if (e == cudaSuccess && P->chunks * 72 > free_b) e = cudaErrorMemoryAllocation;
+    if (e == cudaSuccess) e = plan_build(g, P, T, at);
+    P->ready = e == cudaSuccess;
+    if (P->ready) return GG_OK;
+    plan_release(P);
+    if (e != cudaErrorMemoryAllocation) return cuda_error(g->ctx, e, "PageRank edge layout");
+    cudaGetLastError();
+    return GG_OK;
+}
+
+gg_status pr_plan(gg_graph *g, void *scratch, const PrPlan **out) {
     *out = nullptr;
-    try {
-        return plan_of(g, size, always, out);
-    } catch (const std::bad_alloc &) {  // of the host: no layout either
-        if (g->pr_plan) plan_release((PrPlan *)g->pr_plan);
-        return GG_OK;
+    PrPlan *P = (PrPlan *)g->pr_plan;
+    if (!P->tried) {
+        try {
+            GG_CHECK(plan_make(g, scratch));
+        } catch (const std::bad_alloc &) {  // of the host: no layout either
+            plan_release(P);
+        }
     }
+    if (P->ready) *out = P;
+    return GG_OK;
 }
 
 void pr_plan_free(gg_graph *g) {

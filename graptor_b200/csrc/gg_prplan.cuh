@@ -62,7 +62,7 @@ __host__ __device__ __forceinline__ uint32_t blk_slot(uint32_t v) {
 __host__ __device__ __forceinline__ uint32_t bin_slot(uint32_t p) { return p ^ ((p >> 5) & 31u); }
 
 struct PrPlan {
-    bool counted = false, tried = false, ready = false;
+    bool sampled = false, tried = false, ready = false;
     float spread[2] = {0, 0};  // sectors per edge of 4- and 2-byte values
     uint32_t nblk = 0, nbin = 0, nparts = 0;
     uint64_t chunks = 0;
@@ -78,13 +78,16 @@ struct PrPlan {
     uint32_t *part_seg = nullptr;
 };
 
-// The graph's plan for a gather of values of `size` bytes, built when first
-// asked for; null where the graph does not fit the layout's limits, or the
-// layout and the values not half of the free memory, or (unless `always`) the
-// gather by rows is the faster one (kSpreadLeast).
-gg_status pr_plan(gg_graph *g, size_t size, bool always, const PrPlan **out);
-// Bytes of scratch that a gather of values of `size` bytes takes.
-size_t pr_plan_bytes(const PrPlan *P, size_t size);
+// Whether a gather of values of `size` bytes should go by blocks: not where the
+// graph does not fit the layout's limits or memory, nor (unless `always`) where
+// the gather by rows is the faster one (kSpreadLeast).
+gg_status pr_plan_wanted(gg_graph *g, size_t size, bool always, bool *yes);
+// Bytes of scratch that such a gather takes, as far as is known before the plan
+// is there, and that its building takes.
+size_t pr_plan_scratch(gg_graph *g, size_t size);
+// The graph's plan, built in scratch of pr_plan_scratch when first asked for;
+// null where the layout does not leave half of the free memory.
+gg_status pr_plan(gg_graph *g, void *scratch, const PrPlan **out);
 void pr_plan_free(gg_graph *g);
 
 }  // namespace gg

@@ -19,9 +19,8 @@
  * more, and more than 65536 vertices, whose neighbours' values lie far apart
  * goes by blocks of sources once the graph has run 16 iterations (those
  * counted that a run without a tolerance is sure to take), with a layout of 36
- * bytes for every 8 edges kept with it (about 4.7 bytes an edge; more where
- * there are few edges for each 24576 edges x 32768 vertices); 2: wherever that
- * layout can be built; 0: never),
+ * bytes for every 8 edges kept with it (4.7 bytes an edge at 1 M vertices, 5
+ * at 16 M, 6 at 64 M); 2: wherever that layout can be built; 0: never),
  * persistent (bit mask: 1 BFS levels, 2 BFS parents, 4 CC run as
  * one device-driven cooperative launch; otherwise one launch per iteration
  * from the host), resident (1, the default: BFS levels run as one resident

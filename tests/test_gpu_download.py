@@ -50,3 +50,14 @@ def test_download_leaves_the_current_device(ctx):
         assert np.array_equal(p.download(), a)
         assert torch.cuda.current_device() == 0
     c.close()
+
+
+@pytest.mark.parametrize("n", [(16 << 20) - 1, 16 << 20, (16 << 20) + 1, (17 << 20) + 5])
+def test_download_where_threads_take_over(ctx, n):
+    g = ctx.from_edges(n, np.zeros(0, np.uint32), np.zeros(0, np.uint32))
+    p = g.prop(gg.U8)
+    a = np.random.default_rng(n).integers(0, 256, n, dtype=np.uint8)
+    p.upload(a)
+    for _ in range(3):
+        assert np.array_equal(p.download(), a)
+    g.close()

@@ -19,11 +19,11 @@ namespace gg {
 
 constexpr size_t kPiece = 1u << 20;     // bytes per slot
 constexpr int kMaxCopiers = 8;          // threads; 16 MiB page-locked per context
-// From here on threads: below, starting them costs more than they save (into
-// memory that has its pages, directly -> by threads: 4 MiB 275 -> 525 us, 8 MiB
-// 515 -> 600 to 750, 12 MiB 740 -> 720 to 1010, 16 MiB 960 -> 650 to 900, 64 MiB
-// 3600 -> 1800 to 2200; into fresh pages 64 MiB 13400 -> 3400).
-constexpr size_t kStagedBytes = 16u << 20;
+// From here on threads: below, starting them costs what they save (mean of 100
+// copies into memory that has its pages, directly -> by threads: 4 MiB 275 -> 340
+// us, 6 MiB 387 -> 415, 8 MiB 500 -> 505, 12 MiB 745 -> 690, 16 MiB 975 -> 815, 24 MiB
+// 1450 -> 960; into fresh pages 64 MiB 13400 -> 3400).
+constexpr size_t kStagedBytes = 8u << 20;
 
 void host_stage_free(gg_ctx *ctx) {
     for (auto &e : ctx->stage_ev) {

@@ -52,7 +52,7 @@ def test_download_leaves_the_current_device(ctx):
     c.close()
 
 
-@pytest.mark.parametrize("n", [(16 << 20) - 1, 16 << 20, (16 << 20) + 1, (17 << 20) + 5])
+@pytest.mark.parametrize("n", [(8 << 20) - 1, 8 << 20, (8 << 20) + 1, (9 << 20) + 5])
 def test_download_where_threads_take_over(ctx, n):
     g = ctx.from_edges(n, np.zeros(0, np.uint32), np.zeros(0, np.uint32))
     p = g.prop(gg.U8)

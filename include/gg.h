@@ -15,6 +15,9 @@
  *     gives a message for the calling context.
  *   - Handles are opaque and owned by the caller (explicit *_destroy).
  *     Device memory belongs to the library.
+ *   - A graph keeps the working memory of its calls for the next ones.  Where a
+ *     new graph of the same context does not fit, the others give theirs back
+ *     and the call is tried once more.
  *   - One CUDA stream per context; calls on one context come from one host
  *     thread at a time (Graptor's own contract: one host thread calls the
  *     library, all parallelism is inside).
